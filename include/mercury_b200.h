@@ -199,9 +199,9 @@ MB_API mb_status mb_collect(mb_context* ctx, float* pos, float* vel, float* stre
 MB_API mb_status mb_centre_of_mass(mb_context* ctx, float* com);
 
 /* Per-robot status after the last run: bit 0 = a position became NaN/Inf;
- * bit 1 = the robot's bin did not fit the shared memory the launch was
- * sized for and was not stepped (a safeguard of the register-row kernel;
- * the host sizes every launch so that it does not happen).  Synchronous.
+ * bit 1 = the robot's bin was not stepped because it did not fit the
+ * launch's shared memory (the host sizes every launch so that it does not
+ * happen).  Synchronous.
  * The reference asserts on NaN in Collect (Simulator.cu:550). */
 MB_API mb_status mb_robot_flags(mb_context* ctx, uint32_t* flags);
 
@@ -293,11 +293,11 @@ MB_API mb_status mb_get_launch_config(const mb_context* ctx, mb_launch_config* c
 MB_API mb_status mb_set_launch_config(mb_context* ctx, const mb_launch_config* cfg);
 
 /* The step kernel the next launches of the uploaded batch use:
- * *register_rows = 1 when each mass's row of incident springs is held in
- * registers (resident bins of a 1,024-thread shape with at most one mass per
- * thread, no face drag, and room for 8 more bytes of shared memory per
- * spring), else 0; *smem_bytes = the dynamic shared memory per CTA of those
- * launches.  Either pointer may be NULL.  No reference counterpart. */
+ * *register_rows = 1 when each mass's row of incident springs is held per
+ * thread (resident bins of a 1,024-thread shape with at most one mass per
+ * thread and no face drag), else 0; *smem_bytes = the dynamic shared memory
+ * per CTA of those launches (without stress tracking).  May wait for the
+ * stream.  Either pointer may be NULL.  No reference counterpart. */
 MB_API mb_status mb_get_step_variant(const mb_context* ctx, uint32_t* register_rows, uint32_t* smem_bytes);
 
 /* The packed spring slots of the uploaded batch, in device order: *count =
@@ -437,6 +437,12 @@ MB_API mb_status mb_surrogate_train_step(mb_surrogate* s, const uint8_t* genomes
  * bytes of device memory and synchronises.
  * -------------------------------------------------------------------- */
 MB_API mb_status mb_measure_smem_bandwidth(int device, double* bytes_per_s, double* bytes_per_clk_sm);
+
+/* Compares the step kernels' length and reciprocal of a spring with the
+ * correctly rounded square root and reciprocal for every non-negative float;
+ * *mismatches = the number of inputs where they differ (0 expected).
+ * Synchronous.  No reference counterpart. */
+MB_API mb_status mb_check_spring_math(int device, uint64_t* mismatches);
 
 /* Library version string. */
 MB_API const char* mb_version(void);

@@ -137,6 +137,7 @@ def _load() -> ctypes.CDLL:
         "mb_surrogate_set_weight_decay": (I32, [P, F32]),
         "mb_surrogate_use_tcgen05": (I32, [P, I32]),
         "mb_measure_smem_bandwidth": (I32, [I32, ctypes.POINTER(ctypes.c_double), ctypes.POINTER(ctypes.c_double)]),
+        "mb_check_spring_math": (I32, [I32, ctypes.POINTER(ctypes.c_uint64)]),
         "mb_version": (ctypes.c_char_p, []),
     }
     for name, (res, args) in sigs.items():

@@ -35,6 +35,7 @@
 #include "mb_devo.h"
 #include "mb_internal.h"
 #include "mb_pack.h"
+#include "mb_tm.h"
 #include "mb_voxel.h"
 #include "mb_voxel_dev.h"
 
@@ -122,9 +123,21 @@ struct mb_context {
     mb::KernelShape shape{512, 8, 2};
     uint32_t n_bins = 0;
     uint32_t max_bin_mass = 0;  // most (own) masses in one bin
-    uint32_t rr_smem = 0;       // shared memory of the register-row kernel over every bin
+    // resident bins on the tensor-memory step kernel (mb_tm.h): the rows it
+    // reads, built on the device before the first step after the packed rows
+    // changed, and the launch plan without and with stress tracking
+    struct TmLaunch {
+        mb::TmPlan plan;
+        bool planned = false;
+        size_t groups = 0, bins = 0;  // bytes into `arrays`
+        mb::DevBuf<uint8_t> arrays;
+    } tm[2];
+    bool tm_stale = true;
+    uint32_t n_slices = 0;
+    mb::TmRows tm_rows{};          // into tm_arena
+    mb::DevBuf<uint8_t> tm_arena;
+    std::vector<uint32_t> tm_slots;  // per bin: correction slots
     uint32_t max_degree = 0;    // most springs at one mass when uploaded
-    uint32_t smem_optin = 0;    // the device's shared memory per CTA (opt-in)
     uint32_t grid = 0;  // CTAs per step launch (0 = one per bin)
     uint32_t chunk = 1000;
     bool use_graph = true;
@@ -278,7 +291,9 @@ mb_status cuda_fail(mb_context* c, cudaError_t e, const char* what) {
 
 namespace mb_detail {
 
-uint32_t row_reg_smem(const mb_context* c);
+bool tm_eligible(const mb_context* c);
+bool use_tm(const mb_context* c, bool track);
+cudaError_t tm_update(mb_context* c, bool track);
 
 // Whether the step applies the face drag (water mode, rho != 0): split
 // robots are then packed with their faces (velocities exchanged with the
@@ -329,15 +344,9 @@ mb_status upload_packed(mb_context* ctx, const mb::Packed& out, bool* rows_faile
     ctx->shape = out.shape;
     ctx->n_bins = out.n_bins;
     ctx->grid = out.grid;
-    // the register-row kernel's layout: the usual one without the rows, 8
-    // bytes of alignment, 8 bytes per spring (mb::row_reg_supported)
-    ctx->max_bin_mass = ctx->rr_smem = 0;
+    ctx->max_bin_mass = 0;
     ctx->max_degree = out.max_degree;
-    for (const mb::BinDesc& d : out.bins) {
-        ctx->max_bin_mass = std::max(ctx->max_bin_mass, d.n_mass);
-        ctx->rr_smem = std::max(ctx->rr_smem, mb::bin_smem_bytes(d.n_mass, d.n_spring, 0) + 8u + 8u * d.n_spring);
-    }
-    if (!ctx->smem_optin) ctx->smem_optin = mb::max_step_smem(ctx->device);
+    for (const mb::BinDesc& d : out.bins) ctx->max_bin_mass = std::max(ctx->max_bin_mass, d.n_mass);
     ctx->smem_bytes = out.max_smem;
     ctx->streamed = out.streamed;
     ctx->cluster = out.cluster;
@@ -480,6 +489,8 @@ mb_status upload_packed(mb_context* ctx, const mb::Packed& out, bool* rows_faile
         }
         ctx->smem_bytes = status[1];  // the largest bin's need, exactly
     }
+    ctx->tm_stale = true;
+    ctx->n_slices = (uint32_t)out.slice_off.size();
     // the host vectors of `out` may die after this call: wait for the copies
     MB_CUDA(ctx, cudaStreamSynchronize(st));
     return MB_OK;
@@ -758,6 +769,7 @@ mb_status devo_setup(mb_context* c) {
     MB_CUDA(c, up(c->bins, c->h_bins.data(), nb));
     MB_CUDA(c, cudaStreamSynchronize(st));
     c->clear_graphs();
+    c->tm_stale = true;
     c->devo_ready = true;
     return MB_OK;
 }
@@ -1052,9 +1064,12 @@ mb_status mb_get_launch_config(const mb_context* ctx, mb_launch_config* cfg) {
 mb_status mb_get_step_variant(const mb_context* ctx, uint32_t* register_rows, uint32_t* smem_bytes) {
     if (!ctx) return MB_ERR_ARGUMENT;
     if (!ctx->loaded) return MB_ERR_STATE;
-    const uint32_t rr = mb_detail::row_reg_smem(ctx);
-    if (register_rows) *register_rows = rr ? 1u : 0u;
-    if (smem_bytes) *smem_bytes = rr ? rr : ctx->smem_bytes;
+    cudaSetDevice(ctx->device);
+    // (the launch plan is made on demand; it is not part of the caller's state)
+    if (mb_detail::tm_eligible(ctx) && mb_detail::tm_update(const_cast<mb_context*>(ctx), false) != cudaSuccess) return MB_ERR_CUDA;
+    const bool tm = mb_detail::use_tm(ctx, false);
+    if (register_rows) *register_rows = tm ? 1u : 0u;
+    if (smem_bytes) *smem_bytes = tm ? ctx->tm[0].plan.smem : ctx->smem_bytes;
     return MB_OK;
 }
 
@@ -1268,20 +1283,82 @@ mb_status mb_set_state(mb_context* ctx, const float* pos, const float* vel) {
 // Internal helpers: C++ linkage, internal to this file.
 namespace mb_detail {
 
-// Shared memory of the register-row step kernel, or 0 when it does not
-// apply: streamed or split bins, a bin of more than one mass per thread, a
-// mass with more springs than the registers hold rows for (at upload: the
-// kernel stays correct when development adds springs, reading longer rows
-// from global memory), face drag, a shape without the variant, or too little
-// shared memory.  Device development of resident bins keeps every bin's
-// spring count, and the device voxel builder only removes springs, so the
-// planned bins bound the need.
-uint32_t row_reg_smem(const mb_context* c) {
+// Whether the tensor-memory kernel holds the population: resident bins of a
+// 1,024-thread shape with at most one mass per thread, no mass with more
+// springs than a lattice has when uploaded (the kernel stays correct when
+// development adds some, reading longer rows from global memory), and no
+// face drag.
+bool tm_eligible(const mb_context* c) {
     const bool faces = face_drag_on(c) && c->faces_packed;
-    if (c->streamed || c->cluster || faces || !mb::row_reg_supported(c->shape) ||
-        c->max_bin_mass > c->shape.threads || c->max_degree > mb::row_reg_width())
-        return 0;
-    return c->rr_smem <= c->smem_optin ? c->rr_smem : 0u;
+    return !c->streamed && !c->cluster && !faces && mb::tm_shape(c->shape) &&
+           c->max_bin_mass <= c->shape.threads && c->max_degree <= mb::kTmMaxDegree;
+}
+
+// The rows of the tensor-memory kernel, when the packed rows changed (waits
+// for the stream), and its launch plan.
+cudaError_t tm_update(mb_context* c, bool track) {
+    cudaError_t e = cudaSuccess;
+    if (c->tm_stale) {
+        // one allocation for all arrays
+        const size_t n = c->inc.n + 32ull * c->n_slices;
+        size_t bytes = 0;
+        auto carve = [&](size_t count, size_t size) {
+            const size_t at = bytes;
+            bytes += (count * size + 255) & ~size_t(255);
+            return at;
+        };
+        const size_t own = carve(n, 8), gidx = carve(n, 4), gather = carve(n, 4), head = carve(c->n_slices, 16),
+                     slots = carve(c->n_bins, 4), n_mat = carve(c->n_bins, 4), mat = carve(c->n_bins, 256),
+                     col = carve(c->n_packed, 2);
+        e = c->tm_arena.alloc(bytes);
+        if (e != cudaSuccess) return e;
+        uint8_t* p = c->tm_arena.p;
+        c->tm_rows = mb::TmRows{reinterpret_cast<uint2*>(p + own),      reinterpret_cast<uint32_t*>(p + gidx),
+                                reinterpret_cast<uint32_t*>(p + gather), reinterpret_cast<uint4*>(p + head),
+                                reinterpret_cast<uint32_t*>(p + slots),  reinterpret_cast<uint32_t*>(p + n_mat),
+                                p + mat,                                 reinterpret_cast<uint16_t*>(p + col)};
+        const mb::TmSource in{c->bins.p,        c->n_bins,  c->spring_pair.p, c->spring_lbar.p,
+                              c->spring_gidx.p, c->inc.p,   c->slice_off.p,   c->slice_width.p};
+        e = mb::launch_tm_rows(in, c->tm_rows, c->stream);
+        c->tm_slots.resize(c->n_bins);
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(c->tm_slots.data(), c->tm_rows.n_slots, c->n_bins * sizeof(uint32_t),
+                                cudaMemcpyDeviceToHost, c->stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+        if (e != cudaSuccess) return e;
+        c->clear_graphs();  // they hold the old rows and plan
+        c->tm_stale = c->tm[0].planned = c->tm[1].planned = false;
+    }
+    mb_context::TmLaunch& l = c->tm[track ? 1 : 0];
+    if (l.planned) return cudaSuccess;
+    // stresses add to a thread's words: one mass per thread then
+    mb::tm_plan(c->h_bins, c->tm_slots, c->grid ? c->grid : c->n_bins, c->n_mat_host, mb::max_step_smem(c->device),
+                track ? 1u : mb::kTmMaxMpt, l.plan);
+    if (l.plan.ok) {
+        std::vector<uint8_t> host;
+        auto put = [&](const auto& v) {
+            const size_t at = (host.size() + 15) & ~size_t(15), n = v.size() * sizeof(v[0]);
+            host.resize(at + n);
+            std::memcpy(host.data() + at, v.data(), n);
+            return at;
+        };
+        l.groups = put(l.plan.groups);
+        l.bins = put(l.plan.bins);
+        const uint8_t* old = l.arrays.p;
+        e = l.arrays.alloc(host.size());
+        if (l.arrays.p != old) c->clear_graphs();
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(l.arrays.p, host.data(), host.size(), cudaMemcpyHostToDevice, c->stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);  // `host` dies here
+    }
+    l.planned = e == cudaSuccess;
+    return e;
+}
+
+// Whether the next steps run on it (after tm_update).
+bool use_tm(const mb_context* c, bool track) {
+    const mb_context::TmLaunch& l = c->tm[track ? 1 : 0];
+    return tm_eligible(c) && !c->tm_stale && l.planned && l.plan.ok;
 }
 
 mb::StepParams make_params(mb_context* c, float t0, uint32_t steps, bool track) {
@@ -1304,6 +1381,8 @@ mb::StepParams make_params(mb_context* c, float t0, uint32_t steps, bool track) 
     p.invk = c->invk.p;
     p.bin_flags = c->bin_flags.p;
     p.dt = c->dt;
+    p.inv_dt = 1.0 / (double)c->dt;
+    p.inv_dt_f = 1.0f / c->dt;
     p.t0 = t0;
     p.steps = steps;
     p.track = track ? 1u : 0u;
@@ -1325,11 +1404,23 @@ mb::StepParams make_params(mb_context* c, float t0, uint32_t steps, bool track) 
     p.fd = c->fd_scratch.p;
     p.face_coef = (float)(-(double)c->env.face_drag / 6.0);
     p.face_on = c->mode == MB_MODE_FORCE_WATER && c->env.face_drag != 0.0f && c->faces_packed ? 1u : 0u;
-    if (const uint32_t rr = row_reg_smem(c)) {
-        p.one_mass_per_thread = 1u;
-        p.smem_bytes = rr;
-    }
     return p;
+}
+
+cudaError_t launch_tm_steps(mb_context* c, const mb::StepParams& p) {
+    const mb_context::TmLaunch& l = c->tm[p.track ? 1 : 0];
+    const mb::TmParams q{p, reinterpret_cast<const mb::TmGroup*>(l.arrays.p + l.groups),
+                         reinterpret_cast<const mb::TmBinRef*>(l.arrays.p + l.bins), c->tm_rows};
+    return mb::launch_tm(q, l.plan, c->stream);
+}
+
+// Kernel attributes of the next launches (they cannot change inside a capture).
+cudaError_t prepare_launch(mb_context* c, bool track) {
+    const uint32_t mode = (uint32_t)c->mode;
+    if (c->streamed) return mb::prepare_stream(1024, c->stream_mpt, mode, track, c->smem_bytes);
+    if (c->cluster) return mb::prepare_split(c->shape, mode, track, c->smem_bytes);
+    if (use_tm(c, track)) return mb::prepare_tm(mode, track, c->tm[track ? 1 : 0].plan);
+    return mb::prepare_step(c->shape, mode, track, c->smem_bytes);
 }
 
 // Float clock after `n` steps from t (Simulator.cu:447).
@@ -1372,6 +1463,7 @@ cudaError_t issue_chunks(mb_context* c, float t0, uint32_t steps, bool track) {
         mb::StepParams p = make_params(c, t, n, track);
         cudaError_t e = c->streamed  ? mb::launch_stream(p, 1024, c->stream_mpt, c->stream)
                         : c->cluster ? launch_split_groups(c, p)
+                        : use_tm(c, track) ? launch_tm_steps(c, p)
                                      : mb::launch_step(p, c->shape, c->stream);
         if (e != cudaSuccess) return e;
         t = advance(t, c->dt, n);
@@ -1390,6 +1482,7 @@ mb_status run(mb_context* c, uint32_t steps, bool track) {
         if (!c->faces_packed) return fail(c, MB_ERR_CAPACITY, "face drag: the faces do not fit the step kernels");
     }
     cudaSetDevice(c->device);
+    if (tm_eligible(c)) MB_CUDA(c, tm_update(c, track));
     const float t0 = c->total_time;
     if (c->use_graph) {
         uint32_t bits;
@@ -1398,11 +1491,7 @@ mb_status run(mb_context* c, uint32_t steps, bool track) {
         auto it = c->graphs.find(key);
         if (it == c->graphs.end()) {
             if (c->graphs.size() >= 16) c->clear_graphs();
-            // kernel attributes cannot change inside a capture
-            MB_CUDA(c, c->streamed ? mb::prepare_stream(1024, c->stream_mpt, (uint32_t)c->mode, track, c->smem_bytes)
-                                    : c->cluster ? mb::prepare_split(c->shape, (uint32_t)c->mode, track, c->smem_bytes)
-                                    : mb::prepare_step(c->shape, (uint32_t)c->mode, track,
-                                                       std::max(c->smem_bytes, row_reg_smem(c))));
+            MB_CUDA(c, prepare_launch(c, track));
             cudaGraph_t g;
             MB_CUDA(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
             cudaError_t e = issue_chunks(c, t0, steps, track);
@@ -1420,10 +1509,7 @@ mb_status run(mb_context* c, uint32_t steps, bool track) {
         }
         MB_CUDA(c, cudaGraphLaunch(it->second, c->stream));
     } else {
-        MB_CUDA(c, c->streamed ? mb::prepare_stream(1024, c->stream_mpt, (uint32_t)c->mode, track, c->smem_bytes)
-                                    : c->cluster ? mb::prepare_split(c->shape, (uint32_t)c->mode, track, c->smem_bytes)
-                                    : mb::prepare_step(c->shape, (uint32_t)c->mode, track,
-                                                       std::max(c->smem_bytes, row_reg_smem(c))));
+        MB_CUDA(c, prepare_launch(c, track));
         cudaError_t e = issue_chunks(c, t0, steps, track);
         if (e != cudaSuccess) return cuda_fail(c, e, "step launch");
     }
@@ -1586,6 +1672,7 @@ mb_status mb_devo(mb_context* ctx, uint32_t replaced_per_robot, uint64_t seed, u
                              ctx->streamed ? 1u : 0u, ctx->rows_scratch.p, ctx->free_count.p,
                              ctx->free_taken.p,  ctx->devo_status.p};
         MB_CUDA(ctx, mb::launch_rebuild(rp, st));
+        ctx->tm_stale = true;
         MB_CUDA(ctx, cudaMemcpyAsync(status, ctx->devo_status.p, sizeof(status), cudaMemcpyDeviceToHost, st));
     }
     ctx->h_devo.resize(nrec);
@@ -1684,6 +1771,7 @@ mb_status mb_set_voxel_population(mb_context* ctx, uint32_t n_robots, int sx, in
     uint32_t status[2] = {0, 0};
     MB_CUDA(ctx, cudaMemcpyAsync(status, ctx->devo_status.p, sizeof(status), cudaMemcpyDeviceToHost, st));
     MB_CUDA(ctx, cudaStreamSynchronize(st));
+    ctx->tm_stale = true;
     ctx->host_topology_stale = true;
     ctx->vox_live = true;
     ctx->devo_ready = false;

@@ -64,6 +64,8 @@ struct StepParams {
     const float* rates;           // [steps][n_mat]: dL0 * sin(omega t_n + phi) of this launch
     const float* invk;            // [n_mat]: 1 / (2 + 1/(k dt^2))
     uint32_t* bin_flags;          // per bin: bit 0 = non-finite position
+    double inv_dt;                // RN(1/dt) in double
+    float inv_dt_f;               // and in float
     float dt;
     float t0;
     uint32_t steps;
@@ -88,7 +90,6 @@ struct StepParams {
     float4* fd;                   // streamed kernel: face forces of the current step
     float face_coef;              // -rho/6: -rho/2 of the face law and the 1/3 per corner
     uint32_t face_on;             // face drag active (water mode, rho != 0)
-    uint32_t one_mass_per_thread; // every bin has at most 1,024 masses (0 = unknown)
 };
 
 enum StepMode : uint32_t { kModeXpbd = 0, kModeForceLand = 1, kModeForceWater = 2 };
@@ -189,15 +190,6 @@ uint32_t max_step_smem(int device);
 
 // Whether a kernel shape is compiled in.
 bool shape_supported(const KernelShape& shape);
-// Whether the shape of resident bins has a register-row twin (one mass per
-// thread, rows of incident springs in registers), which launch_step uses
-// when StepParams::one_mass_per_thread is set.  Its shared memory per bin:
-// the usual layout without the rows, 8 bytes of alignment, then 8 bytes per
-// spring.  Rows longer than row_reg_width() entries are read from global
-// memory, so the host uses it only when no mass has more incident springs.
-bool row_reg_supported(const KernelShape& shape);
-uint32_t row_reg_width();
-
 // Centre of mass of the non-air masses of each robot: one warp per robot.
 cudaError_t launch_com(const float4* pos, const uint8_t* mass_mat,
                        const int64_t* mass_off, uint32_t n_robots, float* com,

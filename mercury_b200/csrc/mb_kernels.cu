@@ -26,6 +26,7 @@
 
 #include "mb_internal.h"
 #include "mb_sin.cuh"
+#include "mb_step_math.cuh"
 
 namespace mb {
 
@@ -33,140 +34,15 @@ namespace cg = cooperative_groups;
 
 namespace {
 
-constexpr float kEps = 1e-12f;  // sim_kernel.cu:6
-
 // Packed spring word: a (12 bits) | b << 12 (12 bits) | slot << 24 (8 bits).
 __device__ __forceinline__ uint32_t pk_a(uint32_t w) { return w & 0xFFFu; }
 __device__ __forceinline__ uint32_t pk_b(uint32_t w) { return (w >> 12) & 0xFFFu; }
 __device__ __forceinline__ uint32_t pk_slot(uint32_t w) { return w >> 24; }
 
-// Force modes, per mass, after the spring forces (fx, fy, fz) are gathered:
-// environment forces, then x' = x + v dt + (F/m) dt^2, v' = damping (x' - x)/dt.
-//   land : gravity -m g along z; below z = 0 a penalty normal force
-//          fn = k_floor (-z) and Coulomb friction on the horizontal velocity
-//          h = v + (F_h/m) dt the step would reach: static (the friction force
-//          cancels the horizontal motion, F_h = -m v_h/dt) when |h| <= mu_s fn
-//          dt/m, else kinetic, mu_k fn against h.
-//   water: gravity balanced by buoyancy; quadratic drag -drag |v| v.
-// Divisions by m and dt are multiplications by the correctly rounded
-// reciprocals (inv_dt = RN(1/dt) per launch, RN(1/m) per mass and step);
-// only the kinetic friction divides.
-template <int MODE>
-__device__ __forceinline__ void force_integrate(const StepParams& p, float3& x, float3& v, float m,
-                                                float inv_dt, float fx, float fy, float fz) {
-    const float dt = p.dt;
-    const float inv_m = __frcp_rn(m);
-    if (MODE == kModeForceLand) {
-        fz = __fsub_rn(fz, __fmul_rn(m, p.g));
-        if (x.z < 0.0f) {
-            const float fn = __fmul_rn(p.floor_stiffness, -x.z);
-            fz = __fadd_rn(fz, fn);
-            const float hx = __fadd_rn(v.x, __fmul_rn(__fmul_rn(fx, inv_m), dt));
-            const float hy = __fadd_rn(v.y, __fmul_rn(__fmul_rn(fy, inv_m), dt));
-            const float hs = __fsqrt_rn(__fmaf_rn(hx, hx, __fmul_rn(hy, hy)));
-            const float budget = __fmul_rn(__fmul_rn(fn, inv_m), dt);
-            if (hs <= __fmul_rn(p.mu_s, budget)) {
-                fx = __fmul_rn(__fmul_rn(-m, v.x), inv_dt);
-                fy = __fmul_rn(__fmul_rn(-m, v.y), inv_dt);
-            } else {
-                const float s = __fdiv_rn(__fmul_rn(p.mu_k, fn), hs);
-                fx = __fsub_rn(fx, __fmul_rn(s, hx));
-                fy = __fsub_rn(fy, __fmul_rn(s, hy));
-            }
-        }
-    } else {
-        const float sp = __fsqrt_rn(__fmaf_rn(v.x, v.x, __fmaf_rn(v.y, v.y, __fmul_rn(v.z, v.z))));
-        const float c = __fmul_rn(p.drag, sp);
-        fx = __fsub_rn(fx, __fmul_rn(c, v.x));
-        fy = __fsub_rn(fy, __fmul_rn(c, v.y));
-        fz = __fsub_rn(fz, __fmul_rn(c, v.z));
-    }
-    const float dt2 = __fmul_rn(dt, dt);
-    const float nx = __fadd_rn(__fadd_rn(x.x, __fmul_rn(v.x, dt)), __fmul_rn(__fmul_rn(fx, inv_m), dt2));
-    const float ny = __fadd_rn(__fadd_rn(x.y, __fmul_rn(v.y, dt)), __fmul_rn(__fmul_rn(fy, inv_m), dt2));
-    const float nz = __fadd_rn(__fadd_rn(x.z, __fmul_rn(v.z, dt)), __fmul_rn(__fmul_rn(fz, inv_m), dt2));
-    v.x = __fmul_rn(p.damping, __fmul_rn(__fsub_rn(nx, x.x), inv_dt));
-    v.y = __fmul_rn(p.damping, __fmul_rn(__fsub_rn(ny, x.y), inv_dt));
-    v.z = __fmul_rn(p.damping, __fmul_rn(__fsub_rn(nz, x.z), inv_dt));
-    x = make_float3(nx, ny, nz);
-}
-
-// Velocity of the reference step, v = (float)(0.99 * (double)delta / (double)dt)
-// (sim_kernel.cu:265-267): the double product, the correctly rounded double
-// quotient, then rounding to float -- without a double division in the
-// common case.  q = RN(a * inv_dt), with inv_dt = RN(1/dt), differs from
-// the exact a/dt by at most 2u + u^2 relative (u = 2^-53), so from the
-// correctly rounded quotient by less than 3.01 units in the last place of
-// q.  Rounding to float can only differ between q and that quotient if a
-// float rounding boundary -- the midpoint between two floats, whose low 29
-// significand bits are 1 << 28 in double -- lies between them.  So when
-// q's low 29 bits are more than 4 units from 1 << 28 and q lies in the
-// normal float range, (float)q is the result (Ziv's rounding test: Ziv,
-// "Fast evaluation of elementary mathematical functions with correctly
-// rounded last bit", ACM TOMS 17(3), 1991); otherwise -- about 9 inputs in
-// 2^29, zeros excepted -- the division itself is done.
-__device__ __forceinline__ float velocity_of(float delta, double dt, double inv_dt) {
-    const double a = __dmul_rn(0.99, (double)delta);
-    const double q = __dmul_rn(a, inv_dt);
-    const unsigned long long bits = (unsigned long long)__double_as_longlong(q);
-    const uint32_t e = (uint32_t)(bits >> 52) & 0x7FFu;
-    const uint32_t low29 = (uint32_t)bits & 0x1FFFFFFFu;
-    // normal float range 2^-126 <= |q| < 2^127 (biased double exponents 897..1149)
-    const bool clear = (e - 897u) < 253u && (low29 - (0x10000000u - 4u)) > 8u;
-    if (clear || (bits << 1) == 0) return __double2float_rn(q);
-    return __double2float_rn(__ddiv_rn(a, dt));
-}
-
-// Face drag of one surface triangle (water), the share of each corner:
-// mean corner velocity v = (v0 + v1 + v2) * RN(1/3), N = (x1 - x0) x (x2 - x0), A = |N|, unit normal
-// n = N * RN(1/(A + eps)) turned so that v.n > 0 (sim_kernel.cu:106-109),
-// force coef * A * ((v.n) v + 0.2 |v|^2 n) with coef = -rho/6, i.e.
-// -rho/2 A (...) / 3 (sim_kernel.cu:110-111).  Every operation rounds once,
-// in this order.
-__device__ __forceinline__ float4 face_force(const float4 x0, const float4 x1, const float4 x2, const float4 v0,
-                                             const float4 v1, const float4 v2, const float coef) {
-    constexpr float kThird = 0x1.555556p-2f;  // 1/3 rounded to nearest
-    const float vx = __fmul_rn(__fadd_rn(__fadd_rn(v0.x, v1.x), v2.x), kThird);
-    const float vy = __fmul_rn(__fadd_rn(__fadd_rn(v0.y, v1.y), v2.y), kThird);
-    const float vz = __fmul_rn(__fadd_rn(__fadd_rn(v0.z, v1.z), v2.z), kThird);
-    const float ax = __fsub_rn(x1.x, x0.x), ay = __fsub_rn(x1.y, x0.y), az = __fsub_rn(x1.z, x0.z);
-    const float bx = __fsub_rn(x2.x, x0.x), by = __fsub_rn(x2.y, x0.y), bz = __fsub_rn(x2.z, x0.z);
-    const float nx = __fsub_rn(__fmul_rn(ay, bz), __fmul_rn(az, by));
-    const float ny = __fsub_rn(__fmul_rn(az, bx), __fmul_rn(ax, bz));
-    const float nz = __fsub_rn(__fmul_rn(ax, by), __fmul_rn(ay, bx));
-    const float area = __fsqrt_rn(__fmaf_rn(nx, nx, __fmaf_rn(ny, ny, __fmul_rn(nz, nz))));
-    const float r = __frcp_rn(__fadd_rn(area, kEps));
-    float ux = __fmul_rn(nx, r), uy = __fmul_rn(ny, r), uz = __fmul_rn(nz, r);
-    float vn = __fmaf_rn(ux, vx, __fmaf_rn(uy, vy, __fmul_rn(uz, vz)));
-    if (!(vn > 0.0f)) {  // negating n negates the rounded dot product exactly
-        ux = -ux;
-        uy = -uy;
-        uz = -uz;
-        vn = -vn;
-    }
-    const float lift = __fmul_rn(0.2f, __fmaf_rn(vx, vx, __fmaf_rn(vy, vy, __fmul_rn(vz, vz))));
-    const float c = __fmul_rn(coef, area);
-    return make_float4(__fmul_rn(c, __fmaf_rn(lift, ux, __fmul_rn(vn, vx))),
-                       __fmul_rn(c, __fmaf_rn(lift, uy, __fmul_rn(vn, vy))),
-                       __fmul_rn(c, __fmaf_rn(lift, uz, __fmul_rn(vn, vz))), 0.0f);
-}
-
-// RW > 0 (register rows): each thread's row of up to RW entries is kept in
-// registers (two 16-bit entries per register, loaded once per bin), so that
-// the gather's correction loads no longer wait on a row-entry load and
-// issue RG at a time; a slice wider than RW reads its row from global
-// memory.  The rows are not staged in shared memory; to make room, the
-// springs leave the registers for {packed word, mean length} pairs in
-// shared memory where the rows would start (8 bytes per spring in place of
-// 2 per row entry).  One mass per thread (MPT = 1), no face drag.  Same
-// operations in the same order: same bits.  Resident bins only: on the
-// parts of split robots it measured slower.
-template <int T, int SPT, int MPT, int MODE, bool TRACK, bool SPLIT, int RW = 0>
+template <int T, int SPT, int MPT, int MODE, bool TRACK, bool SPLIT>
 __global__ void __launch_bounds__(T, 1024 / T) step_kernel(const StepParams p) {
     constexpr bool XPBD = MODE == kModeXpbd;
     constexpr bool FACES = MODE == kModeForceWaterFaces;  // face drag compiled in
-    constexpr int RG = 2;  // correction loads in flight per group
-    static_assert(RW == 0 || (MPT == 1 && !SPLIT && !FACES && RW % RG == 0), "register rows: one mass per thread");
     extern __shared__ float4 smem4[];
     const int tid = threadIdx.x;
     const float dt = p.dt;
@@ -200,26 +76,7 @@ __global__ void __launch_bounds__(T, 1024 / T) step_kernel(const StepParams p) {
         uint16_t* sfinc = reinterpret_cast<uint16_t*>(sfrow + bd.n_mass);
 
         const uint32_t n_mat = *p.n_mat;
-        // register rows: the rows are not staged in shared memory; the springs
-        // leave the registers to make room, into {packed word, mean length}
-        // pairs where the rows would start (8-byte aligned)
-        uint2* ssl = reinterpret_cast<uint2*>((reinterpret_cast<uintptr_t>(sinc) + 7u) & ~uintptr_t(7));
-        if (RW > 0) {
-            // the host sizes the launch for every bin; a bin that would still
-            // not fit is skipped and flagged (bit 1) rather than overrun
-            uint32_t dyn;
-            asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn));
-            if (reinterpret_cast<const char*>(ssl + bd.n_spring) - reinterpret_cast<const char*>(smem4) > dyn) {
-                if (tid == 0) atomicOr(&p.bin_flags[b], 2u);
-                continue;
-            }
-        }
-        if (RW > 0)
-            for (uint32_t i = tid; i < bd.n_spring; i += T)
-                ssl[i] = make_uint2(__ldg(&p.spring_pair[bd.spring_begin + i]),
-                                    __float_as_uint(__ldg(&p.spring_lbar[bd.spring_begin + i])));
-        else
-            for (uint32_t i = tid; i < bd.n_inc; i += T) sinc[i] = __ldg(&p.inc[bd.inc_begin + i]);
+        for (uint32_t i = tid; i < bd.n_inc; i += T) sinc[i] = __ldg(&p.inc[bd.inc_begin + i]);
         if (n_face) {
             for (uint32_t i = tid; i < n_face; i += T) sface[i] = __ldg(&p.faces[bd.face_begin + i]);
             for (uint32_t i = tid; i < bd.n_mass; i += T) sfrow[i] = __ldg(&p.face_row[bd.mass_begin + i]);
@@ -247,10 +104,8 @@ __global__ void __launch_bounds__(T, 1024 / T) step_kernel(const StepParams p) {
             st[j] = 0.0f;
             if (s < bd.n_spring) {
                 const uint32_t g = bd.spring_begin + s;
-                if (RW == 0) {
-                    sw[j] = __ldg(&p.spring_pair[g]);
-                    lb[j] = __ldg(&p.spring_lbar[g]);
-                }
+                sw[j] = __ldg(&p.spring_pair[g]);
+                lb[j] = __ldg(&p.spring_lbar[g]);
                 if (TRACK) st[j] = p.stress[__ldg(&p.spring_gidx[g]) & 0x7FFFFFFFu];
             }
         }
@@ -273,18 +128,6 @@ __global__ void __launch_bounds__(T, 1024 / T) step_kernel(const StepParams p) {
                 v[j] = make_float3(V.x, V.y, V.z);
                 const uint32_t sl = bd.slice_begin + m / kSliceWidth;
                 row[j] = (__ldg(&p.slice_off[sl]) + (m % kSliceWidth)) | (__ldg(&p.slice_width[sl]) << 20);
-            }
-        }
-        // register rows: entry k of this thread's mass in half k & 1 of rr[k / 2]
-        uint32_t rr[RW > 0 ? RW / 2 : 1];
-        if constexpr (RW > 0) {
-            const uint32_t w = row[0] >> 20;
-            const uint16_t* gp = p.inc + bd.inc_begin + (row[0] & 0xFFFFFu);
-#pragma unroll
-            for (int k = 0; k < RW; k += 2) {
-                const uint32_t lo = (uint32_t)k < w ? (uint32_t)__ldg(gp + k * kSliceWidth) : kPadEntry;
-                const uint32_t hi = (uint32_t)k + 1u < w ? (uint32_t)__ldg(gp + (k + 1) * kSliceWidth) : kPadEntry;
-                rr[k / 2] = lo | hi << 16;
             }
         }
         if (SPLIT)
@@ -337,11 +180,10 @@ __global__ void __launch_bounds__(T, 1024 / T) step_kernel(const StepParams p) {
             for (int j = 0; j < SPT; ++j) {
                 const uint32_t s = tid + j * T;
                 if (s >= bd.n_spring) break;
-                const uint2 q = RW > 0 ? ssl[s] : make_uint2(sw[j], __float_as_uint(lb[j]));
-                const uint32_t wj = q.x;
+                const uint32_t wj = sw[j];
                 const float4 pa = X[pk_a(wj)], pb = X[pk_b(wj)];
                 const float2 mt = smat[pk_slot(wj)];
-                const float lbj = __uint_as_float(q.y);
+                const float lbj = lb[j];
                 const float L = __fmaf_rn(lbj, mt.x, lbj);
                 const float dx = __fsub_rn(pa.x, pb.x);
                 const float dy = __fsub_rn(pa.y, pb.y);
@@ -373,33 +215,8 @@ __global__ void __launch_bounds__(T, 1024 / T) step_kernel(const StepParams p) {
                 float ax = 0.0f, ay = 0.0f, az = 0.0f;
                 const uint16_t* rp = sinc + (row[j] & 0xFFFFFu);
                 const uint32_t w = row[j] >> 20;  // the same for the warp (one slice)
-                if (RW > 0 && w <= (uint32_t)RW) {
-                    // entries in [w, RW) are padding; a padding entry adds a
-                    // zero (acc + -0 == acc: a sum that starts at +0 is never -0)
-#pragma unroll
-                    for (int k0 = 0; k0 < RW; k0 += RG) {
-                        if ((uint32_t)k0 >= w) break;
-                        float4 c[RG];
-                        float sg[RG];
-#pragma unroll
-                        for (int u = 0; u < RG; ++u) {
-                            const int k = k0 + u;
-                            const uint32_t e = (k & 1) ? rr[k / 2] >> 16 : rr[k / 2] & 0xFFFFu;
-                            c[u] = e != kPadEntry ? sdp[e >> 1] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                            sg[u] = __uint_as_float(0x3f800000u | ((e & 1u) << 31));
-                        }
-#pragma unroll
-                        for (int u = 0; u < RG; ++u) {
-                            ax = __fmaf_rn(c[u].x, sg[u], ax);
-                            ay = __fmaf_rn(c[u].y, sg[u], ay);
-                            az = __fmaf_rn(c[u].z, sg[u], az);
-                        }
-                    }
-                } else
                 for (uint32_t k = 0; k < w; ++k) {
-                    // (register rows: a slice wider than RW reads its row from global memory)
-                    const uint32_t e = RW > 0 ? __ldg(p.inc + bd.inc_begin + (row[j] & 0xFFFFFu) + k * kSliceWidth)
-                                              : rp[k * kSliceWidth];
+                    const uint32_t e = rp[k * kSliceWidth];
                     if (e != kPadEntry) {
                         const float4 c = sdp[e >> 1];
                         const float sg = __uint_as_float(0x3f800000u | ((e & 1u) << 31));
@@ -630,8 +447,8 @@ __global__ void __launch_bounds__(T, 1024 / T) stream_kernel(const StepParams p)
 
 // Actuation factors of one launch.  Block b covers steps [256 b, 256 b + 256):
 // thread 0 accumulates the float clock from t0 (the clock is a sequential
-// float sum, Simulator.cu:447, so it is not reassociated), then every thread
-// evaluates its step for every material.
+// float sum, Simulator.cu:447, so it is not reassociated), then the threads
+// share the steps' materials (4 steps of 10 materials: 5.4 -> 3.9 us).
 __global__ void __launch_bounds__(256) actuation_kernel(const float4* __restrict__ table,
                                                         const uint8_t* __restrict__ mat_ids,
                                                         const uint32_t* __restrict__ n_mat_ptr,
@@ -644,7 +461,8 @@ __global__ void __launch_bounds__(256) actuation_kernel(const float4* __restrict
     if (threadIdx.x == 0) {
         float t = t0;
         for (uint32_t i = 0; i < base; ++i) t = __fadd_rn(t, dt);
-        for (uint32_t i = 0; i < 256u; ++i) {
+        const uint32_t n = min(256u, steps - base);
+        for (uint32_t i = 0; i < n; ++i) {
             s_t[i] = t;
             t = __fadd_rn(t, dt);
         }
@@ -662,13 +480,13 @@ __global__ void __launch_bounds__(256) actuation_kernel(const float4* __restrict
         }
     }
     __syncthreads();
-    const uint32_t n = base + threadIdx.x;
-    if (n >= steps) return;
-    const float t = s_t[threadIdx.x];
-    for (uint32_t i = 0; i < n_mat; ++i) {
+    // the block's (step, material) pairs over its threads, materials first
+    const uint32_t pairs = min(256u, steps - base) * n_mat;
+    for (uint32_t k = threadIdx.x; k < pairs; k += 256u) {
+        const uint32_t n = k / n_mat, i = k - n * n_mat;
         const float4 mt = table[mat_ids[i]];
-        const float arg = __fmaf_rn(mt.z, t, mt.w);
-        rates[(size_t)n * n_mat + i] = __fmul_rn(mt.y, __double2float_rn(sin_cw((double)arg)));
+        const float arg = __fmaf_rn(mt.z, s_t[n], mt.w);
+        rates[(size_t)base * n_mat + k] = __fmul_rn(mt.y, __double2float_rn(sin_cw((double)arg)));
     }
 }
 
@@ -754,25 +572,6 @@ const ShapeEntry kShapes[] = {
     MB_SHAPE(512, 16, 4, false),  MB_SHAPE(1024, 4, 1, false),  MB_SHAPE(1024, 6, 2, false),
     MB_SHAPE(1024, 8, 2, false),  MB_SHAPE(1024, 10, 2, false), MB_SHAPE(1024, 12, 2, false),
 };
-// register-row twins of the 1,024-thread shapes (one mass per thread; no
-// face drag): launch_step uses one when the host marks the launch eligible
-// (StepParams::one_mass_per_thread)
-#define MB_RR(T, S, RW)                                                                          \
-    {                                                                                            \
-        T, S, 1, {                                                                               \
-            {step_kernel<T, S, 1, kModeXpbd, false, false, RW>,                                  \
-             step_kernel<T, S, 1, kModeXpbd, true, false, RW>},                                  \
-                {step_kernel<T, S, 1, kModeForceLand, false, false, RW>,                         \
-                 step_kernel<T, S, 1, kModeForceLand, true, false, RW>},                         \
-                {step_kernel<T, S, 1, kModeForceWater, false, false, RW>,                        \
-                 step_kernel<T, S, 1, kModeForceWater, true, false, RW>},                        \
-                {nullptr, nullptr},                                                              \
-        }                                                                                        \
-    }
-constexpr int kRowRegWidth = 26;  // register rows: entries per mass (lattice robots: at most 26)
-const ShapeEntry kRowRegShapes[] = {MB_RR(1024, 8, kRowRegWidth), MB_RR(1024, 10, kRowRegWidth),
-                                    MB_RR(1024, 12, kRowRegWidth)};
-#undef MB_RR
 // the parts of split robots (thread-block clusters)
 const ShapeEntry kSplitShapes[] = {
     MB_SHAPE(1024, 8, 1, true),
@@ -816,15 +615,6 @@ const ShapeEntry* find_shape(const KernelShape& s) {
     return nullptr;
 }
 
-// The register-row twin of a 1,024-thread shape, for the launches the host
-// marks eligible (no face drag).
-const ShapeEntry* find_row_reg(const KernelShape& s, const StepParams& p) {
-    if (s.threads != 1024 || !p.one_mass_per_thread || p.face_on) return nullptr;
-    for (const auto& e : kRowRegShapes)
-        if (e.spt == s.spt) return &e;
-    return nullptr;
-}
-
 const ShapeEntry* find_split(const KernelShape& s) {
     for (const auto& e : kSplitShapes)
         if (e.threads == s.threads && e.spt == s.spt && e.mpt == s.mpt) return &e;
@@ -844,15 +634,6 @@ uint32_t max_step_smem(int device) {
 }
 
 bool shape_supported(const KernelShape& shape) { return find_shape(shape) != nullptr; }
-
-bool row_reg_supported(const KernelShape& shape) {
-    if (shape.threads != 1024) return false;
-    for (const auto& e : kRowRegShapes)
-        if (e.spt == shape.spt) return true;
-    return false;
-}
-
-uint32_t row_reg_width() { return kRowRegWidth; }
 
 bool split_supported(const KernelShape& shape) { return find_split(shape) != nullptr; }
 
@@ -894,11 +675,6 @@ cudaError_t prepare_step(const KernelShape& shape, uint32_t mode, bool track, ui
     const ShapeEntry* e = find_shape(shape);
     if (!e || mode > kModeForceWater) return cudaErrorInvalidValue;
     cudaError_t r = cudaFuncSetAttribute(e->fn[mode][track ? 1 : 0], cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem_bytes);
-    if (shape.threads == 1024)  // the register-row twin, when there is one
-        for (const auto& t : kRowRegShapes)
-            if (r == cudaSuccess && t.spt == shape.spt)
-                r = cudaFuncSetAttribute(t.fn[mode][track ? 1 : 0], cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)smem_bytes);
     if (r == cudaSuccess && mode == kModeForceWater)  // and the face-drag variant
         r = cudaFuncSetAttribute(e->fn[kModeForceWaterFaces][track ? 1 : 0],
@@ -991,7 +767,6 @@ cudaError_t launch_step(const StepParams& p, const KernelShape& shape, cudaStrea
     if (p.mode > kModeForceWater) return cudaErrorInvalidValue;
     const uint32_t grid = p.grid ? std::min(p.grid, p.n_bins) : p.n_bins;
     const uint32_t variant = p.mode == kModeForceWater && p.face_on ? kModeForceWaterFaces : p.mode;
-    if (const ShapeEntry* rr = find_row_reg(shape, p)) e = rr;
     e->fn[variant][p.track ? 1 : 0]<<<grid, shape.threads, p.smem_bytes, s>>>(p);
     return cudaGetLastError();
 }

@@ -20,6 +20,7 @@
 // Robots are preprocessed and bins built in parallel over host threads; the
 // result does not depend on the number of threads.
 #include "mb_pack.h"
+#include "mb_tm.h"
 
 #include <algorithm>
 #include <tuple>
@@ -283,11 +284,8 @@ void preprocess(const mb_batch_desc* b, uint32_t r, RobotPack& p) {
 
 // LPT assignment of robots to `nb` bins by cost, within the shape's and the
 // shared memory's capacity.
-// spring_extra (the register-row kernel, when nonzero): the bin must also
-// fit that kernel's layout -- the usual one without the rows, 8 bytes of
-// alignment, spring_extra bytes per spring.
 bool plan_bins(const std::vector<RobotPack>& packs, uint32_t nb, const KernelShape& sh,
-               uint32_t smem_cap, std::vector<std::vector<uint32_t>>& plan, uint32_t spring_extra = 0) {
+               uint32_t smem_cap, std::vector<std::vector<uint32_t>>& plan) {
     const uint32_t n = (uint32_t)packs.size();
     std::vector<uint32_t> order(n);
     for (uint32_t i = 0; i < n; ++i) order[i] = i;
@@ -303,8 +301,7 @@ bool plan_bins(const std::vector<RobotPack>& packs, uint32_t nb, const KernelSha
         for (uint32_t b = 0; b < nb; ++b) {
             if (bm[b] + p.n_mass > cap_m || bs[b] + p.springs.size() > cap_s) continue;
             const uint32_t m1 = (uint32_t)(bm[b] + p.n_mass), s1 = (uint32_t)(bs[b] + p.springs.size());
-            if (bin_smem_bytes(m1, s1, (uint32_t)(bi[b] + p.inc_estimate)) + bx[b] + p.face_smem > smem_cap ||
-                (spring_extra && bin_smem_bytes(m1, s1, 0) + 8u + spring_extra * s1 > smem_cap))
+            if (bin_smem_bytes(m1, s1, (uint32_t)(bi[b] + p.inc_estimate)) + bx[b] + p.face_smem > smem_cap)
                 continue;
             if (best < 0 || load[b] < load[best]) best = (int)b;
         }
@@ -329,7 +326,7 @@ bool plan_bins(const std::vector<RobotPack>& packs, uint32_t nb, const KernelSha
 // and the caller falls back to plan_bins.
 bool plan_bins_grouped(const std::vector<RobotPack>& packs, uint32_t nb, uint32_t groups,
                        const KernelShape& sh, uint32_t smem_cap,
-                       std::vector<std::vector<uint32_t>>& plan, uint32_t spring_extra = 0) {
+                       std::vector<std::vector<uint32_t>>& plan) {
     if (groups == 0 || nb <= groups || nb % groups) return false;
     const uint32_t per = nb / groups;
     const uint32_t n = (uint32_t)packs.size();
@@ -363,8 +360,7 @@ bool plan_bins_grouped(const std::vector<RobotPack>& packs, uint32_t nb, uint32_
             for (uint32_t j = 0; j < per; ++j) {
                 if (bm[j] + p.n_mass > cap_m || bs[j] + p.springs.size() > cap_s) continue;
                 const uint32_t m1 = (uint32_t)(bm[j] + p.n_mass), s1 = (uint32_t)(bs[j] + p.springs.size());
-                if (bin_smem_bytes(m1, s1, (uint32_t)(bi[j] + p.inc_estimate)) + bx[j] + p.face_smem > smem_cap ||
-                    (spring_extra && bin_smem_bytes(m1, s1, 0) + 8u + spring_extra * s1 > smem_cap))
+                if (bin_smem_bytes(m1, s1, (uint32_t)(bi[j] + p.inc_estimate)) + bx[j] + p.face_smem > smem_cap)
                     continue;
                 if (best < 0 || load[j] < load[best]) best = (int)j;
             }
@@ -1330,13 +1326,13 @@ mb_status pack_population(const mb_batch_desc* b, const PackOptions& o, Packed& 
     const uint32_t sms = std::max<uint32_t>(o.sms, 1);
     std::vector<std::vector<uint32_t>> plan;
     bool ok = false;
-    // Automatic choice: a shape with a register-row variant is first planned
-    // for it -- at most one mass per thread in every bin and room for its 8
-    // bytes of shared memory per spring -- then, if that fails, as usual.
+    // Automatic choice: a shape the tensor-memory kernel runs is first
+    // planned for it -- at most one mass per thread in every bin -- then, if
+    // that fails, as usual.
     std::vector<std::pair<KernelShape, bool>> attempts;
     for (const auto& sh : shapes) {
-        if (!o.override.threads && out.n_faces == 0 && max_m <= sh.threads && row_reg_supported(sh) &&
-            out.max_degree <= row_reg_width())
+        if (!o.override.threads && out.n_faces == 0 && max_m <= sh.threads && tm_shape(sh) &&
+            out.max_degree <= kTmMaxDegree)
             attempts.push_back({sh, true});
         attempts.push_back({sh, false});
     }
@@ -1360,10 +1356,16 @@ mb_status pack_population(const mb_batch_desc* b, const PackOptions& o, Packed& 
         }
         if (!nb) {
             const uint64_t need = std::max<uint64_t>((tot_s + cap_s - 1) / cap_s, (tot_m + cap_m - 1) / cap_m);
-            nb = (uint32_t)std::max<uint64_t>(need, 1);
+            // fewer robots than SMs: an SM each (a step of 32 robots of 4x4x4
+            // cells takes 5.0 us in four bins, 1.55 us in 32)
+            nb = (uint32_t)std::max<uint64_t>(need, R < sms ? R : 1);
             if (R >= sms) {
                 nb = std::max<uint32_t>(nb, wave);
-                nb = (nb + wave - 1) / wave * wave;  // whole waves
+                // whole waves; for the tensor-memory kernel, which steps a
+                // CTA's bins side by side, about a robot a bin (512 uneven
+                // robots: 5.46 us a step in 444 bins, 5.73 in 296)
+                if (one_mass) nb = std::max(nb, R / wave * wave);
+                nb = (nb + wave - 1) / wave * wave;
             }
             nb = std::min<uint32_t>(nb, R);
         }
@@ -1374,21 +1376,15 @@ mb_status pack_population(const mb_batch_desc* b, const PackOptions& o, Packed& 
             grid = 0;
             bool planned = false;
             const KernelShape psh{sh.threads, sh.spt, one_mass ? 1u : sh.mpt};
-            const uint32_t extra = one_mass ? 8u : 0u;
             if (R >= sms && nb >= 2 * wave && nb % wave == 0 &&
-                plan_bins_grouped(packs, nb, wave, psh, o.smem_cap, plan, extra)) {
+                plan_bins_grouped(packs, nb, wave, psh, o.smem_cap, plan)) {
                 planned = true;
                 grid = wave;
             }
-            if (!planned) planned = plan_bins(packs, nb, psh, o.smem_cap, plan, extra);
+            if (!planned) planned = plan_bins(packs, nb, psh, o.smem_cap, plan);
             if (planned) {
                 build_all(b, packs, plan, slot_of, false, threads, out, o.rows_on_device);
-                uint64_t need = out.max_smem;
-                if (one_mass)
-                    for (const BinDesc& d : out.bins)
-                        need = std::max<uint64_t>(need, bin_smem_bytes(d.n_mass, d.n_spring, 0) + 8ull +
-                                                            8ull * d.n_spring);
-                if (need <= o.smem_cap) {
+                if (out.max_smem <= o.smem_cap) {
                     ok = true;
                     break;
                 }

@@ -15,6 +15,7 @@
 #include <cuda_runtime.h>
 
 #include "../../include/mercury_b200.h"
+#include "mb_step_math.cuh"
 
 namespace {
 
@@ -52,9 +53,49 @@ smem_read_kernel(uint32_t iters, uint32_t* sink, unsigned long long* cycles) {
     if (acc == 0x9e3779b9u) sink[blockIdx.x] = acc;  // keeps the loads live
 }
 
+// Every non-negative float (and positive NaN) as a squared length: where the fast path is taken, its length
+// and reciprocal against the intrinsics'; the packed form against both.
+__global__ void __launch_bounds__(256) spring_math_kernel(unsigned long long* bad) {
+    unsigned long long n = 0;
+    for (unsigned long long b = blockIdx.x * 256ull + threadIdx.x; b < 1ull << 31; b += gridDim.x * 256ull) {
+        const float ns = -__uint_as_float((uint32_t)b);
+        float nd, e, q, xd, xq;
+        mb::length_and_reciprocal_fast(ns, nd, e, q);
+        mb::length_and_reciprocal_exact(ns, xd, xq);
+        mb::f32x2 pd, pe, pq;
+        mb::lengths_and_reciprocals_fast(mb::pack2(ns, -1.0f), pd, pe, pq);
+        float d0, d1, e0, e1, q0, q1;
+        mb::unpack2(pd, d0, d1);
+        mb::unpack2(pe, e0, e1);
+        mb::unpack2(pq, q0, q1);
+        auto same = [](float x, float y) { return __float_as_uint(x) == __float_as_uint(y); };
+        const bool fast = mb::length_is_fast(nd, e);
+        n += fast != mb::length_is_fast(d0, e0) || d1 != -1.0f || q1 != 1.0f;
+        if (fast) n += !(same(nd, xd) && same(q, xq) && same(d0, xd) && same(q0, xq));
+    }
+    if (n) atomicAdd(bad, n);
+}
+
 }  // namespace
 
 extern "C" {
+
+mb_status mb_check_spring_math(int device, uint64_t* mismatches) {
+    if (!mismatches) return MB_ERR_ARGUMENT;
+    if (cudaSetDevice(device) != cudaSuccess) return MB_ERR_CUDA;
+    unsigned long long* bad = nullptr;
+    unsigned long long n = 0;
+    if (cudaMalloc(&bad, sizeof(*bad)) != cudaSuccess) return MB_ERR_CUDA;
+    cudaError_t e = cudaMemset(bad, 0, sizeof(*bad));
+    if (e == cudaSuccess) {
+        spring_math_kernel<<<148 * 8, 256>>>(bad);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpy(&n, bad, sizeof(n), cudaMemcpyDeviceToHost);
+    cudaFree(bad);
+    *mismatches = n;
+    return e == cudaSuccess ? MB_OK : MB_ERR_CUDA;
+}
 
 mb_status mb_measure_smem_bandwidth(int device, double* bytes_per_s, double* bytes_per_clk_sm) {
     if (!bytes_per_s) return MB_ERR_ARGUMENT;

@@ -1,0 +1,914 @@
+// Resident step kernel with per-thread operands in tensor memory (sm_100a).
+//
+// The step of mb_kernels.cu (reference sim_kernel.cu:141-269) for resident
+// bins, laid out for what bounded it there: the shared-memory pipe (71 % busy,
+// 33 wavefronts per 32 springs) and the issue slots (70 %, 130 instructions
+// per spring; counters of 512 robots of 3-8 cells).
+//   - A mass sums its springs in ascending order of the other end, so first
+//     those to lower masses.  The thread of a mass computes exactly these
+//     (its own position stays in registers, one position load a spring
+//     instead of two), adds them up as they come, and stores each for the
+//     lower end; after a barrier it adds the springs to higher masses, read
+//     from their owners.  Each correction is stored once and loaded once.
+//   - Corrections are kept as {x, y} and z (3 wavefronts a warp instead of 4)
+//     at slot 32 k + lane of the owner's slice: consecutive masses read
+//     consecutive slots, free of bank conflicts in every direction of a
+//     lattice.
+//   - Operands that belong to one thread for a whole launch (address of the
+//     other end, material, mean length, stress, slots to gather) live in
+//     tensor memory, which is read beside the shared-memory pipe: 32 warps x
+//     8 words in 81 cycles, no slower next to LDS.128 at full rate.
+//   - A CTA is split into warp groups with their own bins and barriers, so
+//     that one bin's latencies run under another's work.
+//   - Square root and reciprocal come from one approximation and are
+//     correctly rounded without branches (mb_step_math.cuh).
+// A step of those 512 robots then takes 21 wavefronts and 102 instructions
+// per spring, 5.5 us instead of 7.4; 1,638 robots of 6x6x6 cells 19.3 us
+// instead of 23.8.  What bounds it now is issue (69 %) and the warps waiting
+// at barriers (a quarter of the stalls).  24 warps of 80 registers are kept:
+// 28 (72 registers) and 32 (64) spill inside the step and measured 7.4 and
+// 8.3 us, 20 warps 5.4 us there but 25 us on the 6x6x6 robots.
+// Same operations in the same order as the oracle: same bits.
+#include <algorithm>
+#include <cmath>
+#include <type_traits>
+
+#include "mb_step_math.cuh"
+#include "mb_tm.h"
+
+namespace mb {
+
+namespace {
+
+__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+// ---- tensor memory: warp w of a CTA owns lanes 32 (w % 4) .. + 31 and its
+// share of the columns; thread t of the warp holds one word per column
+template <int N>
+__device__ __forceinline__ void tm_ld(uint32_t addr, uint32_t (&r)[N]) {
+    static_assert(N == 1 || N == 2 || N == 4, "");
+    if constexpr (N == 1)
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(r[0]) : "r"(addr));
+    else if constexpr (N == 2)
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0, %1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"(addr));
+    else  // (the wait before the first use names the registers)
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                     : "r"(addr));
+}
+__device__ __forceinline__ void tm_st(uint32_t addr, uint32_t v) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(addr), "r"(v) : "memory");
+}
+__device__ __forceinline__ void tm_st2(uint32_t addr, uint32_t a, uint32_t b) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x2.b32 [%0], {%1, %2};" ::"r"(addr), "r"(a), "r"(b) : "memory");
+}
+__device__ __forceinline__ void tm_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
+__device__ __forceinline__ void group_sync(uint32_t id, uint32_t threads) {
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+
+// Shared memory by 32-bit address: operands hold addresses, so that an
+// access needs no address arithmetic.
+__device__ __forceinline__ float2 lds2(uint32_t a) {
+    float2 v;
+    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ float lds1(uint32_t a) {
+    float v;
+    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ void sts4(uint32_t a, float x, float y, float z, float w) {
+    asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(a), "f"(x), "f"(y), "f"(z), "f"(w) : "memory");
+}
+__device__ __forceinline__ void sts2(uint32_t a, float x, float y) {
+    asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(a), "f"(x), "f"(y) : "memory");
+}
+__device__ __forceinline__ void lds_xyz(uint32_t a, f32x2& xy, float& z) {  // 16-byte position
+    f32x2 zw;
+    asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(xy), "=l"(zw) : "r"(a));
+    float w;
+    unpack2(zw, z, w);
+}
+__device__ __forceinline__ f32x2 lds_pair(uint32_t a) {
+    f32x2 v;
+    asm volatile("ld.shared.b64 %0, [%1];" : "=l"(v) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ void sts_pair(uint32_t a, f32x2 v) {
+    asm volatile("st.shared.b64 [%0], %1;" ::"r"(a), "l"(v) : "memory");
+}
+__device__ __forceinline__ uint4 lds_info(uint32_t a) {
+    uint4 v;
+    asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ void sts_info(uint32_t a, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
+    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
+}
+__device__ __forceinline__ void sts1(uint32_t a, float x) {
+    asm volatile("st.shared.f32 [%0], %1;" ::"r"(a), "f"(x) : "memory");
+}
+
+// What a group needs of its bin outside the hot path of a step, in shared
+// memory so that the step loop holds no registers for it.
+struct TmBin {
+    uint32_t bin, mass_begin, n_mass, slice_begin;
+    uint32_t n_mat;     // material factors of the bin; the next one is zero
+    uint32_t x0, mat0;  // shared addresses of the positions and the factors
+    uint32_t xy0, z0;   // of slot 0's correction
+    uint32_t row;       // row length of the actuation table
+};
+
+// Operand of an own spring: address of the other end | of the material
+// factors << 16.
+__device__ __forceinline__ uint32_t spring_word(uint32_t entry, uint32_t x0, uint32_t mat0, uint32_t n_mat) {
+    if (entry >> 31) return (x0 + 16u * (entry & 7u)) | (mat0 + 8u * n_mat) << 16;
+    return (x0 + 16u * (kTmStandIns + (entry & 0xFFFFu))) | (mat0 + 8u * (entry >> 16)) << 16;
+}
+
+// Columns of one mass: `own` springs in pairs {address of the other end |
+// of the material factors << 16} x 2, {mean length} x 2, their stresses in
+// pairs, the gather words.
+struct TmColumns {
+    uint32_t stress, gather, end;
+    __host__ __device__ TmColumns(uint32_t own, uint32_t words, bool track) {
+        stress = 4 * ((own + 1) / 2);
+        gather = (stress + (track ? 2 * ((own + 1) / 2) : 0u) + 3u) & ~3u;
+        end = (gather + words + 3u) & ~3u;
+    }
+};
+
+// WIDE: at most kTmWideWarps warps, so registers for four springs at a time:
+// with few warps an SM, latency has to be hidden within the warp (32 robots of
+// 4x4x4 cells, one an SM: 1.84 -> 1.55 us a step; 5.0 us when they shared
+// four CTAs of the other kernel).
+template <int MODE, bool TRACK, int MPT, bool WIDE>
+__global__ void __launch_bounds__(32 * (WIDE ? kTmWideWarps : kTmMaxWarps), 1) tm_step_kernel(const __grid_constant__ TmParams q) {
+    constexpr bool XPBD = MODE == kModeXpbd;
+    extern __shared__ __align__(128) uint8_t tm_smem[];
+    __shared__ uint32_t tmem_slot;
+    __shared__ TmBin bin_all[kTmMaxGroups];
+    const StepParams& p = q.p;
+    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    // the CTA's columns, a power of two, shared by its warps' four lane quarters
+    const uint32_t per_quarter = (blockDim.x / 32 + 3) / 4;
+    const uint32_t cols = per_quarter <= 2 ? 256u : 512u, my_cols = (cols / per_quarter) & ~3u;
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&tmem_slot)),
+                     "r"(cols)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem0 = tmem_slot;
+    const uint32_t tm = tmem0 + ((warp & 3u) << 21) + (warp >> 2) * my_cols;  // this warp's words
+
+    // this warp's group (lane g of 8 looks at group g); warps without one wait
+    // for the others at the end
+    uint32_t gi;
+    TmGroup grp;
+    {
+        const TmGroup mine = q.groups[blockIdx.x * kTmMaxGroups + (lane & 7u)];
+        const uint32_t in = __ballot_sync(0xffffffffu, warp >= mine.warp0 && warp < mine.warp0 + mine.warps) & 0xFFu;
+        gi = in ? (uint32_t)__ffs(in) - 1u : 0u;
+        auto of = [&](uint32_t v) { return __shfl_sync(0xffffffffu, v, gi); };
+        grp.first = of(mine.first);
+        grp.count = in ? of(mine.count) : 0u * of(mine.count);
+        grp.warp0 = of(mine.warp0);
+        grp.warps = of(mine.warps);
+        grp.mat_off = of(mine.mat_off);
+        grp.x_off = of(mine.x_off);
+        grp.xy_off = of(mine.xy_off);
+        grp.z_off = of(mine.z_off);
+        grp.info_off = of(mine.info_off);
+        grp.spare_off = of(mine.spare_off);
+    }
+    const uint32_t gw = warp - grp.warp0;  // warp of the group
+    const uint32_t gt = gw * 32 + lane;    // thread of the group
+    const uint32_t GT = 32u * grp.warps;   // the group's threads
+    const uint32_t bar = 1 + gi;
+    volatile TmBin& t = bin_all[gi];
+    const float dt = p.dt;
+    // shared memory of the group: material factors {dL0 sin(..), 1/K}, the
+    // positions, the corrections
+    const uint32_t smem0 = smem_addr(tm_smem), mat_mine = smem0 + grp.mat_off + 8u * gt;
+    const uint32_t x_mine = smem0 + grp.x_off + 16u * (kTmStandIns + gt);
+    // What the warp's slices (sl = gw, gw + warps) need in a step is read from
+    // shared memory, 32 bytes a slice, rather than held in registers:
+    //   {first address of the own corrections {x, y}, of z, own springs kept
+    //    in tensor memory | all << 16, their first column}
+    //   {column of the gather words, words kept | all << 16, address of the
+    //    words kept in shared memory, or 0}
+    const uint32_t info_mine = smem0 + grp.info_off + 32u * gw;
+
+    for (uint32_t bi = 0; bi < grp.count; ++bi) {
+        // ---- the bin, its materials and one of stiffness 0, the zero slots
+        // and the stand-in positions (far from any robot)
+        const TmBinRef ref = q.bins[grp.first + bi];
+        const uint32_t n_mat = __ldg(&q.r.n_mat[ref.bin]);
+        const uint32_t x0 = smem0 + grp.x_off, mat0 = smem0 + grp.mat_off, xy0 = smem0 + grp.xy_off, z0 = smem0 + grp.z_off;
+        // the actuation factor of material gt, loaded one step ahead; further
+        // materials (more than threads): loaded when needed
+        uint32_t rate_at = gt < 256u ? __ldg(&q.r.mat[256u * ref.bin + gt]) : 0u;
+        const bool my_mat = gt < n_mat, more_mats = gt + GT < n_mat;
+        float next_rate = my_mat ? __ldg(p.rates + rate_at) : 0.0f;
+        if (my_mat) sts1(mat_mine + 4u, __ldg(&p.invk[rate_at]));  // 1/K (reference step) or k (force modes)
+        for (uint32_t i = gt + GT; i < n_mat; i += GT)
+            sts1(mat0 + 8u * i + 4u, __ldg(&p.invk[__ldg(&q.r.mat[256u * ref.bin + i])]));
+        if (gt == 0) {
+            t.bin = ref.bin;
+            t.mass_begin = ref.mass_begin;
+            t.n_mass = ref.n_mass;
+            t.slice_begin = ref.slice_begin;
+            t.n_mat = n_mat;
+            t.x0 = x0;
+            t.mat0 = mat0;
+            t.xy0 = xy0;
+            t.z0 = z0;
+            t.row = *p.n_mat;
+            sts2(mat0 + 8u * n_mat, 0.0f, 0.0f);
+        }
+        if (gt < kTmZeros) {
+            sts2(xy0 + 8u * gt, 0.0f, 0.0f);
+            sts1(z0 + 4u * gt, 0.0f);
+        }
+        if (gt < kTmStandIns) sts4(x0 + 16u * gt, 1.0e6f, 0.0f, 0.0f, 0.0f);
+        // ---- masses m = gt + j GT, and their operands into tensor memory
+        const uint32_t n_slices = (ref.n_mass + 31) / 32;
+        // slices of this warp
+        const uint32_t mine = gw >= n_slices ? 0u : 1u + (MPT > 1 && gw + grp.warps < n_slices);
+        float3 x[MPT], v[MPT];
+        float mass[MPT];
+        uint32_t gidx = 0;  // WIDE: the mass's index and w components, for the write-back
+        float vw = 0.0f;
+        uint32_t free_col = 0;
+#pragma unroll
+        for (int j = 0; j < MPT; ++j) {
+            const uint32_t m = gt + j * GT, sl = gw + j * grp.warps;
+            x[j] = make_float3(0.f, 0.f, 0.f);
+            v[j] = make_float3(0.f, 0.f, 0.f);
+            mass[j] = 1.0f;
+            if (j >= mine) continue;
+            const uint4 h = __ldg(&q.r.head[ref.slice_begin + sl]);
+            if (m < ref.n_mass) {
+                const uint32_t g = __ldg(&p.mass_gidx[ref.mass_begin + m]);
+                const float4 P = p.pos[g], V = p.vel[g];
+                x[j] = make_float3(P.x, P.y, P.z);
+                mass[j] = P.w;
+                v[j] = make_float3(V.x, V.y, V.z);
+                if (WIDE) {
+                    gidx = g;
+                    vw = V.w;
+                }
+            }
+            __syncwarp();
+            const uint32_t own = h.x & 0xFFFFu, words = h.x >> 16, rw = h.z + lane;
+            // what fits the columns left: own springs first (in pairs), then
+            // the gather words
+            // (the step loop reads up to two pairs past the last one: room for them)
+            constexpr uint32_t kPast = WIDE && !TRACK ? 8u : 4u;
+            const uint32_t left = my_cols - free_col, room = left - kPast;
+            const uint32_t own_kept = left < kPast ? 0u : min(own, TRACK ? 2 * (room / 6u) : 2 * (room / 4u) + 1u);
+            const TmColumns tc(own_kept, words, TRACK);
+            const uint32_t words_kept = tc.gather <= left ? min(words, left - tc.gather) : 0u;
+            // gather words that the columns do not hold: in the group's spare
+            // shared memory, else in global memory
+            const uint32_t spare = j && words > words_kept && words - words_kept <= kTmSpareWords
+                                       ? smem0 + grp.spare_off + (128u * kTmSpareWords) * gw : 0u;
+            if (lane == 0) {
+                sts_info(info_mine + j * GT, xy0 + 8u * h.y, z0 + 4u * h.y, own_kept | own << 16, tm + free_col);
+                sts_info(info_mine + j * GT + 16u, tm + free_col + tc.gather, words_kept | words << 16, spare, 0u);
+            }
+            const uint32_t c0 = tm + free_col;
+#pragma unroll 4
+            for (uint32_t k = 0; k < own_kept; k += 2) {
+                const uint2 e0 = __ldg(&q.r.own[rw + 32 * k]);
+                const uint2 e1 = k + 1 < own_kept ? __ldg(&q.r.own[rw + 32 * (k + 1)]) : make_uint2(1u << 31, 0u);
+                tm_st2(c0 + 2 * k, spring_word(e0.x, x0, mat0, n_mat), spring_word(e1.x, x0, mat0, n_mat));
+                tm_st2(c0 + 2 * k + 2, e0.y, e1.y);
+            }
+            if (TRACK)
+                for (uint32_t k = 0; k < own_kept; ++k) {
+                    const uint32_t g = __ldg(&q.r.gidx[rw + 32 * k]);
+                    const float st = g != ~0u ? p.stress[g & 0x7FFFFFFFu] : 0.0f;
+                    __syncwarp();
+                    tm_st(c0 + tc.stress + k, __float_as_uint(st));
+                }
+#pragma unroll 4
+            for (uint32_t k = 0; k < words; ++k) {
+                const uint32_t w = __ldg(&q.r.gather[rw + 32 * k]);
+                if (k < words_kept)
+                    tm_st(c0 + tc.gather + k, w);
+                else if (spare)
+                    sts1(spare + 128u * (k - words_kept) + 4u * lane, __uint_as_float(w));
+            }
+            free_col = min(my_cols, (tc.gather + words_kept + 3u + free_col) & ~3u);
+        }
+        tm_wait_st();
+        __syncwarp();
+        group_sync(bar, GT);
+
+        for (uint32_t step = 0; step < p.steps; ++step) {
+            // (1) actuation factors (sim_kernel.cu:222); predicted positions
+            // x~ = x + v dt (sim_kernel.cu:147-152), or the current ones
+            if (my_mat) {
+                sts1(mat_mine, next_rate);
+                rate_at += t.row;
+                if (step + 1 < p.steps) next_rate = __ldg(p.rates + rate_at);
+            }
+            if (more_mats)
+                for (uint32_t i = gt + GT; i < t.n_mat; i += GT)
+                    sts1(t.mat0 + 8u * i, __ldg(p.rates + (size_t)step * t.row + __ldg(&q.r.mat[256u * t.bin + i])));
+            float ax[MPT], ay[MPT], az[MPT];
+#pragma unroll
+            for (int j = 0; j < MPT; ++j) {
+                if (j >= mine) break;
+                const float3 xt = XPBD ? make_float3(__fadd_rn(x[j].x, __fmul_rn(v[j].x, dt)), __fadd_rn(x[j].y, __fmul_rn(v[j].y, dt)),
+                                                     __fadd_rn(x[j].z, __fmul_rn(v[j].z, dt)))
+                                       : x[j];
+                sts4(x_mine + 16u * j * GT, xt.x, xt.y, xt.z, 0.0f);
+            }
+            __syncwarp();
+            group_sync(bar, GT);
+            // (2) distance constraints to lower masses (sim_kernel.cu:209-243)
+#pragma unroll
+            for (int j = 0; j < MPT; ++j) {
+                if (j >= mine) break;
+                const uint4 info = lds_info(info_mine + j * GT);
+                const uint32_t kept = info.z & 0xFFFFu, own = info.z >> 16, x_first = x_mine - 16u * gt;
+                // this mass's position, negated: differences are sums then
+                f32x2 nxy;
+                float nz;
+                if (XPBD) {
+                    nxy = pack2(__fsub_rn(-x[j].x, __fmul_rn(v[j].x, dt)), __fsub_rn(-x[j].y, __fmul_rn(v[j].y, dt)));
+                    nz = __fsub_rn(-x[j].z, __fmul_rn(v[j].z, dt));
+                } else {
+                    nxy = pack2(-x[j].x, -x[j].y);
+                    nz = -x[j].z;
+                }
+                // from the lower end's position to this mass: the operands'
+                // order only negates the correction, exactly; sums of what
+                // is subtracted here
+                f32x2 sxy = 0;
+                float sz = 0.0f;
+                uint32_t a_xy = info.x + 8u * lane, a_z = info.y + 4u * lane;
+                bool fast = true;
+                {
+                    auto delta = [&](uint32_t w, f32x2& dxy, float& dz) {
+                        f32x2 oxy;
+                        float oz;
+                        lds_xyz(w & 0xFFFFu, oxy, oz);
+                        dxy = add2(oxy, nxy);
+                        dz = __fadd_rn(oz, nz);
+                        float dx, dy;
+                        unpack2(dxy, dx, dy);
+                        return __fmaf_rn(-dx, dx, __fmaf_rn(-dy, dy, __fmul_rn(-dz, dz)));  // -|d|^2
+                    };
+                    // correction of the lower end, stored and summed
+                    auto apply = [&](float f, f32x2 dxy, float dz, uint32_t off) {
+                        float dx, dy;
+                        unpack2(dxy, dx, dy);
+                        const f32x2 pxy = pack2(__fmul_rn(f, dx), __fmul_rn(f, dy));
+                        const float pz = __fmul_rn(f, dz);
+                        sts_pair(a_xy + 256u * off, pxy);
+                        sts1(a_z + 128u * off, pz);
+                        sxy = add2(sxy, pxy);
+                        sz = __fadd_rn(sz, pz);
+                    };
+                    // stress: lambda/Lbar (reference, sim_kernel.cu:234); k (d - L)/Lbar (force)
+                    auto stressed = [&](float st, float lam, float lb) {
+                        return __fadd_rn(st, __fmul_rn(XPBD ? lam : -lam, __frcp_rn(lb)));
+                    };
+                    // reference step: lambda = -C/K, dp = lambda n (sim_kernel.cu:230-232);
+                    // force modes: Hooke force, -k (d - L) n
+                    // A row's padding computes a correction of +-0 -- unless
+                    // the mass is so far away or not finite that the length
+                    // is not, when it takes the exact path and is cleared.
+                    auto stand_in = [&](uint32_t w) { return (w & 0xFFFFu) < x_first; };
+                    auto clear = [&](f32x2& d, float& dz, float& nd, float& r, float L) {
+                        d = 0;
+                        dz = 0.0f;
+                        nd = -L;
+                        r = 0.0f;
+                    };
+                    struct Pair {
+                        f32x2 d0, d1, ns, L, nd, r;
+                        float z0, z1, k0, k1, l0, l1;
+                    };
+                    auto load = [&](Pair& u, const uint32_t (&c)[4]) {
+                        const float2 m0 = lds2(c[0] >> 16), m1 = lds2(c[1] >> 16);
+                        const float n0 = delta(c[0], u.d0, u.z0), n1 = delta(c[1], u.d1, u.z1);
+                        u.ns = pack2(n0, n1);
+                        u.l0 = __uint_as_float(c[2]);
+                        u.l1 = __uint_as_float(c[3]);
+                        u.L = pack2(__fmaf_rn(u.l0, m0.x, u.l0), __fmaf_rn(u.l1, m1.x, u.l1));
+                        u.k0 = m0.y;
+                        u.k1 = m1.y;
+                    };
+                    auto lengths = [&](Pair& u) {
+                        f32x2 e;
+                        lengths_and_reciprocals_fast(u.ns, u.nd, e, u.r);
+                        float nd0, nd1, e0, e1;
+                        unpack2(u.nd, nd0, nd1);
+                        unpack2(e, e0, e1);
+                        return length_is_fast(nd0, e0) && length_is_fast(nd1, e1);
+                    };
+                    auto exact = [&](Pair& u, uint32_t w0, uint32_t w1) {
+                        float n0, n1, d0, d1, r0, r1, L0, L1;
+                        unpack2(u.ns, n0, n1);
+                        unpack2(u.L, L0, L1);
+                        length_and_reciprocal_exact(n0, d0, r0);
+                        length_and_reciprocal_exact(n1, d1, r1);
+                        if (stand_in(w0)) clear(u.d0, u.z0, d0, r0, L0);
+                        if (stand_in(w1)) clear(u.d1, u.z1, d1, r1, L1);
+                        u.nd = pack2(d0, d1);
+                        u.r = pack2(r0, r1);
+                        __syncwarp();
+                    };
+                    auto finish = [&](const Pair& u, uint32_t off, const uint32_t (&st)[2], uint32_t ts) {
+                        float t0, t1, f0, f1;
+                        unpack2(add2(u.L, u.nd), t0, t1);  // -C
+                        const float lam0 = __fmul_rn(t0, u.k0), lam1 = __fmul_rn(t1, u.k1);
+                        unpack2(mul2(pack2(lam0, lam1), u.r), f0, f1);
+                        apply(f0, u.d0, u.z0, off);
+                        apply(f1, u.d1, u.z1, off + 1);
+                        if (TRACK)
+                            tm_st2(ts, __float_as_uint(stressed(__uint_as_float(st[0]), lam0, u.l0)),
+                                   __float_as_uint(stressed(__uint_as_float(st[1]), lam1, u.l1)));
+                    };
+                    uint32_t ta = info.w, ts = ta + 4 * ((kept + 1) / 2);
+                    const uint32_t end = ta + 2 * (kept & ~1u);
+                    uint32_t c[4], st[2];
+                    if (kept) {
+                        tm_ld(ta, c);
+                        if (TRACK) tm_ld(ts, st);
+                    }
+                    if (WIDE && !TRACK) {  // four springs at a time
+                        uint32_t c2[4];
+                        if (kept) tm_ld(ta + 4, c2);
+                        while (end - ta >= 8) {
+                            Pair u, w;
+                            asm volatile("tcgen05.wait::ld.sync.aligned;"
+                                         : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3]), "+r"(c2[0]), "+r"(c2[1]), "+r"(c2[2]), "+r"(c2[3]));
+                            load(u, c);
+                            load(w, c2);
+                            ta += 8;
+                            tm_ld(ta, c);
+                            tm_ld(ta + 4, c2);
+                            const bool ok0 = lengths(u), ok1 = lengths(w);
+                            fast = fast && ok0 && ok1;
+                            finish(u, 0, st, 0);
+                            finish(w, 2, st, 0);
+                            a_xy += 1024u;
+                            a_z += 512u;
+                        }
+                        asm volatile("tcgen05.wait::ld.sync.aligned;" : "+r"(c2[0]), "+r"(c2[1]), "+r"(c2[2]), "+r"(c2[3]));
+                    }
+                    while (ta != end) {
+                        Pair u;
+                        if (TRACK)
+                            asm volatile("tcgen05.wait::ld.sync.aligned;"
+                                         : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3]), "+r"(st[0]), "+r"(st[1]));
+                        else
+                            asm volatile("tcgen05.wait::ld.sync.aligned;" : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3]));
+                        load(u, c);
+                        const uint32_t st0[2] = {st[0], st[1]}, w0 = c[0], w1 = c[1];
+                        ta += 4;
+                        tm_ld(ta, c);  // the next pair (or words past the last one), in flight during this one's arithmetic
+                        if (TRACK) tm_ld(ts + 2, st);
+                        const bool ok = lengths(u);
+                        fast = fast && ok;
+                        // (the warp together: tensor-memory accesses want it converged)
+                        if (TRACK && __any_sync(0xffffffffu, !ok)) exact(u, w0, w1);
+                        finish(u, 0, st0, ts);
+                        a_xy += 512u;
+                        a_z += 256u;
+                        ts += 2;
+                    }
+                    // one spring from words {w, length}; returns lambda
+                    auto single = [&](uint32_t w, float lb) {
+                        f32x2 d;
+                        float dz, nd, e, r;
+                        const float2 mt = lds2(w >> 16);
+                        const float n = delta(w, d, dz), L = __fmaf_rn(lb, mt.x, lb);
+                        length_and_reciprocal_fast(n, nd, e, r);
+                        if (__any_sync(0xffffffffu, !length_is_fast(nd, e))) {
+                            length_and_reciprocal_exact(n, nd, r);
+                            if (stand_in(w)) clear(d, dz, nd, r, L);
+                            __syncwarp();
+                        }
+                        const float lam = __fmul_rn(__fadd_rn(L, nd), mt.y);
+                        apply(__fmul_rn(lam, r), d, dz, 0);
+                        a_xy += 256u;
+                        a_z += 128u;
+                        return lam;
+                    };
+                    if (kept)  // (loads past the last pair included)
+                        asm volatile("tcgen05.wait::ld.sync.aligned;"
+                                     : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3]), "+r"(st[0]), "+r"(st[1])::"memory");
+                    if (!TRACK && __any_sync(0xffffffffu, !fast)) {
+                        // some length needs the general square root or
+                        // reciprocal: the row again, one spring at a time
+                        sxy = 0;
+                        sz = 0.0f;
+                        a_xy = info.x + 8u * lane;
+                        a_z = info.y + 4u * lane;
+                        for (uint32_t k = 0; k < kept; ++k) {
+                            uint32_t w[1], lb[1];
+                            tm_ld(info.w + 4 * (k / 2) + (k & 1u), w);
+                            tm_ld(info.w + 4 * (k / 2) + (k & 1u) + 2, lb);
+                            asm volatile("tcgen05.wait::ld.sync.aligned;" : "+r"(w[0]), "+r"(lb[0]));
+                            single(w[0], __uint_as_float(lb[0]));
+                        }
+                    } else if (kept & 1u) {
+                        const float lb = __uint_as_float(c[2]), s0 = __uint_as_float(st[0]);
+                        const float lam = single(c[0], lb);
+                        if (TRACK) tm_st(ts, __float_as_uint(stressed(s0, lam, lb)));
+                    }
+                    // springs beyond the columns (rows grown by development): from global memory
+                    for (uint32_t k = kept; k < own; ++k) {
+                        const uint32_t at = __ldg(&q.r.head[t.slice_begin + gw + j * grp.warps]).z + 32 * k + lane;
+                        const uint2 e = __ldg(&q.r.own[at]);
+                        const float lb = __uint_as_float(e.y);
+                        const float lam = single(spring_word(e.x, t.x0, t.mat0, t.n_mat), lb);
+                        if (TRACK) {
+                            const uint32_t g = __ldg(&q.r.gidx[at]);
+                            if (g != ~0u) {
+                                float* sp = &p.stress[g & 0x7FFFFFFFu];
+                                *sp = stressed(*sp, lam, lb);
+                            }
+                        }
+                        __syncwarp();
+                    }
+                }
+                float sx, sy;
+                unpack2(sxy, sx, sy);
+                ax[j] = __fsub_rn(0.0f, sx);
+                ay[j] = __fsub_rn(0.0f, sy);
+                az[j] = __fsub_rn(0.0f, sz);
+            }
+            if (TRACK) tm_wait_st();
+            group_sync(bar, GT);
+            // (3) add the corrections of the springs to higher masses, in
+            // summation order, and integrate (sim_kernel.cu:246-268)
+#pragma unroll
+            for (int j = 0; j < MPT; ++j) {
+                if (j >= mine) break;
+                const uint4 info = lds_info(info_mine + j * GT + 16u);
+                const uint32_t xy0 = t.xy0, z0 = t.z0;
+                f32x2 fxy = pack2(ax[j], ay[j]);
+                float fz = az[j];
+                auto add = [&](uint32_t w) {
+                    const uint32_t i0 = w & 0xFFFFu, i1 = w >> 16;
+                    const f32x2 c0 = lds_pair(xy0 + 8u * i0), c1 = lds_pair(xy0 + 8u * i1);
+                    const float e0 = lds1(z0 + 4u * i0), e1 = lds1(z0 + 4u * i1);
+                    fxy = add2(add2(fxy, c0), c1);
+                    fz = __fadd_rn(__fadd_rn(fz, e0), e1);
+                };
+                // blocks of four words, then two and one
+                const uint32_t n = info.y & 0xFFFFu, words = info.y >> 16;
+                uint32_t c = info.x;
+                const uint32_t end = c + (n & ~3u);
+                uint32_t c4[4], c2[2], c1[1];
+                if (n & 2u) tm_ld(end, c2);
+                if (n & 1u) tm_ld(end + (n & 2u), c1);
+                for (; c != end; c += 4) {
+                    tm_ld(c, c4);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" : "+r"(c4[0]), "+r"(c4[1]), "+r"(c4[2]), "+r"(c4[3]));
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) add(c4[u]);
+                }
+                asm volatile("tcgen05.wait::ld.sync.aligned;" : "+r"(c2[0]), "+r"(c2[1]), "+r"(c1[0]));
+                if (n & 2u) {
+                    add(c2[0]);
+                    add(c2[1]);
+                }
+                if (n & 1u) add(c1[0]);
+                if (words > n) {  // beyond the columns
+                    const uint32_t rw = __ldg(&q.r.head[t.slice_begin + gw + j * grp.warps]).z + lane;
+                    for (uint32_t k = n; k < words; ++k)
+                        add(info.z ? __float_as_uint(lds1(info.z + 128u * (k - n) + 4u * lane)) : __ldg(&q.r.gather[rw + 32 * k]));
+                }
+                float fx, fy;
+                unpack2(fxy, fx, fy);
+                if (XPBD) {
+                    const float nx = __fadd_rn(__fadd_rn(x[j].x, __fmul_rn(v[j].x, dt)), fx);
+                    const float ny = __fadd_rn(__fadd_rn(x[j].y, __fmul_rn(v[j].y, dt)), fy);
+                    const float nz = __fadd_rn(__fadd_rn(x[j].z, __fmul_rn(v[j].z, dt)), fz);
+                    // v = 0.99*(x~ - x)/dt in double (sim_kernel.cu:265-267)
+                    v[j].x = velocity_of(__fsub_rn(nx, x[j].x), (double)dt, p.inv_dt);
+                    v[j].y = velocity_of(__fsub_rn(ny, x[j].y), (double)dt, p.inv_dt);
+                    v[j].z = velocity_of(__fsub_rn(nz, x[j].z), (double)dt, p.inv_dt);
+                    x[j] = make_float3(nx, ny, nz);
+                } else {
+                    force_integrate<MODE>(p, x[j], v[j], mass[j], p.inv_dt_f, fx, fy, fz);
+                }
+            }
+        }
+
+        // ---- write back in the upload layout; flag non-finite positions
+        bool bad = false;
+#pragma unroll
+        for (int j = 0; j < MPT; ++j) {
+            const uint32_t m = gt + j * GT;
+            if (m < t.n_mass) {
+                const uint32_t g = WIDE ? gidx : __ldg(&p.mass_gidx[t.mass_begin + m]);
+                p.pos[g] = make_float4(x[j].x, x[j].y, x[j].z, WIDE ? mass[j] : p.pos[g].w);
+                p.vel[g] = make_float4(v[j].x, v[j].y, v[j].z, WIDE ? vw : p.vel[g].w);
+                bad |= !(isfinite(x[j].x) && isfinite(x[j].y) && isfinite(x[j].z));
+            }
+            __syncwarp();
+            if (TRACK && j < mine) {
+                const uint32_t rw = __ldg(&q.r.head[t.slice_begin + gw + j * grp.warps]).z + lane;
+                const uint4 info = lds_info(info_mine + j * GT);
+                const uint32_t kept = info.z & 0xFFFFu, ts = info.w + 4 * ((kept + 1) / 2);
+                for (uint32_t k = 0; k < kept; ++k) {
+                    uint32_t st[1];
+                    __syncwarp();
+                    tm_ld(ts + k, st);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" : "+r"(st[0]));
+                    const uint32_t g = __ldg(&q.r.gidx[rw + 32 * k]);
+                    if (!(g >> 31)) p.stress[g] = __uint_as_float(st[0]);  // bit 31: a copy in a split part, or padding
+                }
+            }
+        }
+        __syncwarp();
+        if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(&p.bin_flags[t.bin], 1u);
+        __syncwarp();
+        group_sync(bar, GT);  // the group's shared memory is free for its next bin
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 0) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem0), "r"(cols));
+    }
+}
+
+// One CTA per bin, one warp per slice of 32 masses.
+__global__ void __launch_bounds__(1024) tm_rows_kernel(const TmSource in, const TmRows r) {
+    __shared__ uint32_t n_own[kTmMaxSlices], first_slot[kTmMaxSlices];
+    __shared__ uint32_t used[8];
+    const uint32_t b = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
+    const BinDesc bd = in.bins[b];
+    const uint32_t n_slices = (bd.n_mass + 31) / 32;
+    const uint32_t* pairs = in.spring_pair + bd.spring_begin;
+    uint16_t* col = r.col + bd.spring_begin;
+    // 1. the materials in use, numbered in slot order
+    if (tid < 8) used[tid] = 0;
+    __syncthreads();
+    for (uint32_t s = tid; s < bd.n_spring; s += blockDim.x) {
+        const uint32_t slot = pairs[s] >> 24;
+        if (!((((volatile uint32_t*)used)[slot >> 5] >> (slot & 31u)) & 1u)) atomicOr(&used[slot >> 5], 1u << (slot & 31u));
+    }
+    __syncthreads();
+    auto rank = [&](uint32_t slot) {
+        uint32_t i = __popc(used[slot >> 5] & ((1u << (slot & 31u)) - 1u));
+        for (uint32_t k = 0; k < (slot >> 5); ++k) i += __popc(used[k]);
+        return i;
+    };
+    if (tid < 256 && ((used[tid >> 5] >> (tid & 31u)) & 1u)) r.mat[256u * b + rank(tid)] = (uint8_t)tid;
+    if (tid == 0) {
+        uint32_t n = 0;
+        for (uint32_t k = 0; k < 8; ++k) n += __popc(used[k]);
+        r.n_mat[b] = n;
+    }
+    // an entry of mass m: 0 padding, 1 its own (other end lower), 2 to gather
+    auto kind = [&](uint32_t e, uint32_t m, uint32_t& pw, uint32_t& other) {
+        pw = other = 0;
+        if (e == kPadEntry) return 0u;
+        pw = __ldg(&pairs[e >> 1]);
+        other = (e & 1u) ? pw & 0xFFFu : (pw >> 12) & 0xFFFu;
+        // a spring from a mass to itself (no force): owned once
+        return other < m || (other == m && (e & 1u)) ? 1u : other == m ? 0u : 2u;
+    };
+    // 2. own springs: columns, and every spring's column for its lower end
+    for (uint32_t sl = tid / 32; sl < n_slices; sl += blockDim.x / 32) {
+        const uint32_t gs = bd.slice_begin + sl, w = in.slice_width[gs], m = sl * 32 + lane;
+        const uint32_t off = bd.inc_begin + in.slice_off[gs], at0 = off + 32u * gs + lane;
+        const uint16_t* inc = in.inc + off + lane;
+        uint32_t nneg = 0, npos = 0, cneg = 0, cpos = 0, pw, o;
+        bool pure = true;  // every column is all own or all to gather
+#pragma unroll 4
+        for (uint32_t k = 0; k < w; ++k) {
+            const uint32_t t = kind(inc[32 * k], m, pw, o);
+            const bool an = __any_sync(0xffffffffu, t == 1u), ap = __any_sync(0xffffffffu, t == 2u);
+            nneg += t == 1u;
+            npos += t == 2u;
+            pure &= !(an && ap);
+            cneg += an;
+            cpos += ap;
+        }
+        const uint32_t own = pure ? cneg : __reduce_max_sync(0xffffffffu, nneg);
+        const uint32_t gat = pure ? cpos : __reduce_max_sync(0xffffffffu, npos);
+        if (lane == 0) n_own[sl] = own | (gat + 1) / 2 << 16 | (pure ? 1u << 31 : 0u);
+        if (!pure)
+            for (uint32_t k = nneg; k < own; ++k) {
+                r.own[at0 + 32 * k] = make_uint2(1u << 31, __float_as_uint(1.0f));
+                r.gidx[at0 + 32 * k] = ~0u;
+            }
+        uint32_t at = 0;  // next own column: of the slice when pure, else of the lane
+#pragma unroll 2
+        for (uint32_t k = 0; k < w; ++k) {
+            const uint32_t e = inc[32 * k], t = kind(e, m, pw, o);
+            const bool an = __any_sync(0xffffffffu, t == 1u);
+            if (t == 1u) {
+                r.own[at0 + 32 * at] = make_uint2(o | rank(pw >> 24) << 16, __float_as_uint(in.spring_lbar[bd.spring_begin + (e >> 1)]));
+                r.gidx[at0 + 32 * at] = in.spring_gidx[bd.spring_begin + (e >> 1)];
+                col[e >> 1] = (uint16_t)at;
+            }
+            if (pure && an) {  // stand-ins of a bank group the quarter-warp's others leave free
+                uint32_t mask = t == 1u ? 1u << (o & 7u) : 0u;
+                for (uint32_t x = 1; x < 8; x *= 2) mask |= __shfl_xor_sync(0xffffffffu, mask, x);
+                if (t != 1u) {
+                    r.own[at0 + 32 * at] = make_uint2(1u << 31 | (mask == 0xFFu ? 0u : (uint32_t)__ffs(~mask & 0xFFu) - 1u),
+                                                      __float_as_uint(1.0f));
+                    r.gidx[at0 + 32 * at] = ~0u;
+                }
+            }
+            at += pure ? an : t == 1u;
+        }
+    }
+    __syncthreads();
+    if (tid == 0) {
+        uint32_t s = kTmZeros;
+        for (uint32_t sl = 0; sl < n_slices; ++sl) {
+            first_slot[sl] = s;
+            s += 32u * (n_own[sl] & 0xFFFFu);
+        }
+        r.n_slots[b] = s;
+    }
+    __syncthreads();
+    // 3. gather words
+    for (uint32_t sl = tid / 32; sl < n_slices; sl += blockDim.x / 32) {
+        const uint32_t gs = bd.slice_begin + sl, w = in.slice_width[gs], m = sl * 32 + lane;
+        const uint32_t off = bd.inc_begin + in.slice_off[gs];
+        const uint16_t* inc = in.inc + off + lane;
+        const bool pure = n_own[sl] >> 31;
+        const uint32_t words = (n_own[sl] >> 16) & 0x7FFFu;
+        if (lane == 0) r.head[gs] = make_uint4((n_own[sl] & 0xFFFFu) | words << 16, first_slot[sl], off + 32u * gs, 0u);
+        uint32_t* out = r.gather + off + 32u * gs;
+        uint16_t* half = reinterpret_cast<uint16_t*>(out);
+        for (uint32_t k = 0; k < words; ++k) out[32 * k + lane] = 0xFFFFFFFFu;
+        __syncwarp();
+        uint32_t at = 0, pw, o;
+#pragma unroll 4
+        for (uint32_t k = 0; k < w; ++k) {
+            const uint32_t e = inc[32 * k], t = kind(e, m, pw, o);
+            const bool ap = __any_sync(0xffffffffu, t == 2u);
+            if (t == 2u) {
+                const uint32_t slot = first_slot[o / 32] + 32u * __ldcg(&col[e >> 1]) + (o & 31u);
+                half[2 * (32 * (at / 2) + lane) + (at & 1u)] = (uint16_t)slot;
+            }
+            at += pure ? ap : t == 2u;
+        }
+        __syncwarp();
+        // padding: a zero slot of a bank (of 16 for {x, y}) that no entry of the half-warp uses
+        for (uint32_t k = 0; k < words; ++k) {
+            uint32_t v = out[32 * k + lane];
+#pragma unroll
+            for (uint32_t u = 0; u < 2; ++u) {
+                const uint32_t s = (v >> (16 * u)) & 0xFFFFu;
+                uint32_t mask = s != 0xFFFFu ? 1u << (s & 15u) : 0u;
+                for (uint32_t x = 1; x < 16; x *= 2) mask |= __shfl_xor_sync(0xffffffffu, mask, x);
+                if (s == 0xFFFFu) {
+                    const uint32_t z = (mask == 0xFFFFu ? 0u : (uint32_t)__ffs(~mask & 0xFFFFu) - 1u) + (lane & 16u);
+                    v = (v & ~(0xFFFFu << (16 * u))) | z << (16 * u);
+                }
+            }
+            out[32 * k + lane] = v;
+        }
+    }
+}
+
+using TmFn = void (*)(const TmParams);
+#define MB_TM(M)                                                                                                   \
+    {                                                                                                              \
+        {tm_step_kernel<M, false, 1, false>, tm_step_kernel<M, false, 2, false>, tm_step_kernel<M, false, 1, true>}, \
+            {tm_step_kernel<M, true, 1, false>, nullptr, tm_step_kernel<M, true, 1, true>},                         \
+    }
+const TmFn kTm[3][2][3] = {MB_TM(kModeXpbd), MB_TM(kModeForceLand), MB_TM(kModeForceWater)};
+#undef MB_TM
+
+TmFn tm_kernel(uint32_t mode, bool track, const TmPlan& plan) {
+    if (mode > kModeForceWater || !plan.ok || plan.mpt < 1 || plan.mpt > (track ? 1u : kTmMaxMpt)) return nullptr;
+    return kTm[mode][track ? 1 : 0][plan.mpt == 1 && plan.threads <= 32 * kTmWideWarps ? 2 : plan.mpt - 1];
+}
+
+}  // namespace
+
+cudaError_t launch_tm_rows(const TmSource& in, const TmRows& r, cudaStream_t s) {
+    if (in.n_bins == 0) return cudaSuccess;
+    tm_rows_kernel<<<in.n_bins, 1024, 0, s>>>(in, r);
+    return cudaGetLastError();
+}
+
+cudaError_t prepare_tm(uint32_t mode, bool track, const TmPlan& plan) {
+    const TmFn f = tm_kernel(mode, track, plan);
+    return f ? cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.smem) : cudaErrorInvalidValue;
+}
+
+cudaError_t launch_tm(const TmParams& q, const TmPlan& plan, cudaStream_t s) {
+    const TmFn f = tm_kernel(q.p.mode, q.p.track != 0, plan);
+    if (!f) return cudaErrorInvalidValue;
+    f<<<plan.ctas, plan.threads, plan.smem, s>>>(q);
+    return cudaGetLastError();
+}
+
+void tm_plan(const std::vector<BinDesc>& bins, const std::vector<uint32_t>& slots, uint32_t ctas, uint32_t n_mat,
+             uint32_t smem_cap, uint32_t max_mpt, TmPlan& out) {
+    out = TmPlan{};
+    const uint32_t nb = (uint32_t)bins.size();
+    if (nb == 0 || ctas == 0) return;
+    ctas = std::min(ctas, nb);
+    auto slices = [&](uint32_t b) { return (bins[b].n_mass + 31) / 32; };
+    // a slice's work: its own springs (slots) and its masses
+    auto cost = [&](uint32_t b) { return (double)slots[b] + 64.0 * slices(b); };
+    for (uint32_t c = 0; c < ctas; ++c) {
+        std::vector<uint32_t> mine;
+        for (uint32_t b = c; b < nb; b += ctas) mine.push_back(b);
+        bool placed = false;
+        for (uint32_t G = std::min<uint32_t>((uint32_t)mine.size(), kTmMaxGroups); G >= 1 && !placed; --G) {
+            std::vector<std::vector<uint32_t>> lists(G);
+            std::vector<double> load(G, 0.0);
+            std::vector<uint32_t> order(mine);
+            std::stable_sort(order.begin(), order.end(), [&](uint32_t a, uint32_t b) { return cost(a) > cost(b); });
+            for (uint32_t b : order) {
+                const uint32_t g = (uint32_t)(std::min_element(load.begin(), load.end()) - load.begin());
+                lists[g].push_back(b);
+                load[g] += cost(b);
+            }
+            // warps: a slice each, up to kTmMaxWarps in all; where that is not enough,
+            // one warp at a time off the group with the most for its work
+            std::vector<uint32_t> warps(G, 1), most(G, 1);
+            uint32_t total = 0;
+            for (uint32_t g = 0; g < G; ++g) {
+                for (uint32_t b : lists[g]) most[g] = std::max(most[g], slices(b));
+                warps[g] = most[g];
+                total += warps[g];
+            }
+            bool fits = true;
+            while (total > kTmMaxWarps && fits) {
+                int best = -1;
+                for (uint32_t g = 0; g < G; ++g)
+                    if (warps[g] > 1 && (warps[g] - 1) * max_mpt >= most[g] &&
+                        (best < 0 || load[g] * warps[best] < load[best] * warps[g]))
+                        best = (int)g;
+                fits = best >= 0;
+                if (fits) {
+                    --warps[best];
+                    --total;
+                }
+            }
+            if (!fits) continue;
+            uint32_t off = 0, w0 = 0;
+            std::vector<TmGroup> groups(kTmMaxGroups, TmGroup{});
+            auto take = [&](uint32_t bytes) {
+                const uint32_t at = off;
+                off += (bytes + 127u) & ~127u;
+                return at;
+            };
+            for (uint32_t g = 0; g < G; ++g) {
+                groups[g].mat_off = take(8u * (n_mat + 1));
+                groups[g].x_off = take(16u * (kTmStandIns + 32 * most[g]));
+            }
+            if (off + kTmSmemBase > 65536u) continue;  // 16-bit addresses
+            for (uint32_t g = 0; g < G; ++g) {
+                uint32_t gs = 0;
+                for (uint32_t b : lists[g]) gs = std::max(gs, slots[b]);
+                if (gs > 65535u) fits = false;  // 16-bit slots
+                groups[g].xy_off = take(8u * gs);
+                groups[g].z_off = take(4u * gs);
+                groups[g].info_off = take(32u * most[g]);
+                groups[g].spare_off = take(128u * kTmSpareWords * (most[g] - warps[g]));
+                groups[g].warp0 = w0;
+                groups[g].warps = warps[g];
+                w0 += warps[g];
+            }
+            if (!fits || off > smem_cap) continue;
+            for (uint32_t g = 0; g < G; ++g) {
+                groups[g].first = (uint32_t)out.bins.size();
+                groups[g].count = (uint32_t)lists[g].size();
+                for (uint32_t b : lists[g]) {
+                    const BinDesc& d = bins[b];
+                    out.bins.push_back({b, d.mass_begin, d.n_mass, d.slice_begin, d.inc_begin, {}});
+                }
+                out.mpt = std::max(out.mpt, (most[g] + warps[g] - 1) / warps[g]);
+            }
+            out.groups.insert(out.groups.end(), groups.begin(), groups.end());
+            out.threads = std::max(out.threads, 32 * w0);
+            out.smem = std::max(out.smem, off);
+            placed = true;
+        }
+        if (!placed) return;
+    }
+    out.ctas = ctas;
+    out.ok = true;
+}
+
+}  // namespace mb
