@@ -4,14 +4,15 @@
 // every mass joined to its k nearest masses, each unordered pair once).
 //
 // Per robot:
-//   select_kernel  one thread per mass scans the robot's positions (shared
-//                  memory) and keeps its k nearest in registers, ordered by
-//                  (squared distance, index) -- the order of a stable sort of
-//                  the distance row; squared distances are the float32 sum
-//                  (dx*dx + dy*dy) + dz*dz;
-//   mark_kernel    sets bit (min, max) of an upper-triangular bitset for
-//                  every neighbour pair;
-//   count_kernel   popcounts each row; the host adds them up;
+//   select_kernel  one warp per mass: the lanes compute 32 squared distances
+//                  at a time (the float32 sum (dx*dx + dy*dy) + dz*dz, the
+//                  robot's positions in shared memory), the warp holds the k
+//                  nearest in order of (squared distance, index) -- the order
+//                  of a stable sort of the distance row -- one per lane, and
+//                  inserts what is nearer than the last; then sets bit (min,
+//                  max) of an upper-triangular bitset for every neighbour;
+//   count_kernel   popcounts each row and scans the robot's rows; the host
+//                  adds up the robots;
 //   emit_kernel    writes the pairs row by row, partners ascending (the
 //                  lexicographic order of the unique pairs), with the float32
 //                  distance as mean length and the composite material of the
@@ -32,6 +33,7 @@ namespace {
 constexpr uint32_t kKnnMaxK = 32;
 constexpr uint32_t kKnnMaxMasses = 4096;
 constexpr uint32_t kKnnThreads = 256;
+constexpr uint32_t kKnnMasses = 64;  // masses per CTA of the selection
 
 __device__ __forceinline__ float sqdist(float3 a, float3 b) {
     const float dx = __fsub_rn(a.x, b.x), dy = __fsub_rn(a.y, b.y), dz = __fsub_rn(a.z, b.z);
@@ -49,31 +51,28 @@ struct KnnArgs {
     const float* pos;         // 3 per mass
     const int64_t* mass_off;  // n_robots + 1
     uint32_t k;
-    uint16_t* nn;             // per mass: k neighbours (scratch), ascending (d2, index)
     uint32_t* bits;           // per robot: rows of ceil(m / 32) words
     const uint64_t* bit_off;  // per robot: first word
-    uint32_t* row_count;      // per mass
+    uint32_t* row_first;      // per mass: first spring of its row within the robot
+    uint32_t* n_springs;      // per robot
 };
 
-__global__ void __launch_bounds__(kKnnThreads) select_kernel(const KnnArgs a) {
-    extern __shared__ float3 pts[];
-    const uint32_t r = blockIdx.y;
-    const int64_t m0 = a.mass_off[r];
-    const uint32_t m = (uint32_t)(a.mass_off[r + 1] - m0);
-    for (uint32_t j = threadIdx.x; j < m; j += blockDim.x)
-        pts[j] = make_float3(a.pos[3 * (m0 + j)], a.pos[3 * (m0 + j) + 1], a.pos[3 * (m0 + j) + 2]);
-    __syncthreads();
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= m) return;
-    const uint32_t k = min(a.k, m - 1);
+__device__ __forceinline__ void mark(const KnnArgs& a, uint32_t* bits, uint32_t words, uint32_t i, uint32_t j) {
+    const uint32_t lo = min(i, j), hi = max(i, j);
+    atomicOr(&bits[(size_t)lo * words + hi / 32], 1u << (hi % 32));
+}
+
+// A mass with a NaN distance, one thread: neighbours are inserted in index
+// order before the first of the list that is farther, and a NaN compares
+// farther than none, so the list depends on where the NaNs come.
+__device__ __noinline__ void select_nan(const KnnArgs& a, const float3* pts, uint32_t m, uint32_t i, uint32_t k,
+                                        uint32_t* bits, uint32_t words) {
     float kd[kKnnMaxK];
     uint32_t kj[kKnnMaxK];
     uint32_t n = 0;
-    const float3 pi = pts[i];
     for (uint32_t j = 0; j < m; ++j) {
         if (j == i) continue;
-        const float d = sqdist(pi, pts[j]);
-        // j ascends: an equal distance never displaces an earlier index
+        const float d = sqdist(pts[i], pts[j]);
         if (n == k && !(d < kd[k - 1])) continue;
         uint32_t p = n < k ? n++ : k - 1;
         while (p > 0 && d < kd[p - 1]) {
@@ -84,33 +83,101 @@ __global__ void __launch_bounds__(kKnnThreads) select_kernel(const KnnArgs a) {
         kd[p] = d;
         kj[p] = j;
     }
-    uint16_t* out = a.nn + (size_t)(m0 + i) * a.k;
-    for (uint32_t q = 0; q < a.k; ++q) out[q] = q < n ? (uint16_t)kj[q] : (uint16_t)0xFFFFu;
+    for (uint32_t q = 0; q < n; ++q) mark(a, bits, words, i, kj[q]);
 }
 
-__global__ void mark_kernel(const KnnArgs a) {
-    const uint32_t r = blockIdx.y;
+// A thread per mass with the list in local memory took 17.1 ms for 256 clouds
+// of 500-2,000 points (k = 25); a warp per mass inserts each of the about
+// k (1 + ln(m / k)) candidates that enter the list in a dozen instructions, and
+// the same clouds take 2.06 ms.  Bound by the insertions, a serial chain per
+// mass; 64 masses share one copy of the points, so that loading them is 1/64
+// of the scan and a cloud of 500 still fills 8 CTAs.
+__global__ void __launch_bounds__(kKnnThreads) select_kernel(const KnnArgs a) {
+    extern __shared__ float3 pts[];
+    const uint32_t r = blockIdx.y, lane = threadIdx.x & 31;
     const int64_t m0 = a.mass_off[r];
     const uint32_t m = (uint32_t)(a.mass_off[r + 1] - m0), words = (m + 31) / 32;
+    if (blockIdx.x * kKnnMasses >= m) return;
+    for (uint32_t j = threadIdx.x; j < m; j += blockDim.x)
+        pts[j] = make_float3(a.pos[3 * (m0 + j)], a.pos[3 * (m0 + j) + 1], a.pos[3 * (m0 + j) + 2]);
+    __syncthreads();
     uint32_t* bits = a.bits + a.bit_off[r];
-    for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < m * a.k; e += gridDim.x * blockDim.x) {
-        const uint32_t i = e / a.k, j = a.nn[(size_t)m0 * a.k + e];
-        if (j == 0xFFFFu) continue;
-        const uint32_t lo = min(i, j), hi = max(i, j);
-        atomicOr(&bits[(size_t)lo * words + hi / 32], 1u << (hi % 32));
+    const uint32_t k = min(a.k, m - 1), last = min(m, (blockIdx.x + 1) * kKnnMasses);
+    if (k == 0) return;
+    for (uint32_t i = blockIdx.x * kKnnMasses + threadIdx.x / 32; i < last; i += kKnnThreads / 32) {
+        const float3 pi = pts[i];
+        // lane l < k: the l-th nearest so far, (distance bits << 32) | index;
+        // `far`: the k-th
+        unsigned long long mine = ~0ull, far = ~0ull;
+        bool nan = false;
+        for (uint32_t j0 = 0; j0 < m; j0 += 32) {
+            const uint32_t j = j0 + lane;
+            unsigned long long key = ~0ull;
+            if (j < m && j != i) {
+                const float d = sqdist(pi, pts[j]);
+                nan |= d != d;
+                key = (unsigned long long)__float_as_uint(d) << 32 | j;
+            }
+            uint32_t in = __ballot_sync(0xffffffffu, key < far);
+            while (in) {
+                const int src = __ffs(in) - 1;
+                in &= in - 1;
+                const unsigned long long c = __shfl_sync(0xffffffffu, key, src);
+                if (!(c < far)) continue;  // the list moved on
+                const uint32_t at = __popc(__ballot_sync(0xffffffffu, mine < c));
+                const unsigned long long up = __shfl_up_sync(0xffffffffu, mine, 1);
+                mine = lane < at ? mine : lane == at ? c : up;
+                if (lane >= k) mine = ~0ull;
+                far = __shfl_sync(0xffffffffu, mine, k - 1);
+            }
+        }
+        if (__any_sync(0xffffffffu, nan)) {
+            if (lane == 0) select_nan(a, pts, m, i, k, bits, words);
+            __syncwarp();
+        } else if (lane < k) {
+            mark(a, bits, words, i, (uint32_t)mine);
+        }
     }
 }
 
-__global__ void count_kernel(const KnnArgs a) {
-    const uint32_t r = blockIdx.y;
+// One CTA per robot: springs per row, scanned, so that the host reads and sums
+// one number per robot (86 us; 29 us without the scan, then 1.4 MB of row
+// counts to the host and 2.7 MB of offsets back).
+__global__ void __launch_bounds__(1024) count_kernel(const KnnArgs a) {
+    __shared__ uint32_t warp_sum[32];
+    const uint32_t r = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x / 32;
     const int64_t m0 = a.mass_off[r];
     const uint32_t m = (uint32_t)(a.mass_off[r + 1] - m0), words = (m + 31) / 32;
     const uint32_t* bits = a.bits + a.bit_off[r];
-    for (uint32_t row = blockIdx.x * blockDim.x + threadIdx.x; row < m; row += gridDim.x * blockDim.x) {
+    uint32_t base = 0;
+    for (uint32_t row0 = 0; row0 < m; row0 += 1024) {
+        // a warp's rows one after another, its lanes over the row's words
         uint32_t c = 0;
-        for (uint32_t w = 0; w < words; ++w) c += __popc(bits[(size_t)row * words + w]);
-        a.row_count[m0 + row] = c;
+        for (uint32_t q = 0; q < 32; ++q) {
+            const uint32_t row = row0 + 32 * warp + q;
+            if (row >= m) break;
+            uint32_t n = 0;
+            for (uint32_t w = lane; w < words; w += 32) n += __popc(bits[(size_t)row * words + w]);
+            n = __reduce_add_sync(0xffffffffu, n);
+            if (lane == q) c = n;
+        }
+        uint32_t inc = c;  // inclusive scan over the 1,024 rows
+        for (uint32_t o = 1; o < 32; o *= 2) {
+            const uint32_t v = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += v;
+        }
+        if (lane == 31) warp_sum[warp] = inc;
+        __syncthreads();
+        uint32_t before = 0, total = 0;
+        for (uint32_t w = 0; w < 32; ++w) {
+            if (w < warp) before += warp_sum[w];
+            total += warp_sum[w];
+        }
+        if (row0 + threadIdx.x < m) a.row_first[m0 + row0 + threadIdx.x] = base + before + inc - c;
+        base += total;
+        __syncthreads();
     }
+    if (threadIdx.x == 0) a.n_springs[r] = base;
 }
 
 struct EmitArgs {
@@ -119,31 +186,42 @@ struct EmitArgs {
     const int64_t* mass_off;
     const uint32_t* bits;
     const uint64_t* bit_off;
-    const uint64_t* row_first;  // per mass: first spring of its row (global)
-    uint16_t* pairs;            // robot-local indices
+    const uint32_t* row_first;     // per mass: first spring of its row within the robot
+    const int64_t* spring_off;     // per robot: its first spring
+    uint16_t* pairs;               // robot-local indices
     uint8_t* mat;
     float* lbar;
 };
 
-__global__ void emit_kernel(const EmitArgs a) {
-    const uint32_t r = blockIdx.y;
+// A warp per row: lane w takes the row's words w, w + 32, ...  Bound by the
+// scattered stores; 118 us for 5.9 million springs, a thread per row 197 us.
+__global__ void __launch_bounds__(kKnnThreads) emit_kernel(const EmitArgs a) {
+    const uint32_t r = blockIdx.y, lane = threadIdx.x & 31;
     const int64_t m0 = a.mass_off[r];
     const uint32_t m = (uint32_t)(a.mass_off[r + 1] - m0), words = (m + 31) / 32;
     const uint32_t* bits = a.bits + a.bit_off[r];
-    for (uint32_t row = blockIdx.x * blockDim.x + threadIdx.x; row < m; row += gridDim.x * blockDim.x) {
-        uint64_t s = a.row_first[m0 + row];
+    for (uint32_t row = (blockIdx.x * blockDim.x + threadIdx.x) / 32; row < m; row += gridDim.x * blockDim.x / 32) {
+        uint64_t s0 = (uint64_t)a.spring_off[r] + a.row_first[m0 + row];
         const float3 p = make_float3(a.pos[3 * (m0 + row)], a.pos[3 * (m0 + row) + 1], a.pos[3 * (m0 + row) + 2]);
-        for (uint32_t w = 0; w < words; ++w) {
-            uint32_t v = bits[(size_t)row * words + w];
+        const int mp = a.mass_mat[m0 + row];
+        for (uint32_t w0 = row / 32; w0 < words; w0 += 32) {  // partners are higher
+            const uint32_t w = w0 + lane;
+            uint32_t v = w < words ? bits[(size_t)row * words + w] : 0u;
+            uint32_t n = __popc(v), inc = n;
+            for (uint32_t o = 1; o < 32; o *= 2) {
+                const uint32_t u = __shfl_up_sync(0xffffffffu, inc, o);
+                if (lane >= o) inc += u;
+            }
+            uint64_t s = s0 + inc - n;
+            s0 += __shfl_sync(0xffffffffu, inc, 31);
             while (v) {
                 const uint32_t b = w * 32 + (uint32_t)(__ffs(v) - 1);
                 v &= v - 1;
                 const int64_t g = m0 + b;
                 const float3 q = make_float3(a.pos[3 * g], a.pos[3 * g + 1], a.pos[3 * g + 2]);
-                a.pairs[2 * s] = (uint16_t)row;
-                a.pairs[2 * s + 1] = (uint16_t)b;
+                reinterpret_cast<uint32_t*>(a.pairs)[s] = row | b << 16;
                 a.lbar[s] = __fsqrt_rn(sqdist(p, q));
-                a.mat[s] = (uint8_t)composite_knn(a.mass_mat[m0 + row], a.mass_mat[g]);
+                a.mat[s] = (uint8_t)composite_knn(mp, a.mass_mat[g]);
                 ++s;
             }
         }
@@ -175,10 +253,10 @@ struct KnnScratch {
     cudaStream_t stream = nullptr;
     Dev<float> pos, lbar;
     Dev<uint8_t> mm, mat;
-    Dev<int64_t> off;
-    Dev<uint16_t> nn, pairs;
-    Dev<uint32_t> bits, rc;
-    Dev<uint64_t> boff, first;
+    Dev<int64_t> off, soff;
+    Dev<uint16_t> pairs;
+    Dev<uint32_t> bits, first, count;
+    Dev<uint64_t> boff;
 };
 
 KnnScratch& knn_scratch(int device) {
@@ -222,10 +300,10 @@ extern "C" mb_status mb_knn_springs(int device, uint32_t n_robots, const int64_t
     auto& d_mm = sc.mm;
     auto& d_mat = sc.mat;
     auto& d_off = sc.off;
-    auto& d_nn = sc.nn;
     auto& d_pairs = sc.pairs;
     auto& d_bits = sc.bits;
-    auto& d_rc = sc.rc;
+    auto& d_count = sc.count;
+    auto& d_soff = sc.soff;
     auto& d_boff = sc.boff;
     auto& d_first = sc.first;
 #define KNN_CUDA(x)                               \
@@ -235,43 +313,38 @@ extern "C" mb_status mb_knn_springs(int device, uint32_t n_robots, const int64_t
     KNN_CUDA(d_pos.alloc(3 * M));
     KNN_CUDA(d_mm.alloc(M));
     KNN_CUDA(d_off.alloc(n_robots + 1));
-    KNN_CUDA(d_nn.alloc(M * k));
     KNN_CUDA(d_bits.alloc(bit_off[n_robots]));
     KNN_CUDA(d_boff.alloc(n_robots + 1));
-    KNN_CUDA(d_rc.alloc(M));
+    KNN_CUDA(d_first.alloc(M));
+    KNN_CUDA(d_count.alloc(n_robots));
+    KNN_CUDA(d_soff.alloc(n_robots + 1));
     KNN_CUDA(cudaMemcpyAsync(d_pos.p, pos, 3 * M * sizeof(float), cudaMemcpyHostToDevice, st));
     KNN_CUDA(cudaMemcpyAsync(d_mm.p, mass_material, M, cudaMemcpyHostToDevice, st));
     KNN_CUDA(cudaMemcpyAsync(d_off.p, mass_offsets, (n_robots + 1) * sizeof(int64_t), cudaMemcpyHostToDevice, st));
     KNN_CUDA(cudaMemcpyAsync(d_boff.p, bit_off.data(), (n_robots + 1) * sizeof(uint64_t), cudaMemcpyHostToDevice, st));
     KNN_CUDA(cudaMemsetAsync(d_bits.p, 0, bit_off[n_robots] * sizeof(uint32_t), st));
-    const KnnArgs ka{d_pos.p, d_off.p, k, d_nn.p, d_bits.p, d_boff.p, d_rc.p};
-    const dim3 grid((max_m + kKnnThreads - 1) / kKnnThreads, n_robots);
-    select_kernel<<<grid, kKnnThreads, max_m * sizeof(float3), st>>>(ka);
-    mark_kernel<<<grid, kKnnThreads, 0, st>>>(ka);
-    count_kernel<<<grid, kKnnThreads, 0, st>>>(ka);
+    const KnnArgs ka{d_pos.p, d_off.p, k, d_bits.p, d_boff.p, d_first.p, d_count.p};
+    select_kernel<<<dim3((max_m + kKnnMasses - 1) / kKnnMasses, n_robots), kKnnThreads, max_m * sizeof(float3), st>>>(ka);
     KNN_CUDA(cudaGetLastError());
-    std::vector<uint32_t> rc(M);
-    KNN_CUDA(cudaMemcpyAsync(rc.data(), d_rc.p, M * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+    count_kernel<<<n_robots, 1024, 0, st>>>(ka);
+    KNN_CUDA(cudaGetLastError());
+    std::vector<uint32_t> count(n_robots);
+    KNN_CUDA(cudaMemcpyAsync(count.data(), d_count.p, n_robots * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
     KNN_CUDA(cudaStreamSynchronize(st));
-    std::vector<uint64_t> first(M);
     uint64_t total = 0;
     spring_offsets[0] = 0;
     for (uint32_t r = 0; r < n_robots; ++r) {
-        for (int64_t i = mass_offsets[r]; i < mass_offsets[r + 1]; ++i) {
-            first[i] = total;
-            total += rc[i];
-        }
+        total += count[r];
         spring_offsets[r + 1] = (int64_t)total;
     }
     if (!pairs) return MB_OK;  // counting call
     if (total > capacity || !spring_material || !lbar) return MB_ERR_CAPACITY;
-    KNN_CUDA(d_first.alloc(M));
     KNN_CUDA(d_pairs.alloc(2 * total));
     KNN_CUDA(d_mat.alloc(total));
     KNN_CUDA(d_lbar.alloc(total));
-    KNN_CUDA(cudaMemcpyAsync(d_first.p, first.data(), M * sizeof(uint64_t), cudaMemcpyHostToDevice, st));
-    const EmitArgs ea{d_pos.p, d_mm.p, d_off.p, d_bits.p, d_boff.p, d_first.p, d_pairs.p, d_mat.p, d_lbar.p};
-    emit_kernel<<<grid, kKnnThreads, 0, st>>>(ea);
+    KNN_CUDA(cudaMemcpyAsync(d_soff.p, spring_offsets, (n_robots + 1) * sizeof(int64_t), cudaMemcpyHostToDevice, st));
+    const EmitArgs ea{d_pos.p, d_mm.p, d_off.p, d_bits.p, d_boff.p, d_first.p, d_soff.p, d_pairs.p, d_mat.p, d_lbar.p};
+    emit_kernel<<<dim3((max_m + 63) / 64, n_robots), kKnnThreads, 0, st>>>(ea);
     KNN_CUDA(cudaGetLastError());
     KNN_CUDA(cudaMemcpyAsync(pairs, d_pairs.p, 2 * total * sizeof(uint16_t), cudaMemcpyDeviceToHost, st));
     KNN_CUDA(cudaMemcpyAsync(spring_material, d_mat.p, total, cudaMemcpyDeviceToHost, st));
