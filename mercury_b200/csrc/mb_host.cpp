@@ -1286,11 +1286,9 @@ namespace mb_detail {
 // Whether the tensor-memory kernel holds the population: resident bins of a
 // 1,024-thread shape with at most one mass per thread, no mass with more
 // springs than a lattice has when uploaded (the kernel stays correct when
-// development adds some, reading longer rows from global memory), and no
-// face drag.
+// development adds some, reading longer rows from global memory).
 bool tm_eligible(const mb_context* c) {
-    const bool faces = face_drag_on(c) && c->faces_packed;
-    return !c->streamed && !c->cluster && !faces && mb::tm_shape(c->shape) &&
+    return !c->streamed && !c->cluster && mb::tm_shape(c->shape) &&
            c->max_bin_mass <= c->shape.threads && c->max_degree <= mb::kTmMaxDegree;
 }
 
@@ -1330,10 +1328,13 @@ cudaError_t tm_update(mb_context* c, bool track) {
         c->tm_stale = c->tm[0].planned = c->tm[1].planned = false;
     }
     mb_context::TmLaunch& l = c->tm[track ? 1 : 0];
-    if (l.planned) return cudaSuccess;
+    const bool faces = face_drag_on(c) && c->faces_packed;
+    if (l.planned && l.plan.faces == faces) return cudaSuccess;
+    if (l.planned) c->clear_graphs();  // they hold the plan without, or with, faces
+    l.planned = false;
     // stresses add to a thread's words: one mass per thread then
     mb::tm_plan(c->h_bins, c->tm_slots, c->grid ? c->grid : c->n_bins, c->n_mat_host, mb::max_step_smem(c->device),
-                track ? 1u : mb::kTmMaxMpt, l.plan);
+                track ? 1u : mb::kTmMaxMpt, faces, l.plan);
     if (l.plan.ok) {
         std::vector<uint8_t> host;
         auto put = [&](const auto& v) {
@@ -1358,7 +1359,8 @@ cudaError_t tm_update(mb_context* c, bool track) {
 // Whether the next steps run on it (after tm_update).
 bool use_tm(const mb_context* c, bool track) {
     const mb_context::TmLaunch& l = c->tm[track ? 1 : 0];
-    return tm_eligible(c) && !c->tm_stale && l.planned && l.plan.ok;
+    return tm_eligible(c) && !c->tm_stale && l.planned && l.plan.ok &&
+           l.plan.faces == (face_drag_on(c) && c->faces_packed);
 }
 
 mb::StepParams make_params(mb_context* c, float t0, uint32_t steps, bool track) {

@@ -85,40 +85,6 @@ __device__ __forceinline__ float velocity_of(float delta, double dt, double inv_
     return __double2float_rn(__ddiv_rn(a, dt));
 }
 
-// Face drag of one surface triangle (water), the share of each corner:
-// mean corner velocity v = (v0 + v1 + v2) * RN(1/3), N = (x1 - x0) x (x2 - x0), A = |N|, unit normal
-// n = N * RN(1/(A + eps)) turned so that v.n > 0 (sim_kernel.cu:106-109),
-// force coef * A * ((v.n) v + 0.2 |v|^2 n) with coef = -rho/6, i.e.
-// -rho/2 A (...) / 3 (sim_kernel.cu:110-111).  Every operation rounds once,
-// in this order.
-__device__ __forceinline__ float4 face_force(const float4 x0, const float4 x1, const float4 x2, const float4 v0,
-                                             const float4 v1, const float4 v2, const float coef) {
-    constexpr float kThird = 0x1.555556p-2f;  // 1/3 rounded to nearest
-    const float vx = __fmul_rn(__fadd_rn(__fadd_rn(v0.x, v1.x), v2.x), kThird);
-    const float vy = __fmul_rn(__fadd_rn(__fadd_rn(v0.y, v1.y), v2.y), kThird);
-    const float vz = __fmul_rn(__fadd_rn(__fadd_rn(v0.z, v1.z), v2.z), kThird);
-    const float ax = __fsub_rn(x1.x, x0.x), ay = __fsub_rn(x1.y, x0.y), az = __fsub_rn(x1.z, x0.z);
-    const float bx = __fsub_rn(x2.x, x0.x), by = __fsub_rn(x2.y, x0.y), bz = __fsub_rn(x2.z, x0.z);
-    const float nx = __fsub_rn(__fmul_rn(ay, bz), __fmul_rn(az, by));
-    const float ny = __fsub_rn(__fmul_rn(az, bx), __fmul_rn(ax, bz));
-    const float nz = __fsub_rn(__fmul_rn(ax, by), __fmul_rn(ay, bx));
-    const float area = __fsqrt_rn(__fmaf_rn(nx, nx, __fmaf_rn(ny, ny, __fmul_rn(nz, nz))));
-    const float r = __frcp_rn(__fadd_rn(area, kEps));
-    float ux = __fmul_rn(nx, r), uy = __fmul_rn(ny, r), uz = __fmul_rn(nz, r);
-    float vn = __fmaf_rn(ux, vx, __fmaf_rn(uy, vy, __fmul_rn(uz, vz)));
-    if (!(vn > 0.0f)) {  // negating n negates the rounded dot product exactly
-        ux = -ux;
-        uy = -uy;
-        uz = -uz;
-        vn = -vn;
-    }
-    const float lift = __fmul_rn(0.2f, __fmaf_rn(vx, vx, __fmaf_rn(vy, vy, __fmul_rn(vz, vz))));
-    const float c = __fmul_rn(coef, area);
-    return make_float4(__fmul_rn(c, __fmaf_rn(lift, ux, __fmul_rn(vn, vx))),
-                       __fmul_rn(c, __fmaf_rn(lift, uy, __fmul_rn(vn, vy))),
-                       __fmul_rn(c, __fmaf_rn(lift, uz, __fmul_rn(vn, vz))), 0.0f);
-}
-
 // Length d = RN(sqrt(s)) and q = RN(1 / RN(d + eps)) of a spring from the
 // squared length s, without the branches of the general square root and
 // reciprocal: one approximate reciprocal square root y, then
@@ -151,6 +117,45 @@ __device__ __forceinline__ void length_and_reciprocal_fast(float ns, float& nd, 
 __device__ __forceinline__ void length_and_reciprocal_exact(float ns, float& nd, float& q) {
     nd = -__fsqrt_rn(-ns);
     q = __frcp_rn(__fadd_rn(-nd, kEps));
+}
+__device__ __forceinline__ void length_and_reciprocal(float s, float& nd, float& q) {
+    float e;
+    length_and_reciprocal_fast(-s, nd, e, q);
+    if (!length_is_fast(nd, e)) length_and_reciprocal_exact(-s, nd, q);
+}
+
+// Face drag of one surface triangle (water), the share of each corner:
+// mean corner velocity v = (v0 + v1 + v2) * RN(1/3), N = (x1 - x0) x (x2 - x0), A = |N|, unit normal
+// n = N * RN(1/(A + eps)) turned so that v.n > 0 (sim_kernel.cu:106-109),
+// force coef * A * ((v.n) v + 0.2 |v|^2 n) with coef = -rho/6, i.e.
+// -rho/2 A (...) / 3 (sim_kernel.cu:110-111).  Every operation rounds once,
+// in this order.
+__device__ __forceinline__ float4 face_force(const float4 x0, const float4 x1, const float4 x2, const float4 v0,
+                                             const float4 v1, const float4 v2, const float coef) {
+    constexpr float kThird = 0x1.555556p-2f;  // 1/3 rounded to nearest
+    const float vx = __fmul_rn(__fadd_rn(__fadd_rn(v0.x, v1.x), v2.x), kThird);
+    const float vy = __fmul_rn(__fadd_rn(__fadd_rn(v0.y, v1.y), v2.y), kThird);
+    const float vz = __fmul_rn(__fadd_rn(__fadd_rn(v0.z, v1.z), v2.z), kThird);
+    const float ax = __fsub_rn(x1.x, x0.x), ay = __fsub_rn(x1.y, x0.y), az = __fsub_rn(x1.z, x0.z);
+    const float bx = __fsub_rn(x2.x, x0.x), by = __fsub_rn(x2.y, x0.y), bz = __fsub_rn(x2.z, x0.z);
+    const float nx = __fsub_rn(__fmul_rn(ay, bz), __fmul_rn(az, by));
+    const float ny = __fsub_rn(__fmul_rn(az, bx), __fmul_rn(ax, bz));
+    const float nz = __fsub_rn(__fmul_rn(ax, by), __fmul_rn(ay, bx));
+    float n_area, r;  // -A and RN(1/(A + eps))
+    length_and_reciprocal(__fmaf_rn(nx, nx, __fmaf_rn(ny, ny, __fmul_rn(nz, nz))), n_area, r);
+    float ux = __fmul_rn(nx, r), uy = __fmul_rn(ny, r), uz = __fmul_rn(nz, r);
+    float vn = __fmaf_rn(ux, vx, __fmaf_rn(uy, vy, __fmul_rn(uz, vz)));
+    if (!(vn > 0.0f)) {  // negating n negates the rounded dot product exactly
+        ux = -ux;
+        uy = -uy;
+        uz = -uz;
+        vn = -vn;
+    }
+    const float lift = __fmul_rn(0.2f, __fmaf_rn(vx, vx, __fmaf_rn(vy, vy, __fmul_rn(vz, vz))));
+    const float c = __fmul_rn(coef, -n_area);
+    return make_float4(__fmul_rn(c, __fmaf_rn(lift, ux, __fmul_rn(vn, vx))),
+                       __fmul_rn(c, __fmaf_rn(lift, uy, __fmul_rn(vn, vy))),
+                       __fmul_rn(c, __fmaf_rn(lift, uz, __fmul_rn(vn, vz))), 0.0f);
 }
 
 // Two floats in one 64-bit register pair: each half rounds like the scalar

@@ -28,6 +28,12 @@
 // at barriers (a quarter of the stalls).  24 warps of 80 registers are kept:
 // 28 (72 registers) and 32 (64) spill inside the step and measured 7.4 and
 // 8.3 us, 20 warps 5.4 us there but 25 us on the 6x6x6 robots.
+// With the face drag, a face is one more correction slot: computed by any
+// thread beside the springs (velocities ride in the positions' w and one more
+// plane: 3 x 24 bytes of loads a face instead of 3 x 32), gathered after the
+// springs' slots by words in the same columns.  The 512 robots with 215,000
+// faces: 16.5 -> 10.0 us a step; bound by the shared-memory pipe (73 %, of it
+// 29 % bank conflicts of the faces' corners and gathers).
 // Same operations in the same order as the oracle: same bits.
 #include <algorithm>
 #include <cmath>
@@ -80,6 +86,11 @@ __device__ __forceinline__ float lds1(uint32_t a) {
     asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a));
     return v;
 }
+__device__ __forceinline__ float4 lds4(uint32_t a) {
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a));
+    return v;
+}
 __device__ __forceinline__ void sts4(uint32_t a, float x, float y, float z, float w) {
     asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(a), "f"(x), "f"(y), "f"(z), "f"(w) : "memory");
 }
@@ -120,6 +131,9 @@ struct TmBin {
     uint32_t x0, mat0;  // shared addresses of the positions and the factors
     uint32_t xy0, z0;   // of slot 0's correction
     uint32_t row;       // row length of the actuation table
+    // face drag: faces of the bin, their corners, the velocities' address less
+    // half that of the positions, slot 0's force
+    uint32_t n_face, face0, v_base, face_xy, face_z;
 };
 
 // Operand of an own spring: address of the other end | of the material
@@ -127,6 +141,14 @@ struct TmBin {
 __device__ __forceinline__ uint32_t spring_word(uint32_t entry, uint32_t x0, uint32_t mat0, uint32_t n_mat) {
     if (entry >> 31) return (x0 + 16u * (entry & 7u)) | (mat0 + 8u * n_mat) << 16;
     return (x0 + 16u * (kTmStandIns + (entry & 0xFFFFu))) | (mat0 + 8u * (entry >> 16)) << 16;
+}
+
+// Gather word k of a mass's faces (`row`: first entry | count << 24): slots
+// from `slot0` in face order, then zero slots.
+__device__ __forceinline__ uint32_t face_word(const uint16_t* inc, uint32_t row, uint32_t k, uint32_t slot0, uint32_t lane) {
+    const uint32_t n = row >> 24, at = (row & 0xFFFFFFu) + 2 * k;
+    const uint32_t lo = 2 * k < n ? slot0 + __ldg(&inc[at]) : lane;
+    return lo | (2 * k + 1 < n ? slot0 + __ldg(&inc[at + 1]) : lane) << 16;
 }
 
 // Columns of one mass: `own` springs in pairs {address of the other end |
@@ -148,6 +170,7 @@ struct TmColumns {
 template <int MODE, bool TRACK, int MPT, bool WIDE>
 __global__ void __launch_bounds__(32 * (WIDE ? kTmWideWarps : kTmMaxWarps), 1) tm_step_kernel(const __grid_constant__ TmParams q) {
     constexpr bool XPBD = MODE == kModeXpbd;
+    constexpr bool FACES = MODE == kModeForceWaterFaces;  // face drag compiled in
     extern __shared__ __align__(128) uint8_t tm_smem[];
     __shared__ uint32_t tmem_slot;
     __shared__ TmBin bin_all[kTmMaxGroups];
@@ -187,6 +210,10 @@ __global__ void __launch_bounds__(32 * (WIDE ? kTmWideWarps : kTmMaxWarps), 1) t
         grp.z_off = of(mine.z_off);
         grp.info_off = of(mine.info_off);
         grp.spare_off = of(mine.spare_off);
+        if (FACES) {
+            grp.v_off = of(mine.v_off);
+            grp.face_off = of(mine.face_off);
+        }
     }
     const uint32_t gw = warp - grp.warp0;  // warp of the group
     const uint32_t gt = gw * 32 + lane;    // thread of the group
@@ -231,6 +258,14 @@ __global__ void __launch_bounds__(32 * (WIDE ? kTmWideWarps : kTmMaxWarps), 1) t
             t.xy0 = xy0;
             t.z0 = z0;
             t.row = *p.n_mat;
+            if (FACES) {
+                const uint32_t slots = __ldg(&q.r.n_slots[ref.bin]);
+                t.n_face = ref.n_face;
+                t.face0 = smem0 + grp.face_off;
+                t.v_base = smem0 + grp.v_off - x0 / 2;
+                t.face_xy = xy0 + 8u * slots;
+                t.face_z = z0 + 4u * slots;
+            }
             sts2(mat0 + 8u * n_mat, 0.0f, 0.0f);
         }
         if (gt < kTmZeros) {
@@ -238,6 +273,12 @@ __global__ void __launch_bounds__(32 * (WIDE ? kTmWideWarps : kTmMaxWarps), 1) t
             sts1(z0 + 4u * gt, 0.0f);
         }
         if (gt < kTmStandIns) sts4(x0 + 16u * gt, 1.0e6f, 0.0f, 0.0f, 0.0f);
+        if (FACES)  // addresses of the corners' positions, {first | second << 16, third}
+            for (uint32_t f = gt; f < ref.n_face; f += GT) {
+                const uint2 c = __ldg(&p.faces[ref.face_begin + f]);
+                const uint32_t m0 = x0 + 16u * kTmStandIns, c0 = m0 + 16u * (c.x & 0xFFFFu), c1 = m0 + 16u * (c.x >> 16);
+                sts2(smem0 + grp.face_off + 8u * f, __uint_as_float(c0 | c1 << 16), __uint_as_float(m0 + 16u * c.y));
+            }
         // ---- masses m = gt + j GT, and their operands into tensor memory
         const uint32_t n_slices = (ref.n_mass + 31) / 32;
         // slices of this warp
@@ -255,6 +296,8 @@ __global__ void __launch_bounds__(32 * (WIDE ? kTmWideWarps : kTmMaxWarps), 1) t
             mass[j] = 1.0f;
             if (j >= mine) continue;
             const uint4 h = __ldg(&q.r.head[ref.slice_begin + sl]);
+            uint32_t face_row = 0;
+            if (FACES && ref.n_face && m < ref.n_mass) face_row = __ldg(&p.face_row[ref.mass_begin + m]);
             if (m < ref.n_mass) {
                 const uint32_t g = __ldg(&p.mass_gidx[ref.mass_begin + m]);
                 const float4 P = p.pos[g], V = p.vel[g];
@@ -267,7 +310,9 @@ __global__ void __launch_bounds__(32 * (WIDE ? kTmWideWarps : kTmMaxWarps), 1) t
                 }
             }
             __syncwarp();
-            const uint32_t own = h.x & 0xFFFFu, words = h.x >> 16, rw = h.z + lane;
+            const uint32_t own = h.x & 0xFFFFu, spring_words = h.x >> 16, rw = h.z + lane;
+            // the faces' forces are gathered after the springs' (sim_kernel.cu:246-252)
+            const uint32_t words = spring_words + (FACES ? (__reduce_max_sync(0xffffffffu, face_row >> 24) + 1) / 2 : 0u);
             // what fits the columns left: own springs first (in pairs), then
             // the gather words
             // (the step loop reads up to two pairs past the last one: room for them)
@@ -301,7 +346,11 @@ __global__ void __launch_bounds__(32 * (WIDE ? kTmWideWarps : kTmMaxWarps), 1) t
                 }
 #pragma unroll 4
             for (uint32_t k = 0; k < words; ++k) {
-                const uint32_t w = __ldg(&q.r.gather[rw + 32 * k]);
+                const uint32_t w = !FACES || k < spring_words
+                                       ? __ldg(&q.r.gather[rw + 32 * k])
+                                       : face_word(p.face_inc + ref.face_inc_begin, face_row, k - spring_words,
+                                                   __ldg(&q.r.n_slots[ref.bin]), lane);
+                if (FACES) __syncwarp();
                 if (k < words_kept)
                     tm_st(c0 + tc.gather + k, w);
                 else if (spare)
@@ -331,10 +380,25 @@ __global__ void __launch_bounds__(32 * (WIDE ? kTmWideWarps : kTmMaxWarps), 1) t
                 const float3 xt = XPBD ? make_float3(__fadd_rn(x[j].x, __fmul_rn(v[j].x, dt)), __fadd_rn(x[j].y, __fmul_rn(v[j].y, dt)),
                                                      __fadd_rn(x[j].z, __fmul_rn(v[j].z, dt)))
                                        : x[j];
-                sts4(x_mine + 16u * j * GT, xt.x, xt.y, xt.z, 0.0f);
+                sts4(x_mine + 16u * j * GT, xt.x, xt.y, xt.z, FACES ? v[j].x : 0.0f);
+                if (FACES) sts2(x_mine / 2 + 8u * j * GT + t.v_base, v[j].y, v[j].z);
             }
             __syncwarp();
             group_sync(bar, GT);
+            if (FACES) {  // the share of each corner, per face, stored like a correction
+                const uint32_t n = t.n_face, face0 = t.face0, vb = t.v_base, fxy = t.face_xy, fz = t.face_z;
+                for (uint32_t f = gt; f < n; f += GT) {
+                    const float2 c = lds2(face0 + 8u * f);
+                    const uint32_t a0 = __float_as_uint(c.x) & 0xFFFFu, a1 = __float_as_uint(c.x) >> 16, a2 = __float_as_uint(c.y);
+                    const float4 x0 = lds4(a0), x1 = lds4(a1), x2 = lds4(a2);  // (w: the velocity's x)
+                    const float2 u0 = lds2(a0 / 2 + vb), u1 = lds2(a1 / 2 + vb), u2 = lds2(a2 / 2 + vb);
+                    const float4 r = face_force(x0, x1, x2, make_float4(x0.w, u0.x, u0.y, 0.0f), make_float4(x1.w, u1.x, u1.y, 0.0f),
+                                                make_float4(x2.w, u2.x, u2.y, 0.0f), p.face_coef);
+                    sts2(fxy + 8u * f, r.x, r.y);
+                    sts1(fz + 4u * f, r.z);
+                }
+                __syncwarp();
+            }
             // (2) distance constraints to lower masses (sim_kernel.cu:209-243)
 #pragma unroll
             for (int j = 0; j < MPT; ++j) {
@@ -590,9 +654,17 @@ __global__ void __launch_bounds__(32 * (WIDE ? kTmWideWarps : kTmMaxWarps), 1) t
                 }
                 if (n & 1u) add(c1[0]);
                 if (words > n) {  // beyond the columns
-                    const uint32_t rw = __ldg(&q.r.head[t.slice_begin + gw + j * grp.warps]).z + lane;
-                    for (uint32_t k = n; k < words; ++k)
-                        add(info.z ? __float_as_uint(lds1(info.z + 128u * (k - n) + 4u * lane)) : __ldg(&q.r.gather[rw + 32 * k]));
+                    const uint4 h = __ldg(&q.r.head[t.slice_begin + gw + j * grp.warps]);
+                    auto word = [&](uint32_t k) {
+                        if (info.z) return __float_as_uint(lds1(info.z + 128u * (k - n) + 4u * lane));
+                        if (!FACES || k < h.x >> 16) return __ldg(&q.r.gather[h.z + lane + 32 * k]);
+                        const uint32_t m = gt + j * GT;
+                        return face_word(p.face_inc + p.bins[t.bin].face_inc_begin,
+                                         m < t.n_mass ? __ldg(&p.face_row[t.mass_begin + m]) : 0u, k - (h.x >> 16),
+                                         __ldg(&q.r.n_slots[t.bin]), lane);
+                    };
+                    for (uint32_t k = n; k < words; ++k) add(word(k));
+                    if (FACES) __syncwarp();
                 }
                 float fx, fy;
                 unpack2(fxy, fx, fy);
@@ -792,11 +864,15 @@ using TmFn = void (*)(const TmParams);
         {tm_step_kernel<M, false, 1, false>, tm_step_kernel<M, false, 2, false>, tm_step_kernel<M, false, 1, true>}, \
             {tm_step_kernel<M, true, 1, false>, nullptr, tm_step_kernel<M, true, 1, true>},                         \
     }
-const TmFn kTm[3][2][3] = {MB_TM(kModeXpbd), MB_TM(kModeForceLand), MB_TM(kModeForceWater)};
+const TmFn kTm[4][2][3] = {MB_TM(kModeXpbd), MB_TM(kModeForceLand), MB_TM(kModeForceWater), MB_TM(kModeForceWaterFaces)};
 #undef MB_TM
 
 TmFn tm_kernel(uint32_t mode, bool track, const TmPlan& plan) {
     if (mode > kModeForceWater || !plan.ok || plan.mpt < 1 || plan.mpt > (track ? 1u : kTmMaxMpt)) return nullptr;
+    if (plan.faces) {
+        if (mode != kModeForceWater) return nullptr;
+        mode = kModeForceWaterFaces;
+    }
     return kTm[mode][track ? 1 : 0][plan.mpt == 1 && plan.threads <= 32 * kTmWideWarps ? 2 : plan.mpt - 1];
 }
 
@@ -821,14 +897,17 @@ cudaError_t launch_tm(const TmParams& q, const TmPlan& plan, cudaStream_t s) {
 }
 
 void tm_plan(const std::vector<BinDesc>& bins, const std::vector<uint32_t>& slots, uint32_t ctas, uint32_t n_mat,
-             uint32_t smem_cap, uint32_t max_mpt, TmPlan& out) {
+             uint32_t smem_cap, uint32_t max_mpt, bool faces, TmPlan& out) {
     out = TmPlan{};
+    out.faces = faces;
     const uint32_t nb = (uint32_t)bins.size();
     if (nb == 0 || ctas == 0) return;
     ctas = std::min(ctas, nb);
     auto slices = [&](uint32_t b) { return (bins[b].n_mass + 31) / 32; };
-    // a slice's work: its own springs (slots) and its masses
-    auto cost = [&](uint32_t b) { return (double)slots[b] + 64.0 * slices(b); };
+    auto n_face = [&](uint32_t b) { return faces ? bins[b].n_face : 0u; };
+    // a slice's work: its own springs (slots), its masses, the bin's faces
+    // (about two springs' instructions each)
+    auto cost = [&](uint32_t b) { return (double)slots[b] + 64.0 * slices(b) + 2.0 * n_face(b); };
     for (uint32_t c = 0; c < ctas; ++c) {
         std::vector<uint32_t> mine;
         for (uint32_t b = c; b < nb; b += ctas) mine.push_back(b);
@@ -879,8 +958,15 @@ void tm_plan(const std::vector<BinDesc>& bins, const std::vector<uint32_t>& slot
             }
             if (off + kTmSmemBase > 65536u) continue;  // 16-bit addresses
             for (uint32_t g = 0; g < G; ++g) {
-                uint32_t gs = 0;
-                for (uint32_t b : lists[g]) gs = std::max(gs, slots[b]);
+                uint32_t gs = 0, nf = 0;
+                for (uint32_t b : lists[g]) {
+                    gs = std::max(gs, slots[b] + n_face(b));
+                    nf = std::max(nf, n_face(b));
+                }
+                if (faces) {
+                    groups[g].v_off = take(8u * (kTmStandIns + 32 * most[g]));
+                    groups[g].face_off = take(8u * nf);
+                }
                 if (gs > 65535u) fits = false;  // 16-bit slots
                 groups[g].xy_off = take(8u * gs);
                 groups[g].z_off = take(4u * gs);
@@ -896,7 +982,7 @@ void tm_plan(const std::vector<BinDesc>& bins, const std::vector<uint32_t>& slot
                 groups[g].count = (uint32_t)lists[g].size();
                 for (uint32_t b : lists[g]) {
                     const BinDesc& d = bins[b];
-                    out.bins.push_back({b, d.mass_begin, d.n_mass, d.slice_begin, d.inc_begin, {}});
+                    out.bins.push_back({b, d.mass_begin, d.n_mass, d.slice_begin, d.inc_begin, d.face_begin, n_face(b), d.face_inc_begin});
                 }
                 out.mpt = std::max(out.mpt, (most[g] + warps[g] - 1) / warps[g]);
             }

@@ -19,12 +19,12 @@ struct alignas(16) TmGroup {
     uint32_t xy_off, z_off;    // corrections of the bin's slots: {x, y} and z
     uint32_t info_off;         // 32 bytes per slice
     uint32_t spare_off;        // kTmSpareWords gather words per second slice of a warp
-    uint32_t pad[2];
+    uint32_t v_off, face_off;  // face drag: velocities {y, z} beside the positions, corners of the faces
 };
 // A bin of the list: what of its descriptor the kernel reads.
 struct alignas(16) TmBinRef {
     uint32_t bin, mass_begin, n_mass, slice_begin, inc_begin;
-    uint32_t pad[3];
+    uint32_t face_begin, n_face, face_inc_begin;  // (n_face 0 without face drag)
 };
 
 constexpr uint32_t kTmMaxWarps = 24;      // warps per CTA: 80 registers a thread
@@ -45,6 +45,7 @@ inline bool tm_shape(const KernelShape& s) { return s.threads == 1024 && (s.spt 
 // The launch of a population: which warps of which CTA step which bins.
 struct TmPlan {
     bool ok = false;
+    bool faces = false;  // with the face drag
     uint32_t ctas = 0, threads = 0, mpt = 1, smem = 0;
     std::vector<TmGroup> groups;  // kTmMaxGroups per CTA
     std::vector<TmBinRef> bins;   // the bin list
@@ -52,9 +53,10 @@ struct TmPlan {
 
 // Plans the launch over `bins` (slots[b]: correction slots of bin b, from
 // launch_tm_rows): CTA c of `ctas` steps bins c, c + ctas, ...  max_mpt:
-// masses per thread.  Not ok when a CTA's bins fit no arrangement.
+// masses per thread.  faces: with the face drag.  Not ok when a CTA's bins fit
+// no arrangement.
 void tm_plan(const std::vector<BinDesc>& bins, const std::vector<uint32_t>& slots, uint32_t ctas, uint32_t n_mat,
-             uint32_t smem_cap, uint32_t max_mpt, TmPlan& out);
+             uint32_t smem_cap, uint32_t max_mpt, bool faces, TmPlan& out);
 
 // Rows of the step kernel, from the SELL rows.  Every spring belongs to its
 // end of higher index (the owner).  Per slice of 32 masses:

@@ -116,3 +116,45 @@ def test_length_and_reciprocal_of_every_float():
     n = ctypes.c_uint64(1)
     _lib.check(_lib.LIB.mb_check_spring_math(0, ctypes.byref(n)))
     assert n.value == 0
+
+
+@pytest.mark.parametrize("track", [False, True])
+@pytest.mark.parametrize("sizes", [(1, 3, 2), (32, 33), (255, 256, 257), (700, 769)])
+def test_face_drag_bit_exact(sizes, track):
+    """Random triangles (doubled and degenerate ones among them) on random
+    robots; one mass is a corner of 200, more than its columns hold, one
+    robot has none."""
+    rng = np.random.default_rng([9, sum(sizes)])
+    els = []
+    for n in sizes:
+        e = random_robot(n, rng, 6)
+        if n >= 3:
+            e.faces = rng.integers(0, n, (2 * n, 3)).astype(np.uint16)
+            if n >= 255:
+                e.faces = np.concatenate([e.faces, np.stack([np.full(200, 5), rng.integers(6, n, 200), rng.integers(6, n, 200)], 1)
+                                          .astype(np.uint16)])
+        els.append(e)
+    batch = mb.pack(els)
+    env = S.WATER_FACES
+    sim = mb.Simulator(0)
+    table = mb.materials.force_table()
+    sim.set_materials(table)
+    sim.set_mode(2)
+    sim.set_environment(**env)
+    sim.setTimeStep(1e-4)
+    sim.set_batch(batch)
+    assert sim.step_variant()["register_rows"] == 1
+    keys = ENV_KEYS + ("face_drag",)
+    p, v, s = batch.pos.copy(), batch.vel.copy(), np.zeros(batch.n_springs, np.float32)
+    t0 = 0.0
+    for drag in (env["face_drag"], 0.0, env["face_drag"]):  # the drag off and on again between runs
+        on = dict(env, face_drag=drag)
+        sim.set_environment(**on)
+        sim.run_steps(7, track)
+        with np.errstate(all="ignore"):
+            core.force_run(2, batch, p, v, s, table, [on[k] for k in keys], 1e-4, t0, 7, track)
+        t0 = sim.getTotalTime()
+    pos, vel, stress = sim.collect_arrays()
+    assert same(pos, p) and same(vel, v)
+    if track:
+        assert same(stress, s)
