@@ -6,8 +6,9 @@
 // atomics.  Here one CTA simulates one "bin" (a group of whole robots) for a
 // whole chunk of steps without leaving the SM:
 //
-//   registers : each thread's springs (packed pair + material slot, mean
-//               length, optional 1/length and stress) and masses (x, v);
+//   registers : each thread's masses (x, v);
+//   tensor    : each thread's springs (packed pair + material slot, mean
+//   memory      length, optional stress), two at a time into registers;
 //   shared    : predicted positions x~ (SoA), per-spring corrections dp
 //               (SoA), the bin's incidence lists (SELL-32), and the per-step
 //               actuation factors and 1/K of the bin's materials.
@@ -20,6 +21,19 @@
 // incident springs in a fixed order from its SELL row (no atomics), then
 // integrates x and v (sim_kernel.cu:246-252, 261-268).
 //
+// This kernel steps what the tensor-memory kernel (mb_tm.cu) does not: parts
+// of robots split over a cluster, masses of more springs than a lattice has
+// (point clouds), small shapes.  With the springs in registers, 1,024 threads
+// of 64 registers spilled 28-300 bytes inside the step and held one load in
+// flight; in tensor memory nothing spills at the 1,024-thread shapes and two
+// springs and four row entries are in flight.  64 split robots of 11x11x11
+// masses: 6.24 -> 5.80 us a step, 256 point clouds of 500-2,000 masses: 48.0
+// -> 42.7, 30 clouds of 60: 9.4 -> 3.0.  Five or eight row entries in flight
+// measured 6.03 and 5.92 (clouds 43.4 and 44.2), one at a time 6.45 (46.5).
+// Split robots are bound by issue (71 %), clouds by the shared-memory pipe
+// while it is used (40 % conflict wavefronts of the random rows) and the
+// barriers between the parts.
+//
 // All arithmetic uses explicit round-to-nearest intrinsics so that the
 // result is bit-identical to the CPU restatement in the oracle.
 #include <cooperative_groups.h>
@@ -27,6 +41,7 @@
 #include "mb_internal.h"
 #include "mb_sin.cuh"
 #include "mb_step_math.cuh"
+#include "mb_tmem.cuh"
 
 namespace mb {
 
@@ -45,6 +60,12 @@ __global__ void __launch_bounds__(T, 1024 / T) step_kernel(const StepParams p) {
     constexpr bool FACES = MODE == kModeForceWaterFaces;  // face drag compiled in
     extern __shared__ float4 smem4[];
     const int tid = threadIdx.x;
+    // 64 columns a warp: words of the thread's springs 2 i, 2 i + 1 at
+    // column 4 i {packed word, mean length} x 2, their stresses at kStress + 2 i
+    constexpr uint32_t kCols = T / 2, kPairs = (SPT + 1) / 2, kStress = 4 * kPairs;
+    static_assert(kStress + 2 * kPairs <= 64 && kStress + 4 <= 64, "");
+    const uint32_t tmem0 = tm_alloc(reinterpret_cast<uint32_t*>(smem4), kCols);
+    const uint32_t tm = tmem0 + ((tid / 32 & 3u) << 21) + (tid / 128) * 64u;
     const float dt = p.dt;
     const double ddt = (double)dt;
     const double inv_dt = __drcp_rn(ddt);
@@ -93,22 +114,31 @@ __global__ void __launch_bounds__(T, 1024 / T) step_kernel(const StepParams p) {
             next_rate = __ldg(&p.rates[tid]);
         }
 
-        // Springs of this thread: packed word and mean length (+ stress).
-        uint32_t sw[SPT];
-        float lb[SPT], st[SPT];
+        // Springs of this thread, s = tid + j T: packed word and mean length
+        // (+ stress) into tensor memory; a missing one gets word 0.
+        __syncwarp();
 #pragma unroll
-        for (int j = 0; j < SPT; ++j) {
-            const uint32_t s = tid + j * T;
-            sw[j] = 0;
-            lb[j] = 0.0f;
-            st[j] = 0.0f;
-            if (s < bd.n_spring) {
-                const uint32_t g = bd.spring_begin + s;
-                sw[j] = __ldg(&p.spring_pair[g]);
-                lb[j] = __ldg(&p.spring_lbar[g]);
-                if (TRACK) st[j] = p.stress[__ldg(&p.spring_gidx[g]) & 0x7FFFFFFFu];
+        for (int j = 0; j < 2 * (int)kPairs; j += 2) {
+            uint32_t sw[2] = {0, 0}, lb[2] = {0, 0}, st[2] = {0, 0};
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const uint32_t s = tid + (j + u) * T;
+                if (s < bd.n_spring) {
+                    const uint32_t g = bd.spring_begin + s;
+                    sw[u] = __ldg(&p.spring_pair[g]);
+                    lb[u] = __float_as_uint(__ldg(&p.spring_lbar[g]));
+                    if (TRACK) st[u] = __float_as_uint(p.stress[__ldg(&p.spring_gidx[g]) & 0x7FFFFFFFu]);
+                }
             }
+            __syncwarp();
+            tm_st2(tm + 2 * j, sw[0], lb[0]);
+            tm_st2(tm + 2 * j + 2, sw[1], lb[1]);
+            if (TRACK) tm_st2(tm + kStress + j, st[0], st[1]);
         }
+        tm_wait_st();
+        // columns of pairs this warp has springs in
+        const uint32_t s_warp = tid & ~31u;
+        const uint32_t tm_end = tm + (bd.n_spring > s_warp ? 4u * (((bd.n_spring - s_warp + T - 1) / T + 1) / 2) : 0u);
         // Masses of this thread: x, v, mass and the SELL row (offset | width << 20).
         float3 x[MPT], v[MPT];
         float mass[MPT];
@@ -175,28 +205,70 @@ __global__ void __launch_bounds__(T, 1024 / T) step_kernel(const StepParams p) {
                 }
                 cl.sync();
             }
-            // (2) distance constraints (sim_kernel.cu:209-243)
-#pragma unroll
-            for (int j = 0; j < SPT; ++j) {
-                const uint32_t s = tid + j * T;
-                if (s >= bd.n_spring) break;
-                const uint32_t wj = sw[j];
-                const float4 pa = X[pk_a(wj)], pb = X[pk_b(wj)];
-                const float2 mt = smat[pk_slot(wj)];
-                const float lbj = lb[j];
-                const float L = __fmaf_rn(lbj, mt.x, lbj);
-                const float dx = __fsub_rn(pa.x, pb.x);
-                const float dy = __fsub_rn(pa.y, pb.y);
-                const float dz = __fsub_rn(pa.z, pb.z);
-                const float d = __fsqrt_rn(__fmaf_rn(dx, dx, __fmaf_rn(dy, dy, __fmul_rn(dz, dz))));
-                const float r = __frcp_rn(__fadd_rn(d, kEps));
-                // reference step: lambda = -C/K, dp = lambda n (sim_kernel.cu:230-232);
-                // force modes: Hooke force on the a end, -k (d - L) n
-                const float lam = __fmul_rn(-__fsub_rn(d, L), mt.y);
-                const float coef = __fmul_rn(lam, r);
-                sdp[s] = make_float4(__fmul_rn(coef, dx), __fmul_rn(coef, dy), __fmul_rn(coef, dz), 0.0f);
-                // stress: lambda/Lbar (reference, sim_kernel.cu:234); k (d - L)/Lbar (force)
-                if (TRACK) st[j] = __fadd_rn(st[j], __fmul_rn(XPBD ? lam : -lam, __frcp_rn(lbj)));
+            // (2) distance constraints (sim_kernel.cu:209-243), two springs at a
+            // time; the next two's words arrive during the arithmetic
+            if (tm != tm_end) {
+                uint32_t c[4], st[2], s = tid;
+                tm_ld(tm, c);
+                if (TRACK) tm_ld(tm + kStress, st);
+                for (uint32_t ta = tm; ta != tm_end; s += 2 * T) {
+                    if (TRACK)
+                        asm volatile("tcgen05.wait::ld.sync.aligned;"
+                                     : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3]), "+r"(st[0]), "+r"(st[1]));
+                    else
+                        asm volatile("tcgen05.wait::ld.sync.aligned;" : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3]));
+                    // (a missing spring computes from mass 0 twice, and is not stored)
+                    const float4 a0 = X[pk_a(c[0])], b0 = X[pk_b(c[0])], a1 = X[pk_a(c[2])], b1 = X[pk_b(c[2])];
+                    const float2 m0 = smat[pk_slot(c[0])], m1 = smat[pk_slot(c[2])];
+                    const float lb0 = __uint_as_float(c[1]), lb1 = __uint_as_float(c[3]);
+                    const float st0 = __uint_as_float(st[0]), st1 = __uint_as_float(st[1]);
+                    const uint32_t ts = tm + kStress + (ta - tm) / 2;
+                    ta += 4;
+                    tm_ld(ta, c);  // (past the last pair: words of this warp, not used)
+                    if (TRACK) tm_ld(ts + 2, st);
+                    const f32x2 minus = pack2(-1.0f, -1.0f);
+                    const f32x2 d0 = fma2(pack2(b0.x, b0.y), minus, pack2(a0.x, a0.y));
+                    const f32x2 d1 = fma2(pack2(b1.x, b1.y), minus, pack2(a1.x, a1.y));
+                    const float z0 = __fsub_rn(a0.z, b0.z), z1 = __fsub_rn(a1.z, b1.z);
+                    float x0, y0, x1, y1;
+                    unpack2(d0, x0, y0);
+                    unpack2(d1, x1, y1);
+                    const float n0 = __fmaf_rn(-x0, x0, __fmaf_rn(-y0, y0, __fmul_rn(-z0, z0)));
+                    const float n1 = __fmaf_rn(-x1, x1, __fmaf_rn(-y1, y1, __fmul_rn(-z1, z1)));
+                    f32x2 nd, e, r;  // -d and 1 / (d + eps)
+                    lengths_and_reciprocals_fast(pack2(n0, n1), nd, e, r);
+                    float nd0, nd1, e0, e1, r0, r1;
+                    unpack2(nd, nd0, nd1);
+                    unpack2(e, e0, e1);
+                    unpack2(r, r0, r1);
+                    const bool has0 = s < bd.n_spring, has1 = s + T < bd.n_spring;
+                    const bool ok0 = length_is_fast(nd0, e0) || !has0, ok1 = length_is_fast(nd1, e1) || !has1;
+                    if (__any_sync(0xffffffffu, !ok0 || !ok1)) {
+                        length_and_reciprocal_exact(n0, nd0, r0);
+                        length_and_reciprocal_exact(n1, nd1, r1);
+                        __syncwarp();
+                    }
+                    const float L0 = __fmaf_rn(lb0, m0.x, lb0), L1 = __fmaf_rn(lb1, m1.x, lb1);
+                    // reference step: lambda = -C/K, dp = lambda n (sim_kernel.cu:230-232);
+                    // force modes: Hooke force on the a end, -k (d - L) n
+                    const float lam0 = __fmul_rn(-__fsub_rn(-nd0, L0), m0.y), lam1 = __fmul_rn(-__fsub_rn(-nd1, L1), m1.y);
+                    const float f0 = __fmul_rn(lam0, r0), f1 = __fmul_rn(lam1, r1);
+                    float px, py;
+                    unpack2(mul2(pack2(f0, f0), d0), px, py);
+                    if (has0) sdp[s] = make_float4(px, py, __fmul_rn(f0, z0), 0.0f);
+                    unpack2(mul2(pack2(f1, f1), d1), px, py);
+                    if (has1) sdp[s + T] = make_float4(px, py, __fmul_rn(f1, z1), 0.0f);
+                    // stress: lambda/Lbar (reference, sim_kernel.cu:234); k (d - L)/Lbar (force)
+                    if (TRACK) {
+                        const float t0 = __fadd_rn(st0, __fmul_rn(XPBD ? lam0 : -lam0, __frcp_rn(lb0)));
+                        const float t1 = __fadd_rn(st1, __fmul_rn(XPBD ? lam1 : -lam1, __frcp_rn(lb1)));
+                        __syncwarp();
+                        tm_st2(ts, __float_as_uint(t0), __float_as_uint(t1));
+                    }
+                }
+                asm volatile("tcgen05.wait::ld.sync.aligned;"
+                             : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3]), "+r"(st[0]), "+r"(st[1])::"memory");
+                if (TRACK) tm_wait_st();
             }
             // face drag: the share of each corner, per face
             for (uint32_t f = tid; f < n_face; f += T) {
@@ -215,7 +287,26 @@ __global__ void __launch_bounds__(T, 1024 / T) step_kernel(const StepParams p) {
                 float ax = 0.0f, ay = 0.0f, az = 0.0f;
                 const uint16_t* rp = sinc + (row[j] & 0xFFFFFu);
                 const uint32_t w = row[j] >> 20;  // the same for the warp (one slice)
-                for (uint32_t k = 0; k < w; ++k) {
+                uint32_t k = 0;
+                for (; k + 4 <= w; k += 4) {
+                    uint32_t e[4];
+                    float4 c[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) e[u] = rp[(k + u) * kSliceWidth];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        c[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+                        if (e[u] != kPadEntry) c[u] = sdp[e[u] >> 1];
+                    }
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        const float sg = __uint_as_float(0x3f800000u | ((e[u] & 1u) << 31));
+                        ax = __fmaf_rn(c[u].x, sg, ax);
+                        ay = __fmaf_rn(c[u].y, sg, ay);
+                        az = __fmaf_rn(c[u].z, sg, az);
+                    }
+                }
+                for (; k < w; ++k) {
                     const uint32_t e = rp[k * kSliceWidth];
                     if (e != kPadEntry) {
                         const float4 c = sdp[e >> 1];
@@ -265,18 +356,26 @@ __global__ void __launch_bounds__(T, 1024 / T) step_kernel(const StepParams p) {
             }
         }
         if (TRACK) {
+            __syncwarp();
+            for (uint32_t j = 0; 2 * j < tm_end - tm; j += 2) {
+                uint32_t st[2];
+                tm_ld(tm + kStress + j, st);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" : "+r"(st[0]), "+r"(st[1]));
 #pragma unroll
-            for (int j = 0; j < SPT; ++j) {
-                const uint32_t s = tid + j * T;
-                if (s < bd.n_spring) {
-                    const uint32_t g = __ldg(&p.spring_gidx[bd.spring_begin + s]);
-                    if (!(g >> 31)) p.stress[g] = st[j];  // bit 31: a copy in a split part
+                for (int u = 0; u < 2; ++u) {
+                    const uint32_t s = tid + (j + u) * T;
+                    if (s < bd.n_spring) {
+                        const uint32_t g = __ldg(&p.spring_gidx[bd.spring_begin + s]);
+                        if (!(g >> 31)) p.stress[g] = __uint_as_float(st[u]);  // bit 31: a copy in a split part
+                    }
                 }
+                __syncwarp();
             }
         }
         if (__syncthreads_or(bad) && tid == 0) atomicOr(&p.bin_flags[b], 1u);
         if (SPLIT) cg::this_cluster().sync();
     }
+    tm_free(tmem0, kCols);
 }
 
 
@@ -375,9 +474,9 @@ __global__ void __launch_bounds__(T, 1024 / T) stream_kernel(const StepParams p)
                 const float dx = __fsub_rn(pa.x, pb.x);
                 const float dy = __fsub_rn(pa.y, pb.y);
                 const float dz = __fsub_rn(pa.z, pb.z);
-                const float d = __fsqrt_rn(__fmaf_rn(dx, dx, __fmaf_rn(dy, dy, __fmul_rn(dz, dz))));
-                const float r = __frcp_rn(__fadd_rn(d, kEps));
-                const float lam = __fmul_rn(-__fsub_rn(d, L), mt.y);
+                float nd, r;  // -d and 1 / (d + eps)
+                length_and_reciprocal(__fmaf_rn(dx, dx, __fmaf_rn(dy, dy, __fmul_rn(dz, dz))), nd, r);
+                const float lam = __fmul_rn(-__fsub_rn(-nd, L), mt.y);
                 const float coef = __fmul_rn(lam, r);
                 __stcg(&dp[s], make_float4(__fmul_rn(coef, dx), __fmul_rn(coef, dy), __fmul_rn(coef, dz), 0.0f));
                 if (TRACK) stp[s] = __fadd_rn(stp[s], __fmul_rn(XPBD ? lam : -lam, __frcp_rn(lb)));

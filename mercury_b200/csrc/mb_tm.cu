@@ -41,34 +41,11 @@
 
 #include "mb_step_math.cuh"
 #include "mb_tm.h"
+#include "mb_tmem.cuh"
 
 namespace mb {
 
 namespace {
-
-__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-// ---- tensor memory: warp w of a CTA owns lanes 32 (w % 4) .. + 31 and its
-// share of the columns; thread t of the warp holds one word per column
-template <int N>
-__device__ __forceinline__ void tm_ld(uint32_t addr, uint32_t (&r)[N]) {
-    static_assert(N == 1 || N == 2 || N == 4, "");
-    if constexpr (N == 1)
-        asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(r[0]) : "r"(addr));
-    else if constexpr (N == 2)
-        asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0, %1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"(addr));
-    else  // (the wait before the first use names the registers)
-        asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
-                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-                     : "r"(addr));
-}
-__device__ __forceinline__ void tm_st(uint32_t addr, uint32_t v) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(addr), "r"(v) : "memory");
-}
-__device__ __forceinline__ void tm_st2(uint32_t addr, uint32_t a, uint32_t b) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x2.b32 [%0], {%1, %2};" ::"r"(addr), "r"(a), "r"(b) : "memory");
-}
-__device__ __forceinline__ void tm_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 __device__ __forceinline__ void group_sync(uint32_t id, uint32_t threads) {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
@@ -179,16 +156,7 @@ __global__ void __launch_bounds__(32 * (WIDE ? kTmWideWarps : kTmMaxWarps), 1) t
     // the CTA's columns, a power of two, shared by its warps' four lane quarters
     const uint32_t per_quarter = (blockDim.x / 32 + 3) / 4;
     const uint32_t cols = per_quarter <= 2 ? 256u : 512u, my_cols = (cols / per_quarter) & ~3u;
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&tmem_slot)),
-                     "r"(cols)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem0 = tmem_slot;
+    const uint32_t tmem0 = tm_alloc(&tmem_slot, cols);
     const uint32_t tm = tmem0 + ((warp & 3u) << 21) + (warp >> 2) * my_cols;  // this warp's words
 
     // this warp's group (lane g of 8 looks at group g); warps without one wait
@@ -714,12 +682,7 @@ __global__ void __launch_bounds__(32 * (WIDE ? kTmWideWarps : kTmMaxWarps), 1) t
         __syncwarp();
         group_sync(bar, GT);  // the group's shared memory is free for its next bin
     }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    if (warp == 0) {
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem0), "r"(cols));
-    }
+    tm_free(tmem0, cols);
 }
 
 // One CTA per bin, one warp per slice of 32 masses.
