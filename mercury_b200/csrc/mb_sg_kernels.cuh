@@ -11,8 +11,7 @@
 //                   row r = b * 216 + v (sample b, voxel v), column
 //                   j = o * C + c (offset o of 27, channel c) is
 //                   act[(b * 216 + u) * C + c] with u = v + d(o) (or v - d(o)
-//                   with `flip`), 0 outside the grid.  For A it is the M x K
-//                   matrix (rows r); for B the K x N one (rows r = k).
+//                   with `flip`), 0 outside the grid (A only: M x K, rows r).
 // Every view moves 16-byte chunks of 8 consecutive elements along its
 // contiguous dimension, so that dimension and every leading dimension are
 // multiples of 8 and pointers 16-byte aligned (the host checks).
@@ -30,7 +29,7 @@ struct GemmArgs {
     const __nv_bfloat16* B;
     int M, N, K;
     int lda, ldb;         // dense views: leading dimension; im2col: channels C
-    int flip_a, flip_b;   // im2col: u = v - d(o)
+    int flip_a;           // im2col: u = v - d(o)
     // epilogue
     const float* bias;              // per column, or null
     int relu;

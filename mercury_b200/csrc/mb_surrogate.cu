@@ -102,7 +102,7 @@ __device__ __forceinline__ void load_stage(const GemmArgs& g, bf16* as, bf16* bs
             const int kr = i >> 3, ch = i & 7, gk = k0 + kr, gn = n0 + ch * 8;
             const bf16* src = nullptr;
             if (gk < k_end && gn < g.N)
-                src = BV == kIm2col ? im2col_chunk(g.B, g.ldb, gk, gn, g.flip_b) : g.B + (size_t)gk * g.ldb + gn;
+                src = g.B + (size_t)gk * g.ldb + gn;
             cp_async16(bs + kr * kLdMN + ch * 8, src ? src : g.B, src != nullptr);
         }
     }
@@ -621,12 +621,136 @@ __global__ void onehot_planar_kernel(const uint8_t* __restrict__ cls, uint32_t n
     }
 }
 
-// Split-K: partial sums added in split order, then the epilogue.
+// ---------------------------------------------------------------------------
+// Weight gradient of a 3x3x3 convolution: dW[32][27 C] = sum over rows r =
+// (sample, voxel) of dz[r][32] x im2col(x)[r][27 C], the sums of rows
+// [z k_chunk, (z+1) k_chunk) per split z in ascending order (mma.sync
+// m16n8k16).  The general GEMM read every activation 27 times from L2 through
+// its im2col view, for tiles half empty (32 of 64 rows): 47.5 us at 256
+// samples and C = 32.  Here a CTA holds 128 rows of dz and of x with their
+// halo (43 rows, the reach of the farthest neighbour, either side) and reads
+// the 27 shifts of x from shared memory, a zero row where the neighbour is
+// outside the grid; warp w takes offset 9 blockIdx.y + w (C = 32: 162 CTAs at
+// 256 samples, about one per SM) or offsets 3 w .. 3 w + 2 (C = 8):
+// 25 and 13 us.  Same sums in the same order.  Bound by the latency of a tile's
+// load and its 8 k steps (two barriers a tile, 9 warps an SM).
+constexpr int kWgRows = 128, kWgHalo = 43, kWgWarps = 9;
+
+template <int C>
+__global__ void __launch_bounds__(32 * kWgWarps) conv_wgrad_kernel(const GemmArgs g) {
+    constexpr int kX = kWgRows + 2 * kWgHalo;          // rows of x
+    constexpr int kTiles = C == 32 ? 4 : 3;            // 8-column tiles of a warp
+    constexpr int kChunks = C / 8;                     // 16-byte chunks of a row of x
+    __shared__ __align__(128) bf16 as[2][kWgRows * 32];
+    __shared__ __align__(128) bf16 xs[2][(kX + 2) * C];
+    __shared__ __align__(128) bf16 zero[8];
+    __shared__ uint32_t inside[2][kWgRows];            // bit o: row r has neighbour o
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int k_begin = blockIdx.x * g.k_chunk, k_end = min(g.K, k_begin + g.k_chunk);
+    const int nk = k_end > k_begin ? (k_end - k_begin + kWgRows - 1) / kWgRows : 0;
+    if (tid < 8) zero[tid] = __float2bfloat16_rn(0.0f);
+    // 16-byte chunk c of row r: 64-byte rows are swizzled so that 8
+    // consecutive rows lie in distinct banks
+    auto at32 = [](int r, int c) { return r * 32 + ((c ^ (r >> 1)) & 3) * 8; };
+    auto load = [&](int buf, int k0) {
+        for (int i = tid; i < kWgRows * 4; i += 32 * kWgWarps) {
+            const int r = i >> 2, c = i & 3;
+            const bool ok = k0 + r < k_end;
+            cp_async16(&as[buf][at32(r, c)], ok ? g.A + (size_t)(k0 + r) * 32 + c * 8 : g.A, ok);
+        }
+        for (int i = tid; i < kX * kChunks; i += 32 * kWgWarps) {
+            const int r = i / kChunks, c = i % kChunks, gr = k0 + r - kWgHalo;
+            const bool ok = gr >= 0 && gr < g.K;
+            cp_async16(&xs[buf][C == 32 ? at32(r, c) : r * 8], ok ? g.B + (size_t)gr * C + c * 8 : g.B, ok);
+        }
+        if (tid < kWgRows) {
+            const int v = (k0 + tid) % kVox, x = v % kGrid, y = v / kGrid % kGrid, z = v / (kGrid * kGrid);
+            // offsets o = dx + 1 + 3 (dy + 1) + 9 (dz + 1) with dx, dy, dz = -1
+            constexpr uint32_t kX0 = 0x1249249u, kY0 = 0x1C0E07u, kZ0 = 0x1FFu;
+            const uint32_t out = (x == 0 ? kX0 : 0u) | (x == kGrid - 1 ? kX0 << 2 : 0u) | (y == 0 ? kY0 : 0u) |
+                                 (y == kGrid - 1 ? kY0 << 6 : 0u) | (z == 0 ? kZ0 : 0u) | (z == kGrid - 1 ? kZ0 << 18 : 0u);
+            inside[buf][tid] = k0 + tid < k_end ? 0x7FFFFFFu & ~out : 0u;
+        }
+    };
+    // offset and first column of tile q of this warp
+    auto offset = [&](int q) { return C == 32 ? (int)blockIdx.y * kWgWarps + warp : 3 * warp + q; };
+    float acc[2][kTiles][4];
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < kTiles; ++j)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) acc[i][j][q] = 0.0f;
+    if (nk > 0) {
+        load(0, k_begin);
+        cp_async_commit();
+    }
+    for (int t = 0; t < nk; ++t) {
+        cp_async_wait_all();
+        __syncthreads();
+        if (t + 1 < nk) {
+            load((t + 1) & 1, k_begin + (t + 1) * kWgRows);
+            cp_async_commit();
+        }
+        const bf16 *a_s = as[t & 1], *x_s = xs[t & 1];
+        const uint32_t* in = inside[t & 1];
+#pragma unroll 2
+        for (int kk = 0; kk < kWgRows; kk += 16) {
+            if (k_begin + t * kWgRows + kk >= k_end) break;
+            uint32_t a[2][4], b[kTiles + 1][2];
+            const int ar = kk + (lane & 7) + ((lane >> 4) << 3);
+#pragma unroll
+            for (int i = 0; i < 2; ++i) ldsm_x4_t(a[i], a_s + at32(ar, 2 * i + ((lane >> 3) & 1)));
+            // two column tiles at a time: lanes 0-15 give the rows of the first
+            const int br = kk + (lane & 15);
+            const uint32_t ok = in[br];
+#pragma unroll
+            for (int q = 0; q < kTiles; q += 2) {
+                const int mine = min(q + (lane >> 4), kTiles - 1), o = offset(mine);
+                const int r = br + kWgHalo + (o % 3 - 1) + kGrid * (o / 3 % 3 - 1) + kGrid * kGrid * (o / 9 - 1);
+                const bf16* p = x_s + (C == 32 ? at32(r, mine) : r * 8);
+                uint32_t v[4];
+                ldsm_x4_t(v, (ok >> o) & 1u ? p : zero);
+                b[q][0] = v[0];
+                b[q][1] = v[1];
+                b[q + 1][0] = v[2];
+                b[q + 1][1] = v[3];
+            }
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+#pragma unroll
+                for (int j = 0; j < kTiles; ++j) mma_bf16(acc[i][j], a[i], b[j]);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < kTiles; ++j) {
+            const int col = offset(j) * C + (C == 32 ? 8 * j : 0) + 2 * (lane & 3);
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int row = 16 * i + (lane >> 2) + 8 * h;
+                float* out = gridDim.x > 1 ? g.partial + ((size_t)blockIdx.x * 32 + row) * g.N : g.c32 + (size_t)row * g.N;
+                *reinterpret_cast<float2*>(out + col) = make_float2(acc[i][j][2 * h], acc[i][j][2 * h + 1]);
+            }
+        }
+}
+
+// Split-K: partial sums added in split order, then the epilogue.  Bound by
+// latency: 16 partial sums in flight (27,648 outputs of 54
+// splits: 8.4 -> 4.7 us).
 __global__ void splitk_reduce_kernel(const GemmArgs g, int splits) {
     const size_t n = (size_t)g.M * g.N;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         float s = 0.0f;
-        for (int z = 0; z < splits; ++z) s += g.partial[(size_t)z * n + i];
+        for (int z = 0; z < splits; z += 16) {
+            float x[16];
+#pragma unroll
+            for (int u = 0; u < 16; ++u) x[u] = g.partial[(size_t)min(z + u, splits - 1) * n + i];
+#pragma unroll
+            for (int u = 0; u < 16; ++u)
+                if (z + u < splits) s += x[u];
+        }
         const int row = (int)(i / g.N), col = (int)(i % g.N);
         store(g, row, col, epilogue(g, row, col, s));
     }
@@ -664,74 +788,118 @@ __global__ void head_kernel(const bf16* __restrict__ h2, const bf16* __restrict_
 
 // Loss and the gradients of the head: dy = 2 (y - t) / n; dW6[j] = sum_b dy
 // h2[b, j] (thread j, samples in order); db6 = sum_b dy; dz2 = dy w6 where
-// h2 > 0.  One block of 128 threads.
-__global__ void head_backward_kernel(const float* __restrict__ y, const float* __restrict__ t,
-                                     const bf16* __restrict__ h2, const bf16* __restrict__ w6, uint32_t n,
-                                     float* __restrict__ dw6, float* __restrict__ db6, bf16* __restrict__ dz2,
-                                     float* __restrict__ loss) {
+// h2 > 0.  One block: 128 threads for the columns, one more warp whose first
+// lane sums db6 and the loss beside them.  Bound by the latency of the
+// samples' loads, so 32 are in flight (256 samples: 22.5
+// -> 12.2 us).
+constexpr int kHeadTile = 256;
+__global__ void __launch_bounds__(160) head_backward_kernel(const float* __restrict__ y, const float* __restrict__ t,
+                                                            const bf16* __restrict__ h2, const bf16* __restrict__ w6,
+                                                            uint32_t n, float* __restrict__ dw6, float* __restrict__ db6,
+                                                            bf16* __restrict__ dz2, float* __restrict__ loss) {
+    __shared__ float err[kHeadTile];
     const uint32_t j = threadIdx.x;
     const float inv = 1.0f / (float)n;
-    float g = 0.0f;
-    for (uint32_t b = 0; b < n; ++b) {
-        const float dy = 2.0f * (y[b] - t[b]) * inv;
-        const float hv = __bfloat162float(h2[(size_t)b * 128 + j]);
-        g = fmaf(dy, hv, g);
-        dz2[(size_t)b * 128 + j] = __float2bfloat16_rn(hv > 0.0f ? dy * __bfloat162float(w6[j]) : 0.0f);
-    }
-    dw6[j] = g;
-    if (j == 0) {
-        float s = 0.0f, l = 0.0f;
-        for (uint32_t b = 0; b < n; ++b) {
-            const float e = y[b] - t[b];
-            s += 2.0f * e * inv;
-            l = fmaf(e, e, l);
+    const float w = j < 128 ? __bfloat162float(w6[j]) : 0.0f;
+    float g = 0.0f, s = 0.0f, l = 0.0f;
+    for (uint32_t b0 = 0; b0 < n; b0 += kHeadTile) {
+        const uint32_t nb = min((uint32_t)kHeadTile, n - b0);
+        __syncthreads();
+        for (uint32_t i = j; i < nb; i += blockDim.x) err[i] = y[b0 + i] - t[b0 + i];
+        __syncthreads();
+        if (j < 128) {
+            const bf16* h = h2 + (size_t)b0 * 128 + j;
+            bf16* dz = dz2 + (size_t)b0 * 128 + j;
+            auto add = [&](uint32_t b, bf16 x) {
+                const float dy = 2.0f * err[b] * inv, hv = __bfloat162float(x);
+                g = fmaf(dy, hv, g);
+                dz[b * 128] = __float2bfloat16_rn(hv > 0.0f ? dy * w : 0.0f);
+            };
+            uint32_t b = 0;
+            for (; b + 32 <= nb; b += 32) {
+                bf16 x[32];
+#pragma unroll
+                for (uint32_t u = 0; u < 32; ++u) x[u] = h[(b + u) * 128];
+#pragma unroll
+                for (uint32_t u = 0; u < 32; ++u) add(b + u, x[u]);
+            }
+            for (; b < nb; ++b) add(b, h[b * 128]);
+        } else if (j == 128) {
+#pragma unroll 8
+            for (uint32_t b = 0; b < nb; ++b) {
+                const float e = err[b];
+                s = fmaf(2.0f * e, inv, s);
+                l = fmaf(e, e, l);
+            }
         }
+    }
+    if (j < 128) dw6[j] = g;
+    if (j == 128) {
         db6[0] = s;
         loss[0] = l * inv;
     }
 }
 
-// Column sums in two fixed-order stages (coalesced rows): block b sums rows
-// [b chunk, (b+1) chunk); thread t takes column t % cols and every
-// (256 / cols)-th row from phase t / cols, the phases are added in order;
-// colsum_final_kernel then adds the blocks' partial sums in contiguous
-// ranges of blocks and the ranges in order.
+// Column sums (coalesced rows), in a fixed order: block b sums rows [b chunk,
+// (b+1) chunk); thread t takes column t % cols and every (256 / cols)-th row
+// from phase t / cols, the phases are added in order.  The last block to end
+// (`done` counts them, and is 0 again afterwards) adds the blocks' partial
+// sums: for column c and part q of 1024 / cols those of a contiguous range of
+// blocks, then the parts in order.  Bound by latency: 9 rows in flight, and
+// one launch instead of two (55,296 x 32: 10.9 -> 8.0
+// us).
 constexpr int kColsumBlocks = 256;
-__global__ void __launch_bounds__(256) colsum_partial_kernel(const bf16* __restrict__ a, uint32_t rows, uint32_t cols,
-                                                             uint32_t chunk, float* __restrict__ partial) {
-    __shared__ float red[256];
-    const uint32_t t = threadIdx.x, phases = 256 / cols, c = t % cols, ph = t / cols;
-    const uint32_t r0 = blockIdx.x * chunk, r1 = min(rows, r0 + chunk);
-    float s = 0.0f;
-    if (ph < phases)
-        for (uint32_t r = r0 + ph; r < r1; r += phases) s += __bfloat162float(a[(size_t)r * cols + c]);
-    red[t] = s;
+__global__ void __launch_bounds__(256) colsum_kernel(const bf16* __restrict__ a, uint32_t rows, uint32_t cols,
+                                                     uint32_t chunk, float* __restrict__ partial,
+                                                     uint32_t* __restrict__ done, float* __restrict__ out) {
+    __shared__ float red[1024];
+    __shared__ bool last;
+    const uint32_t t = threadIdx.x, phases = 256 / cols;
+    {
+        const uint32_t c = t % cols, ph = t / cols, r0 = blockIdx.x * chunk, r1 = min(rows, r0 + chunk);
+        float s = 0.0f;
+        if (ph < phases) {
+            uint32_t r = r0 + ph;
+            const bf16* p = a + (size_t)r * cols + c;
+            const size_t row = (size_t)phases * cols;
+            for (; r + 8 * phases < r1; r += 9 * phases, p += 9 * row) {
+                bf16 x[9];
+#pragma unroll
+                for (uint32_t u = 0; u < 9; ++u) x[u] = p[u * row];
+#pragma unroll
+                for (uint32_t u = 0; u < 9; ++u) s += __bfloat162float(x[u]);
+            }
+            for (; r < r1; r += phases, p += row) s += __bfloat162float(*p);
+        }
+        red[t] = s;
+    }
     __syncthreads();
     if (t < cols) {
         float v = 0.0f;
         for (uint32_t q = 0; q < phases; ++q) v += red[q * cols + t];
         partial[(size_t)blockIdx.x * cols + t] = v;
+        __threadfence();
     }
-}
-
-// 1,024 threads: thread t adds, for column t % cols, the partial sums of a
-// contiguous range of blocks (part t / cols of 1024 / cols); the parts are
-// then added in order.  Every load of a thread is independent of the others,
-// so the stage costs about one memory latency.
-__global__ void __launch_bounds__(1024) colsum_final_kernel(const float* __restrict__ partial, uint32_t blocks,
-                                                            uint32_t cols, float* __restrict__ out) {
-    __shared__ float red[1024];
-    const uint32_t t = threadIdx.x, parts = 1024 / cols, c = t % cols, p = t / cols;
-    const uint32_t per = (blocks + parts - 1) / parts, b0 = p * per, b1 = min(blocks, b0 + per);
-    float v = 0.0f;
-    for (uint32_t b = b0; b < b1; ++b) v += partial[(size_t)b * cols + c];
-    red[t] = v;
+    __syncthreads();
+    if (t == 0) last = atomicAdd(done, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    const uint32_t parts = 1024 / cols, per = (gridDim.x + parts - 1) / parts;
+    for (uint32_t i = t; i < 1024; i += 256) {
+        const uint32_t c = i % cols, b0 = i / cols * per, b1 = min(gridDim.x, b0 + per);
+        float v = 0.0f;
+#pragma unroll 8
+        for (uint32_t b = b0; b < b1; ++b) v += __ldcg(&partial[(size_t)b * cols + c]);
+        red[i] = v;
+    }
     __syncthreads();
     if (t < cols) {
         float s = 0.0f;
         for (uint32_t q = 0; q < parts; ++q) s += red[q * cols + t];
         out[t] = s;
     }
+    if (t == 0) *done = 0;
 }
 
 // wt[(o*32 + co) * cin + ci] = w[co * 27*cin + o*cin + ci]: the weights of
@@ -773,6 +941,20 @@ cudaError_t gemm(GemmArgs g, int splits, cudaStream_t s) {
     splits = std::max(1, (g.K + g.k_chunk - 1) / g.k_chunk);
     const dim3 grid((g.N + kTileN - 1) / kTileN, (g.M + kTileM - 1) / kTileM, splits);
     gemm_kernel<AV, BV><<<grid, kGemmThreads, 0, s>>>(g);
+    if (splits > 1) {
+        const size_t n = (size_t)g.M * g.N;
+        splitk_reduce_kernel<<<(unsigned)std::min<size_t>((n + 255) / 256, 4096), 256, 0, s>>>(g, splits);
+    }
+    return cudaGetLastError();
+}
+
+// Weight gradient (args: A the gradient, B the input, K rows).
+template <int C>
+cudaError_t conv_wgrad(GemmArgs g, int splits, cudaStream_t s) {
+    splits = std::max(1, std::min<int>(splits, (int)(g.partial_cap / ((size_t)g.M * g.N))));
+    g.k_chunk = ((g.K + splits - 1) / splits + kTileK - 1) / kTileK * kTileK;
+    splits = std::max(1, (g.K + g.k_chunk - 1) / g.k_chunk);
+    conv_wgrad_kernel<C><<<dim3(splits, C == 32 ? 3 : 1), 32 * kWgWarps, 0, s>>>(g);
     if (splits > 1) {
         const size_t n = (size_t)g.M * g.N;
         splitk_reduce_kernel<<<(unsigned)std::min<size_t>((n + 255) / 256, 4096), 256, 0, s>>>(g, splits);
@@ -881,7 +1063,7 @@ struct mb_surrogate {
     float weight_decay = 0.0f;
     bool tcgen05 = true;   // forward GEMMs on the 5th-generation tensor cores
     int num_sms = 148;
-    Buf<uint32_t> tc_err;
+    Buf<uint32_t> tc_err, done;
     Buf<bf16> x0p, a1p, a2p;  // padded planar activations of the tcgen05 convolutions
     Buf<bf16> dz3p, dz2p, wf2, wf3;  // backward on tcgen05: planar gradients, mirrored weights
     Buf<float> w, m, v, g, loss, y, t, partial;
@@ -991,11 +1173,10 @@ int splits_for(int K) { return std::max(1, std::min(64, K / 1024)); }
 // Bias gradients: column sums of a [rows][cols] gradient (cols 32 or 128),
 // in a fixed order (partial sums in the split-K scratch).
 void colsum(mb_surrogate* s, const bf16* a, uint32_t rows, uint32_t cols, float* out) {
-    assert(cols <= 256 && 256 % cols == 0);  // both stages split 256 / 1024 threads into whole columns
+    assert(cols <= 256 && 256 % cols == 0);  // both stages split 256 / 1024 lanes into whole columns
     const uint32_t chunk = std::max<uint32_t>(1, (rows + kColsumBlocks - 1) / kColsumBlocks);
     const uint32_t blocks = (rows + chunk - 1) / chunk;
-    colsum_partial_kernel<<<blocks, 256, 0, s->stream>>>(a, rows, cols, chunk, s->partial.p);
-    colsum_final_kernel<<<1, 1024, 0, s->stream>>>(s->partial.p, blocks, cols, out);
+    colsum_kernel<<<blocks, 256, 0, s->stream>>>(a, rows, cols, chunk, s->partial.p, s->done.p, out);
 }
 
 // Backward of the last forward against targets s->t; gradients into s->g.
@@ -1003,7 +1184,7 @@ cudaError_t backward(mb_surrogate* s, uint32_t n) {
     cudaStream_t st = s->stream;
     const int R = (int)n * kVox;
     cudaError_t e;
-    head_backward_kernel<<<1, 128, 0, st>>>(s->y.p, s->t.p, s->h2.p, PB(s, kW6), n, G(s, kW6), G(s, kB6),
+    head_backward_kernel<<<1, 160, 0, st>>>(s->y.p, s->t.p, s->h2.p, PB(s, kW6), n, G(s, kW6), G(s, kB6),
                                             s->dz2h.p, s->loss.p);
     // fc2: dW5 = dz2^T h1, db5, dz1 = (dz2 W5) where h1 > 0
     {
@@ -1035,7 +1216,7 @@ cudaError_t backward(mb_surrogate* s, uint32_t n) {
     {
         GemmArgs a = args(s, s->dz3.p, 32, s->a2.p, 32, 32, 27 * 32, R);
         a.c32 = G(s, kW3);
-        if ((e = gemm<kDenseMN, kIm2col>(a, splits_for(R), st)) != cudaSuccess) return e;
+        if ((e = conv_wgrad<32>(a, splits_for(R), st)) != cudaSuccess) return e;
     }
     colsum(s, s->dz3.p, (uint32_t)R, 32, G(s, kB3));
     if (s->tcgen05) {
@@ -1059,7 +1240,7 @@ cudaError_t backward(mb_surrogate* s, uint32_t n) {
     {
         GemmArgs a = args(s, s->dz2c.p, 32, s->a1.p, 32, 32, 27 * 32, R);
         a.c32 = G(s, kW2);
-        if ((e = gemm<kDenseMN, kIm2col>(a, splits_for(R), st)) != cudaSuccess) return e;
+        if ((e = conv_wgrad<32>(a, splits_for(R), st)) != cudaSuccess) return e;
     }
     colsum(s, s->dz2c.p, (uint32_t)R, 32, G(s, kB2));
     if (s->tcgen05) {
@@ -1079,7 +1260,7 @@ cudaError_t backward(mb_surrogate* s, uint32_t n) {
     {
         GemmArgs a = args(s, s->dz1c.p, 32, s->x0.p, 8, 32, 27 * 8, R);
         a.c32 = G(s, kW1);
-        if ((e = gemm<kDenseMN, kIm2col>(a, splits_for(R), st)) != cudaSuccess) return e;
+        if ((e = conv_wgrad<8>(a, splits_for(R), st)) != cudaSuccess) return e;
     }
     colsum(s, s->dz1c.p, (uint32_t)R, 32, G(s, kB1));
     return cudaGetLastError();
@@ -1122,13 +1303,14 @@ mb_status mb_surrogate_create(int device, uint32_t max_batch, uint64_t seed, mb_
           ok(s->a2.alloc(R * 32)) && ok(s->a3.alloc(R * 32)) && ok(s->h1.alloc((size_t)max_batch * 128)) &&
           ok(s->h2.alloc((size_t)max_batch * 128)) && ok(s->dz2h.alloc((size_t)max_batch * 128)) &&
           ok(s->dz1h.alloc((size_t)max_batch * 128)) && ok(s->dz3.alloc(R * 32)) && ok(s->dz2c.alloc(R * 32)) &&
-          ok(s->dz1c.alloc(R * 32)) && ok(s->cls.alloc(R)) && ok(s->tc_err.alloc(1)) &&
+          ok(s->dz1c.alloc(R * 32)) && ok(s->cls.alloc(R)) && ok(s->tc_err.alloc(1)) && ok(s->done.alloc(1)) &&
           ok(s->x0p.alloc((size_t)cv_rows(max_batch) * 8)) && ok(s->a1p.alloc((size_t)cv_rows(max_batch) * 4 * 8)) &&
           ok(s->a2p.alloc((size_t)cv_rows(max_batch) * 4 * 8)) && ok(s->dz3p.alloc((size_t)cv_rows(max_batch) * 4 * 8)) &&
           ok(s->dz2p.alloc((size_t)cv_rows(max_batch) * 4 * 8)) && ok(s->wf2.alloc(32 * 864)) &&
           ok(s->wf3.alloc(32 * 864))))
         return MB_ERR_CUDA;
     if (cudaMemset(s->tc_err.p, 0, sizeof(uint32_t)) != cudaSuccess) return MB_ERR_CUDA;
+    if (cudaMemset(s->done.p, 0, sizeof(uint32_t)) != cudaSuccess) return MB_ERR_CUDA;
     if (cudaDeviceGetAttribute(&s->num_sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return MB_ERR_CUDA;
     // He-normal weights (fan-in of the real inputs), zero biases, zero
     // weights on the padding channels of W1; Box-Muller over SplitMix64.
