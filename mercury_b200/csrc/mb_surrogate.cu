@@ -349,7 +349,14 @@ __global__ void __launch_bounds__(kTcThreads) gemm_tc_kernel(const GemmArgs g, u
                            "=r"(r[7])
                          : "r"(taddr));
             asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-            if (row < g.M) {
+            if (row < g.M && gridDim.y > 1 && c0 + 8 <= g.N && g.N % 4 == 0) {
+                // whole sectors: 8 separate stores a lane were half of the
+                // flatten layer (25 us at 256 samples, 39 at 1,024; now 12
+                // and 19)
+                float4* out = reinterpret_cast<float4*>(g.partial + ((size_t)blockIdx.y * g.M + row) * g.N + c0);
+                out[0] = make_float4(__uint_as_float(r[0]), __uint_as_float(r[1]), __uint_as_float(r[2]), __uint_as_float(r[3]));
+                out[1] = make_float4(__uint_as_float(r[4]), __uint_as_float(r[5]), __uint_as_float(r[6]), __uint_as_float(r[7]));
+            } else if (row < g.M) {
 #pragma unroll
                 for (int j = 0; j < 8; ++j) {
                     const int col = c0 + j;
@@ -422,6 +429,7 @@ template <int P>
 __global__ void __launch_bounds__(128) conv_tc_kernel(const ConvTcArgs g) {
     extern __shared__ __align__(1024) uint8_t cv_smem[];
     __shared__ __align__(8) uint64_t bars[2];
+    __shared__ float bias[32];
     __shared__ uint32_t tmem_slot;
     constexpr int K = 27 * 8 * P;
     constexpr int kWChunks = P == 1 ? 28 : K / 8;           // 8-element k chunks (one zero chunk pads K = 216)
@@ -432,6 +440,7 @@ __global__ void __launch_bounds__(128) conv_tc_kernel(const ConvTcArgs g) {
     uint8_t* sw = cv_smem;
     uint8_t* sa[2] = {cv_smem + kWBytes, cv_smem + kWBytes + kABytes};
     const int rows = (int)cv_rows((uint32_t)g.n), tiles = rows / kCvTile, real_rows = g.n * kCvGenome;
+    if (tid < 32) bias[tid] = g.bias ? g.bias[tid] : 0.0f;
     if (tid == 0) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&bars[0])));
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&bars[1])));
@@ -461,26 +470,42 @@ __global__ void __launch_bounds__(128) conv_tc_kernel(const ConvTcArgs g) {
         const int x = loc % kCvSide, y = (loc / kCvSide) % kCvSide, z = loc / (kCvSide * kCvSide);
         const bool real = b < g.n && x < 6 && y < 6 && z < 6;
         const int v = x + 6 * y + 36 * z;
+        // the row's 32 columns together: one wait, and the masks' loads in
+        // flight (1,024 samples, 32 channels: 53 -> 47 us, with the compact
+        // copy left out where nothing reads it)
+        uint4 mask4[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+            mask4[c] = g.mask && real ? *reinterpret_cast<const uint4*>(g.mask + ((size_t)b * 216 + v) * 32 + 8 * c)
+                                      : make_uint4(0, 0, 0, 0);
+        uint32_t r[32];
+#pragma unroll
+        for (int c = 0; c < 32; c += 8)
+            asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
+                         : "=r"(r[c]), "=r"(r[c + 1]), "=r"(r[c + 2]), "=r"(r[c + 3]), "=r"(r[c + 4]), "=r"(r[c + 5]),
+                           "=r"(r[c + 6]), "=r"(r[c + 7])
+                         : "r"(acc + ((uint32_t)(warp * 32) << 16) + (uint32_t)c));
+        asm volatile("tcgen05.wait::ld.sync.aligned;\n"
+                     : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
+                       "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15]),
+                       "+r"(r[16]), "+r"(r[17]), "+r"(r[18]), "+r"(r[19]), "+r"(r[20]), "+r"(r[21]), "+r"(r[22]), "+r"(r[23]),
+                       "+r"(r[24]), "+r"(r[25]), "+r"(r[26]), "+r"(r[27])
+                     :
+                     : "memory");
+        asm volatile("" : "+r"(r[28]), "+r"(r[29]), "+r"(r[30]), "+r"(r[31])::"memory");
 #pragma unroll
         for (int c0 = 0; c0 < 32; c0 += 8) {
-            uint32_t r[8];
-            asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
-                         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-                           "=r"(r[7])
-                         : "r"(acc + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0));
-            asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
             alignas(16) bf16 h[8];
             if (g.mask) {
                 alignas(16) bf16 mk[8];
-                *reinterpret_cast<uint4*>(mk) =
-                    real ? *reinterpret_cast<const uint4*>(g.mask + ((size_t)b * 216 + v) * 32 + c0) : make_uint4(0, 0, 0, 0);
+                *reinterpret_cast<uint4*>(mk) = mask4[c0 / 8];
 #pragma unroll
                 for (int j = 0; j < 8; ++j)
-                    h[j] = __float2bfloat16_rn(__bfloat162float(mk[j]) > 0.0f ? __uint_as_float(r[j]) : 0.0f);
+                    h[j] = __float2bfloat16_rn(__bfloat162float(mk[j]) > 0.0f ? __uint_as_float(r[c0 + j]) : 0.0f);
             } else {
 #pragma unroll
                 for (int j = 0; j < 8; ++j)
-                    h[j] = __float2bfloat16_rn(real ? fmaxf(__uint_as_float(r[j]) + g.bias[c0 + j], 0.0f) : 0.0f);
+                    h[j] = __float2bfloat16_rn(real ? fmaxf(__uint_as_float(r[c0 + j]) + bias[c0 + j], 0.0f) : 0.0f);
             }
             const uint4 pk = *reinterpret_cast<const uint4*>(h);
             if (g.out_planar) *reinterpret_cast<uint4*>(g.out_planar + ((size_t)(c0 / 8) * rows + p) * 8) = pk;
@@ -1111,9 +1136,11 @@ GemmArgs args(mb_surrogate* s, const bf16* A, int lda, const bf16* B, int ldb, i
     return a;
 }
 
-// Forward of n samples already one-hot in s->x0; leaves a1..a3, h1, h2, y.
-// The products run on tcgen05 (or, when switched off, on mma.sync).
-cudaError_t forward(mb_surrogate* s, uint32_t n) {
+// Forward of n samples (classes in s->cls; one-hot in s->x0 unless !keep on
+// tcgen05); leaves a1..a3 (a3 only, unless keep: the compact a1, a2 are read by
+// the backward pass alone), h1, h2, y.  The products run on tcgen05 (or, when
+// switched off, on mma.sync).
+cudaError_t forward(mb_surrogate* s, uint32_t n, bool keep) {
     cudaStream_t st = s->stream;
     const int R = (int)n * kVox;
     cudaError_t e;
@@ -1139,8 +1166,8 @@ cudaError_t forward(mb_surrogate* s, uint32_t n) {
     };
     if (s->tcgen05) {
         onehot_planar_kernel<<<std::min<uint32_t>((cv_rows(n) + 255) / 256, 4096), 256, 0, st>>>(s->cls.p, n, s->x0p.p);
-        const ConvTcArgs c1{s->x0p.p, 1, PB(s, kW1), P(s, kB1), (int)n, s->a1p.p, s->a1.p, s->tc_err.p};
-        const ConvTcArgs c2{s->a1p.p, 4, PB(s, kW2), P(s, kB2), (int)n, s->a2p.p, s->a2.p, s->tc_err.p};
+        const ConvTcArgs c1{s->x0p.p, 1, PB(s, kW1), P(s, kB1), (int)n, s->a1p.p, keep ? s->a1.p : nullptr, s->tc_err.p};
+        const ConvTcArgs c2{s->a1p.p, 4, PB(s, kW2), P(s, kB2), (int)n, s->a2p.p, keep ? s->a2.p : nullptr, s->tc_err.p};
         const ConvTcArgs c3{s->a2p.p, 4, PB(s, kW3), P(s, kB3), (int)n, nullptr, s->a3.p, s->tc_err.p};
         if ((e = conv_tc<1>(c1, s->num_sms, st)) != cudaSuccess) return e;
         if ((e = conv_tc<4>(c2, s->num_sms, st)) != cudaSuccess) return e;
@@ -1266,11 +1293,13 @@ cudaError_t backward(mb_surrogate* s, uint32_t n) {
     return cudaGetLastError();
 }
 
+// (the one-hot input of the tcgen05 forward is made in its own layout)
 mb_status upload_batch(mb_surrogate* s, const uint8_t* genomes, const float* targets, uint32_t n) {
     cudaStream_t st = s->stream;
     SG_CUDA(s, cudaMemcpyAsync(s->cls.p, genomes, (size_t)n * kVox, cudaMemcpyHostToDevice, st));
     if (targets) SG_CUDA(s, cudaMemcpyAsync(s->t.p, targets, n * sizeof(float), cudaMemcpyHostToDevice, st));
-    onehot_kernel<<<std::min<uint32_t>((n * kVox + 255) / 256, 4096), 256, 0, st>>>(s->cls.p, n * kVox, s->x0.p);
+    if (targets || !s->tcgen05)
+        onehot_kernel<<<std::min<uint32_t>((n * kVox + 255) / 256, 4096), 256, 0, st>>>(s->cls.p, n * kVox, s->x0.p);
     SG_CUDA(s, cudaGetLastError());
     return MB_OK;
 }
@@ -1384,7 +1413,7 @@ mb_status mb_surrogate_predict(mb_surrogate* s, const uint8_t* genomes, uint32_t
         const uint32_t nb = std::min(s->max_batch, n - b0);
         const mb_status st = upload_batch(s, genomes + (size_t)b0 * kVox, nullptr, nb);
         if (st != MB_OK) return st;
-        SG_CUDA(s, forward(s, nb));
+        SG_CUDA(s, forward(s, nb, false));
         SG_CUDA(s, cudaMemcpyAsync(out + b0, s->y.p, nb * sizeof(float), cudaMemcpyDeviceToHost, s->stream));
     }
     SG_CUDA(s, cudaStreamSynchronize(s->stream));
@@ -1399,7 +1428,7 @@ mb_status mb_surrogate_gradients(mb_surrogate* s, const uint8_t* genomes, const 
     mb_status st = upload_batch(s, genomes, targets, n);
     if (st != MB_OK) return st;
     SG_CUDA(s, cudaMemsetAsync(s->g.p, 0, kLayout.off[kTensors] * sizeof(float), s->stream));
-    SG_CUDA(s, forward(s, n));
+    SG_CUDA(s, forward(s, n, true));
     SG_CUDA(s, backward(s, n));
     if (grads)
         SG_CUDA(s, cudaMemcpyAsync(grads, s->g.p, kLayout.off[kTensors] * sizeof(float), cudaMemcpyDeviceToHost,
