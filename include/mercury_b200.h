@@ -294,8 +294,8 @@ MB_API mb_status mb_set_launch_config(mb_context* ctx, const mb_launch_config* c
 
 /* The step kernel the next launches of the uploaded batch use:
  * *register_rows = 1 when each mass's row of incident springs is held per
- * thread (resident bins of a 1,024-thread shape with at most one mass per
- * thread and no face drag), else 0; *smem_bytes = the dynamic shared memory
+ * thread (resident bins of a 1,024-thread shape with at most 1,024 masses a
+ * bin and 26 springs a mass), else 0; *smem_bytes = the dynamic shared memory
  * per CTA of those launches (without stress tracking).  May wait for the
  * stream.  Either pointer may be NULL.  No reference counterpart. */
 MB_API mb_status mb_get_step_variant(const mb_context* ctx, uint32_t* register_rows, uint32_t* smem_bytes);

@@ -312,7 +312,7 @@ class Simulator:
 
     def step_variant(self) -> dict:
         """The step kernel the next launches use (mb_get_step_variant):
-        register_rows (each mass's row held in registers) and the dynamic
+        register_rows (1 when each mass's row is held per thread) and the dynamic
         shared memory per CTA."""
         rr, smem = ctypes.c_uint32(), ctypes.c_uint32()
         _lib.check(_lib.LIB.mb_get_step_variant(self._ctx, ctypes.byref(rr), ctypes.byref(smem)), self._ctx)
