@@ -333,7 +333,7 @@ def run_ours(args, rank, local_rank, world):
                      "bytes_per_update": SMEM_B,
                      "peak_source": f"measured: shared-memory read probe (mb_measure_smem_bandwidth) on this GPU, "
                                     f"{smem_clk:.1f} B/clk/SM",
-                     "kernel": "step_kernel (resident: robots on chip for the whole launch)"},
+                     "kernel": "tm_step_kernel (resident: robots on chip for the whole launch)"},
         "roofline_hbm": {"bound": "hbm", "achieved": hbm_ach, "peak": hbm_peak, "unit": "GB/s",
                          "frac": hbm_ach / hbm_peak, "bytes_per_update": hbm_b, "peak_source": hbm_src,
                          "note": "the HBM bytes a step that keeps nothing on chip (the reference's design) "
