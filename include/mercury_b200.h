@@ -330,6 +330,12 @@ typedef struct mb_plan_stats {
 MB_API mb_status mb_plan_population(const mb_batch_desc* batch, const mb_launch_config* cfg,
                                     uint32_t num_sms, uint32_t smem_bytes, mb_plan_stats* stats);
 
+/* What mb_get_step_variant will report for the population, with or without
+ * stress tracking and face drag, planned like mb_plan_population.  Host only. */
+MB_API mb_status mb_plan_step_variant(const mb_batch_desc* batch, const mb_launch_config* cfg, uint32_t num_sms,
+                                      uint32_t smem_bytes, int track_stresses, int face_drag, uint32_t* register_rows,
+                                      uint32_t* cta_smem_bytes);
+
 /* Compiled kernel shapes, for autotuners: writes up to `capacity` entries
  * (threads, springs_per_thread, masses_per_thread; streamed = 1 for the
  * streamed kernel, whose springs_per_thread is 0) and returns the count.  No

@@ -117,6 +117,8 @@ def _load() -> ctypes.CDLL:
         "mb_kernel_shapes": (U32, [ctypes.POINTER(LaunchConfig), U32]),
         "mb_plan_population": (I32, [ctypes.POINTER(BatchDesc), ctypes.POINTER(LaunchConfig), U32, U32,
                                      ctypes.POINTER(PlanStats)]),
+        "mb_plan_step_variant": (I32, [ctypes.POINTER(BatchDesc), ctypes.POINTER(LaunchConfig), U32, U32, I32, I32,
+                                       ctypes.POINTER(U32), ctypes.POINTER(U32)]),
         "mb_voxel_build": (I32, [I32, I32, I32, F32, P, ctypes.POINTER(I32), ctypes.POINTER(I32), P, P, P, P, P]),
         "mb_devo": (I32, [P, U32, ctypes.c_uint64, U32, ctypes.POINTER(U32)]),
         "mb_collect_springs": (I32, [P, P, P, P]),

@@ -954,6 +954,21 @@ mb_status voxel_setup(mb_context* c, uint32_t R, int sx, int sy, int sz, float h
     return MB_OK;
 }
 
+// Planning on the host, without a GPU (zero SMs or shared memory: B200's).
+constexpr uint32_t kPlanSmem = 232448;
+mb_status plan_packed(const mb_batch_desc* batch, const mb_launch_config* cfg, uint32_t num_sms, uint32_t smem_bytes,
+                      mb::Packed& out) {
+    if (!batch || batch->n_robots == 0 || !batch->mass_offsets || !batch->spring_offsets || !batch->mass_material ||
+        (batch->spring_offsets[batch->n_robots] && (!batch->pairs || !batch->spring_material || !batch->lbar)))
+        return MB_ERR_ARGUMENT;
+    mb::PackOptions po;
+    po.sms = num_sms ? num_sms : 148;
+    po.smem_cap = smem_bytes ? smem_bytes : kPlanSmem;
+    if (cfg) po.override = *cfg;
+    std::string err;
+    return mb::pack_population(batch, po, out, err);
+}
+
 }  // namespace mb_detail
 
 extern "C" {
@@ -1089,17 +1104,9 @@ mb_status mb_get_packed_springs(const mb_context* ctx, uint32_t* words, uint64_t
 
 mb_status mb_plan_population(const mb_batch_desc* batch, const mb_launch_config* cfg, uint32_t num_sms,
                              uint32_t smem_bytes, mb_plan_stats* stats) {
-    if (!batch || !stats || batch->n_robots == 0 || !batch->mass_offsets || !batch->spring_offsets ||
-        !batch->mass_material || (batch->spring_offsets[batch->n_robots] &&
-                                  (!batch->pairs || !batch->spring_material || !batch->lbar)))
-        return MB_ERR_ARGUMENT;
-    mb::PackOptions po;
-    po.sms = num_sms ? num_sms : 148;
-    po.smem_cap = smem_bytes ? smem_bytes : 232448;
-    if (cfg) po.override = *cfg;
+    if (!stats) return MB_ERR_ARGUMENT;
     mb::Packed out;
-    std::string err;
-    const mb_status st = mb::pack_population(batch, po, out, err);
+    const mb_status st = mb_detail::plan_packed(batch, cfg, num_sms, smem_bytes, out);
     if (st != MB_OK) return st;
     std::memset(stats, 0, sizeof(*stats));
     stats->threads = out.shape.threads;
@@ -1131,6 +1138,28 @@ mb_status mb_plan_population(const mb_batch_desc* batch, const mb_launch_config*
     stats->ctas = ctas;
     stats->max_cta_springs = per.empty() ? 0 : (uint32_t)*std::max_element(per.begin(), per.end());
     stats->min_cta_springs = per.empty() ? 0 : (uint32_t)*std::min_element(per.begin(), per.end());
+    return MB_OK;
+}
+
+mb_status mb_plan_step_variant(const mb_batch_desc* batch, const mb_launch_config* cfg, uint32_t num_sms,
+                               uint32_t smem_bytes, int track_stresses, int face_drag, uint32_t* register_rows,
+                               uint32_t* cta_smem_bytes) {
+    mb::Packed out;
+    const mb_status st = mb_detail::plan_packed(batch, cfg, num_sms, smem_bytes, out);
+    if (st != MB_OK) return st;
+    uint32_t most = 0;
+    for (const auto& d : out.bins) most = std::max(most, d.n_mass);
+    mb::TmPlan plan;
+    if (mb::tm_holds(out.shape, out.streamed, out.cluster, most, out.max_degree)) {
+        std::vector<uint32_t> slots;
+        for (const auto& d : out.bins)
+            slots.push_back(mb::tm_count_slots(d, out.pair.data(), out.inc.data(), out.slice_off.data(), out.slice_width.data()));
+        mb::tm_plan(out.bins, slots, out.grid ? out.grid : out.n_bins, (uint32_t)out.mat_ids.size(),
+                    smem_bytes ? smem_bytes : mb_detail::kPlanSmem, mb::tm_max_mpt(track_stresses != 0),
+                    face_drag && !out.face_row.empty(), plan);
+    }
+    if (register_rows) *register_rows = plan.ok ? 1u : 0u;
+    if (cta_smem_bytes) *cta_smem_bytes = plan.ok ? plan.smem : out.max_smem;
     return MB_OK;
 }
 
@@ -1288,8 +1317,7 @@ namespace mb_detail {
 // springs than a lattice has when uploaded (the kernel stays correct when
 // development adds some, reading longer rows from global memory).
 bool tm_eligible(const mb_context* c) {
-    return !c->streamed && !c->cluster && mb::tm_shape(c->shape) &&
-           c->max_bin_mass <= c->shape.threads && c->max_degree <= mb::kTmMaxDegree;
+    return mb::tm_holds(c->shape, c->streamed, c->cluster, c->max_bin_mass, c->max_degree);
 }
 
 // The rows of the tensor-memory kernel, when the packed rows changed (waits
@@ -1332,9 +1360,8 @@ cudaError_t tm_update(mb_context* c, bool track) {
     if (l.planned && l.plan.faces == faces) return cudaSuccess;
     if (l.planned) c->clear_graphs();  // they hold the plan without, or with, faces
     l.planned = false;
-    // stresses add to a thread's words: one mass per thread then
     mb::tm_plan(c->h_bins, c->tm_slots, c->grid ? c->grid : c->n_bins, c->n_mat_host, mb::max_step_smem(c->device),
-                track ? 1u : mb::kTmMaxMpt, faces, l.plan);
+                mb::tm_max_mpt(track), faces, l.plan);
     if (l.plan.ok) {
         std::vector<uint8_t> host;
         auto put = [&](const auto& v) {

@@ -112,6 +112,7 @@ struct TmBin {
     // half that of the positions, slot 0's force
     uint32_t n_face, face0, v_base, face_xy, face_z;
 };
+static_assert(sizeof(TmBin) * kTmMaxGroups + sizeof(uint32_t) <= kTmHeadBytes, "");
 
 // Operand of an own spring: address of the other end | of the material
 // factors << 16.
@@ -148,15 +149,16 @@ template <int MODE, bool TRACK, int MPT, bool WIDE>
 __global__ void __launch_bounds__(32 * (WIDE ? kTmWideWarps : kTmMaxWarps), 1) tm_step_kernel(const __grid_constant__ TmParams q) {
     constexpr bool XPBD = MODE == kModeXpbd;
     constexpr bool FACES = MODE == kModeForceWaterFaces;  // face drag compiled in
+    // (all shared memory is dynamic, so that the plan's sum is what a launch asks
+    // for; its first kTmHeadBytes: every group's TmBin, the allocation's word)
     extern __shared__ __align__(128) uint8_t tm_smem[];
-    __shared__ uint32_t tmem_slot;
-    __shared__ TmBin bin_all[kTmMaxGroups];
+    TmBin* const bin_all = reinterpret_cast<TmBin*>(tm_smem);
     const StepParams& p = q.p;
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     // the CTA's columns, a power of two, shared by its warps' four lane quarters
     const uint32_t per_quarter = (blockDim.x / 32 + 3) / 4;
     const uint32_t cols = per_quarter <= 2 ? 256u : 512u, my_cols = (cols / per_quarter) & ~3u;
-    const uint32_t tmem0 = tm_alloc(&tmem_slot, cols);
+    const uint32_t tmem0 = tm_alloc(reinterpret_cast<uint32_t*>(bin_all + kTmMaxGroups), cols);
     const uint32_t tm = tmem0 + ((warp & 3u) << 21) + (warp >> 2) * my_cols;  // this warp's words
 
     // this warp's group (lane g of 8 looks at group g); warps without one wait
@@ -831,7 +833,7 @@ const TmFn kTm[4][2][3] = {MB_TM(kModeXpbd), MB_TM(kModeForceLand), MB_TM(kModeF
 #undef MB_TM
 
 TmFn tm_kernel(uint32_t mode, bool track, const TmPlan& plan) {
-    if (mode > kModeForceWater || !plan.ok || plan.mpt < 1 || plan.mpt > (track ? 1u : kTmMaxMpt)) return nullptr;
+    if (mode > kModeForceWater || !plan.ok || plan.mpt < 1 || plan.mpt > tm_max_mpt(track)) return nullptr;
     if (plan.faces) {
         if (mode != kModeForceWater) return nullptr;
         mode = kModeForceWaterFaces;
@@ -857,6 +859,33 @@ cudaError_t launch_tm(const TmParams& q, const TmPlan& plan, cudaStream_t s) {
     if (!f) return cudaErrorInvalidValue;
     f<<<plan.ctas, plan.threads, plan.smem, s>>>(q);
     return cudaGetLastError();
+}
+
+uint32_t tm_count_slots(const BinDesc& d, const uint32_t* pair, const uint16_t* inc, const uint32_t* slice_off,
+                        const uint32_t* slice_width) {
+    uint32_t slots = kTmZeros;
+    for (uint32_t sl = 0; sl < (d.n_mass + 31) / 32; ++sl) {
+        const uint32_t gs = d.slice_begin + sl;
+        const uint16_t* row = inc + d.inc_begin + slice_off[gs];
+        uint32_t n[32] = {}, own_columns = 0;
+        bool pure = true;  // every column is all own or all to gather
+        for (uint32_t k = 0; k < slice_width[gs]; ++k) {
+            bool own = false, gather = false;
+            for (uint32_t l = 0; l < 32; ++l) {
+                const uint32_t e = row[32 * k + l], m = 32 * sl + l;
+                if (e == kPadEntry) continue;
+                const uint32_t w = pair[d.spring_begin + (e >> 1)], other = (e & 1u) ? w & 0xFFFu : (w >> 12) & 0xFFFu;
+                const bool mine = other < m || (other == m && (e & 1u));
+                own |= mine;
+                gather |= other > m;
+                n[l] += mine;
+            }
+            own_columns += own;
+            pure &= !(own && gather);
+        }
+        slots += 32 * (pure ? own_columns : *std::max_element(n, n + 32));
+    }
+    return slots;
 }
 
 void tm_plan(const std::vector<BinDesc>& bins, const std::vector<uint32_t>& slots, uint32_t ctas, uint32_t n_mat,
@@ -915,6 +944,7 @@ void tm_plan(const std::vector<BinDesc>& bins, const std::vector<uint32_t>& slot
                 off += (bytes + 127u) & ~127u;
                 return at;
             };
+            take(kTmHeadBytes);
             for (uint32_t g = 0; g < G; ++g) {
                 groups[g].mat_off = take(8u * (n_mat + 1));
                 groups[g].x_off = take(16u * (kTmStandIns + 32 * most[g]));

@@ -34,13 +34,20 @@ constexpr uint32_t kTmMaxMpt = 2;         // masses per thread
 constexpr uint32_t kTmZeros = 32;         // zero slots before a bin's corrections, one per bank
 constexpr uint32_t kTmStandIns = 8;       // stand-in positions before a bin's, one per bank group
 constexpr uint32_t kTmSmemBase = 4096;    // bound on the address where dynamic shared memory starts
+constexpr uint32_t kTmHeadBytes = 512;    // start of the dynamic shared memory: what the groups need of their bins
 constexpr uint32_t kTmMaxSlices = 128;    // slices of 32 masses per bin
 constexpr uint32_t kTmSpareWords = 8;     // gather words of a slice kept in shared memory when the columns are full
+
+// Masses per thread: stresses add to a thread's words, one mass then.
+inline uint32_t tm_max_mpt(bool track) { return track ? 1u : kTmMaxMpt; }
 
 // Populations the kernel steps: resident bins of a 1,024-thread shape with at
 // most one mass per thread, no mass with more springs than a lattice has.
 constexpr uint32_t kTmMaxDegree = 26;
 inline bool tm_shape(const KernelShape& s) { return s.threads == 1024 && (s.spt == 8 || s.spt == 10 || s.spt == 12); }
+inline bool tm_holds(const KernelShape& s, bool streamed, uint32_t cluster, uint32_t max_bin_mass, uint32_t max_degree) {
+    return !streamed && !cluster && tm_shape(s) && max_bin_mass <= s.threads && max_degree <= kTmMaxDegree;
+}
 
 // The launch of a population: which warps of which CTA step which bins.
 struct TmPlan {
@@ -57,6 +64,11 @@ struct TmPlan {
 // no arrangement.
 void tm_plan(const std::vector<BinDesc>& bins, const std::vector<uint32_t>& slots, uint32_t ctas, uint32_t n_mat,
              uint32_t smem_cap, uint32_t max_mpt, bool faces, TmPlan& out);
+
+// Correction slots of a bin from its SELL rows on the host, as the row kernel
+// counts them (launch planning without a GPU).
+uint32_t tm_count_slots(const BinDesc& bin, const uint32_t* pair, const uint16_t* inc, const uint32_t* slice_off,
+                        const uint32_t* slice_width);
 
 // Rows of the step kernel, from the SELL rows.  Every spring belongs to its
 // end of higher index (the owner).  Per slice of 32 masses:

@@ -353,13 +353,28 @@ def body_length(batch: Batch) -> np.ndarray:
     return out
 
 
+def _launch_config(cfg: dict):
+    return _lib.LaunchConfig(cfg.get("threads", 0), cfg.get("springs_per_thread", 0),
+                             cfg.get("masses_per_thread", 0), cfg.get("bins", 0), cfg.get("chunk", 0),
+                             cfg.get("use_graph", 1), cfg.get("streamed", 0), cfg.get("cluster", 0))
+
+
+def plan_step_variant(batch: Batch, track_stresses: bool = False, face_drag: bool = False, num_sms: int = 148,
+                      smem_bytes: int = 0, **cfg) -> dict:
+    """What Simulator.step_variant will report for the population, planned on
+    the host without a GPU (mb_plan_step_variant)."""
+    d, c = _desc(batch), _launch_config(cfg)
+    rr, smem = ctypes.c_uint32(), ctypes.c_uint32()
+    _lib.check(_lib.LIB.mb_plan_step_variant(ctypes.byref(d), ctypes.byref(c), num_sms, smem_bytes,
+                                             int(track_stresses), int(face_drag), ctypes.byref(rr), ctypes.byref(smem)))
+    return {"register_rows": rr.value, "smem_bytes": smem.value}
+
+
 def plan(batch: Batch, num_sms: int = 148, smem_bytes: int = 0, **cfg) -> dict:
     """Launch plan of a population computed on the host, without a GPU
     (mb_plan_population): shape, bins, path and packed-layout statistics."""
     d = _desc(batch)
-    c = _lib.LaunchConfig(cfg.get("threads", 0), cfg.get("springs_per_thread", 0),
-                          cfg.get("masses_per_thread", 0), cfg.get("bins", 0), cfg.get("chunk", 0),
-                          cfg.get("use_graph", 1), cfg.get("streamed", 0), cfg.get("cluster", 0))
+    c = _launch_config(cfg)
     st = _lib.PlanStats()
     _lib.check(_lib.LIB.mb_plan_population(ctypes.byref(d), ctypes.byref(c), num_sms, smem_bytes,
                                            ctypes.byref(st)))
