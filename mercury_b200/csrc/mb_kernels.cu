@@ -264,6 +264,8 @@ __global__ void __launch_bounds__(T, 1024 / T) step_kernel(const StepParams p) {
                         const float t1 = __fadd_rn(st1, __fmul_rn(XPBD ? lam1 : -lam1, __frcp_rn(lb1)));
                         __syncwarp();
                         tm_st2(ts, __float_as_uint(t0), __float_as_uint(t1));
+                    } else {
+                        __syncwarp();  // the next wait wants the warp together
                     }
                 }
                 asm volatile("tcgen05.wait::ld.sync.aligned;"

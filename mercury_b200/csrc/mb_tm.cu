@@ -117,8 +117,8 @@ static_assert(sizeof(TmBin) * kTmMaxGroups + sizeof(uint32_t) <= kTmHeadBytes, "
 // Operand of an own spring: address of the other end | of the material
 // factors << 16.
 __device__ __forceinline__ uint32_t spring_word(uint32_t entry, uint32_t x0, uint32_t mat0, uint32_t n_mat) {
-    if (entry >> 31) return (x0 + 16u * (entry & 7u)) | (mat0 + 8u * n_mat) << 16;
-    return (x0 + 16u * (kTmStandIns + (entry & 0xFFFFu))) | (mat0 + 8u * (entry >> 16)) << 16;
+    const bool pad = entry >> 31;
+    return (x0 + 16u * (pad ? entry & 7u : kTmStandIns + (entry & 0xFFFFu))) | (mat0 + 8u * (pad ? n_mat : entry >> 16)) << 16;
 }
 
 // Gather word k of a mass's faces (`row`: first entry | count << 24): slots
@@ -300,6 +300,7 @@ __global__ void __launch_bounds__(32 * (WIDE ? kTmWideWarps : kTmMaxWarps), 1) t
                 sts_info(info_mine + j * GT + 16u, tm + free_col + tc.gather, words_kept | words << 16, spare, 0u);
             }
             const uint32_t c0 = tm + free_col;
+            __syncwarp();
 #pragma unroll 4
             for (uint32_t k = 0; k < own_kept; k += 2) {
                 const uint2 e0 = __ldg(&q.r.own[rw + 32 * k]);
@@ -593,6 +594,7 @@ __global__ void __launch_bounds__(32 * (WIDE ? kTmWideWarps : kTmMaxWarps), 1) t
 #pragma unroll
             for (int j = 0; j < MPT; ++j) {
                 if (j >= mine) break;
+                if (j) __syncwarp();  // (the integration before may diverge)
                 const uint4 info = lds_info(info_mine + j * GT + 16u);
                 const uint32_t xy0 = t.xy0, z0 = t.z0;
                 f32x2 fxy = pack2(ax[j], ay[j]);
