@@ -977,7 +977,7 @@ void tm_plan(const std::vector<BinDesc>& bins, const std::vector<uint32_t>& slot
                 groups[g].count = (uint32_t)lists[g].size();
                 for (uint32_t b : lists[g]) {
                     const BinDesc& d = bins[b];
-                    out.bins.push_back({b, d.mass_begin, d.n_mass, d.slice_begin, d.inc_begin, d.face_begin, n_face(b), d.face_inc_begin});
+                    out.bins.push_back({b, d.mass_begin, d.n_mass, d.slice_begin, d.face_begin, n_face(b), d.face_inc_begin});
                 }
                 out.mpt = std::max(out.mpt, (most[g] + warps[g] - 1) / warps[g]);
             }

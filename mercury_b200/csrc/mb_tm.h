@@ -23,7 +23,7 @@ struct alignas(16) TmGroup {
 };
 // A bin of the list: what of its descriptor the kernel reads.
 struct alignas(16) TmBinRef {
-    uint32_t bin, mass_begin, n_mass, slice_begin, inc_begin;
+    uint32_t bin, mass_begin, n_mass, slice_begin;
     uint32_t face_begin, n_face, face_inc_begin;  // (n_face 0 without face drag)
 };
 
