@@ -954,6 +954,18 @@ mb_status voxel_setup(mb_context* c, uint32_t R, int sx, int sy, int sz, float h
     return MB_OK;
 }
 
+mb_status step_variant(const mb_context* ctx, bool track, uint32_t* register_rows, uint32_t* smem_bytes) {
+    if (!ctx) return MB_ERR_ARGUMENT;
+    if (!ctx->loaded) return MB_ERR_STATE;
+    cudaSetDevice(ctx->device);
+    // (the launch plan is made on demand; it is not part of the caller's state)
+    if (tm_eligible(ctx) && tm_update(const_cast<mb_context*>(ctx), track) != cudaSuccess) return MB_ERR_CUDA;
+    const bool tm = use_tm(ctx, track);
+    if (register_rows) *register_rows = tm ? 1u : 0u;
+    if (smem_bytes) *smem_bytes = tm ? ctx->tm[track ? 1 : 0].plan.smem : ctx->smem_bytes;
+    return MB_OK;
+}
+
 // Planning on the host, without a GPU (zero SMs or shared memory: B200's).
 constexpr uint32_t kPlanSmem = 232448;
 mb_status plan_packed(const mb_batch_desc* batch, const mb_launch_config* cfg, uint32_t num_sms, uint32_t smem_bytes,
@@ -1077,15 +1089,11 @@ mb_status mb_get_launch_config(const mb_context* ctx, mb_launch_config* cfg) {
 }
 
 mb_status mb_get_step_variant(const mb_context* ctx, uint32_t* register_rows, uint32_t* smem_bytes) {
-    if (!ctx) return MB_ERR_ARGUMENT;
-    if (!ctx->loaded) return MB_ERR_STATE;
-    cudaSetDevice(ctx->device);
-    // (the launch plan is made on demand; it is not part of the caller's state)
-    if (mb_detail::tm_eligible(ctx) && mb_detail::tm_update(const_cast<mb_context*>(ctx), false) != cudaSuccess) return MB_ERR_CUDA;
-    const bool tm = mb_detail::use_tm(ctx, false);
-    if (register_rows) *register_rows = tm ? 1u : 0u;
-    if (smem_bytes) *smem_bytes = tm ? ctx->tm[0].plan.smem : ctx->smem_bytes;
-    return MB_OK;
+    return mb_detail::step_variant(ctx, false, register_rows, smem_bytes);
+}
+
+mb_status mb_get_tracked_step_variant(const mb_context* ctx, uint32_t* register_rows, uint32_t* smem_bytes) {
+    return mb_detail::step_variant(ctx, true, register_rows, smem_bytes);
 }
 
 mb_status mb_get_packed_springs(const mb_context* ctx, uint32_t* words, uint64_t capacity, uint64_t* count) {
@@ -1155,7 +1163,7 @@ mb_status mb_plan_step_variant(const mb_batch_desc* batch, const mb_launch_confi
         for (const auto& d : out.bins)
             slots.push_back(mb::tm_count_slots(d, out.pair.data(), out.inc.data(), out.slice_off.data(), out.slice_width.data()));
         mb::tm_plan(out.bins, slots, out.grid ? out.grid : out.n_bins, (uint32_t)out.mat_ids.size(),
-                    smem_bytes ? smem_bytes : mb_detail::kPlanSmem, mb::tm_max_mpt(track_stresses != 0),
+                    smem_bytes ? smem_bytes : mb_detail::kPlanSmem, track_stresses != 0,
                     face_drag && !out.face_row.empty(), plan);
     }
     if (register_rows) *register_rows = plan.ok ? 1u : 0u;
@@ -1361,7 +1369,7 @@ cudaError_t tm_update(mb_context* c, bool track) {
     if (l.planned) c->clear_graphs();  // they hold the plan without, or with, faces
     l.planned = false;
     mb::tm_plan(c->h_bins, c->tm_slots, c->grid ? c->grid : c->n_bins, c->n_mat_host, mb::max_step_smem(c->device),
-                mb::tm_max_mpt(track), faces, l.plan);
+                track, faces, l.plan);
     if (l.plan.ok) {
         std::vector<uint8_t> host;
         auto put = [&](const auto& v) {

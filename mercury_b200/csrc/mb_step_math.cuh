@@ -124,6 +124,15 @@ __device__ __forceinline__ void length_and_reciprocal(float s, float& nd, float&
     if (!length_is_fast(nd, e)) length_and_reciprocal_exact(-s, nd, q);
 }
 
+// RN(1 / x) from an approximation of one unit in the last place and one Newton step
+// (Markstein, as above) for ordinary x.  Where it matters the caller compares
+// the result with __frcp_rn once.
+__device__ __forceinline__ float rcp_fast(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return __fmaf_rn(y, __fmaf_rn(-x, y, 1.0f), y);
+}
+
 // Face drag of one surface triangle (water), the share of each corner:
 // mean corner velocity v = (v0 + v1 + v2) * RN(1/3), N = (x1 - x0) x (x2 - x0), A = |N|, unit normal
 // n = N * RN(1/(A + eps)) turned so that v.n > 0 (sim_kernel.cu:106-109),

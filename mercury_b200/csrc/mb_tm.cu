@@ -22,12 +22,17 @@
 //     that one bin's latencies run under another's work.
 //   - Square root and reciprocal come from one approximation and are
 //     correctly rounded without branches (mb_step_math.cuh).
-// A step of those 512 robots then takes 21 wavefronts and 102 instructions
-// per spring, 5.5 us instead of 7.4; 1,638 robots of 6x6x6 cells 19.3 us
-// instead of 23.8.  What bounds it now is issue (69 %) and the warps waiting
-// at barriers (a quarter of the stalls).  24 warps of 80 registers are kept:
-// 28 (72 registers) and 32 (64) spill inside the step and measured 7.4 and
-// 8.3 us, 20 warps 5.4 us there but 25 us on the 6x6x6 robots.
+// A step of those 512 robots then takes 21 wavefronts per 32 springs and 98
+// instructions per spring, 5.3 us instead of 7.3.  What bounds it now is issue
+// (69 %) and the warps waiting at barriers (a quarter of the stalls).  Two
+// kernels: at most 24 warps of 80 registers (they spill 12-52 bytes a thread;
+// 28 warps of 72 registers and 32 of 64 measured 7.4 and 8.3 us there), and at
+// most 16 of up to 128 (WIDE, below); the plan takes the one whose estimated
+// step is shorter.
+// With stress tracking the same 512 robots take 7.8 us (8.5 with the springs
+// in registers and shared memory); bins of 769-1,024 masses, such as two robots
+// of 5-8 cells, run two masses a thread on 16 warps: 260 such robots 5.2 us
+// instead of 6.1.
 // With the face drag, a face is one more correction slot: computed by any
 // thread beside the springs (velocities ride in the positions' w and one more
 // plane: 3 x 24 bytes of loads a face instead of 3 x 32), gathered after the
@@ -37,6 +42,7 @@
 // Same operations in the same order as the oracle: same bits.
 #include <algorithm>
 #include <cmath>
+#include <cstddef>
 #include <type_traits>
 
 #include "mb_step_math.cuh"
@@ -47,8 +53,12 @@ namespace mb {
 
 namespace {
 
+template <bool WIDE>
 __device__ __forceinline__ void group_sync(uint32_t id, uint32_t threads) {
-    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+    if (WIDE && threads == 32)
+        __syncwarp();  // a group of one warp
+    else
+        asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
 
 // Shared memory by 32-bit address: operands hold addresses, so that an
@@ -93,8 +103,8 @@ __device__ __forceinline__ uint4 lds_info(uint32_t a) {
     asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
     return v;
 }
-__device__ __forceinline__ void sts_info(uint32_t a, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
-    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
+__device__ __forceinline__ void sts_info(uint32_t a, uint4 v) {
+    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
 __device__ __forceinline__ void sts1(uint32_t a, float x) {
     asm volatile("st.shared.f32 [%0], %1;" ::"r"(a), "f"(x) : "memory");
@@ -113,6 +123,20 @@ struct TmBin {
     uint32_t n_face, face0, v_base, face_xy, face_z;
 };
 static_assert(sizeof(TmBin) * kTmMaxGroups + sizeof(uint32_t) <= kTmHeadBytes, "");
+template <int OFFSET>
+__device__ __forceinline__ uint32_t bin_word(uint32_t a) {
+    uint32_t v;
+    asm volatile("ld.shared.b32 %0, [%1+%2];" : "=r"(v) : "r"(a), "n"(OFFSET));
+    return v;
+}
+template <int OFFSET>
+__device__ __forceinline__ void set_bin_word(uint32_t a, uint32_t v) {
+    asm volatile("st.shared.b32 [%0+%1], %2;" ::"r"(a), "n"(OFFSET), "r"(v) : "memory");
+}
+// (through one 32-bit address: as a C++ object at the start of the dynamic
+// shared memory it cost the 24-warp kernels registers, and 3 % of a step)
+#define TM_BIN(field) bin_word<(int)offsetof(TmBin, field)>(bin_mine)
+#define TM_BIN_SET(field, v) set_bin_word<(int)offsetof(TmBin, field)>(bin_mine, v)
 
 // Operand of an own spring: address of the other end | of the material
 // factors << 16.
@@ -143,22 +167,27 @@ struct TmColumns {
 
 // WIDE: at most kTmWideWarps warps, so registers for four springs at a time:
 // with few warps an SM, latency has to be hidden within the warp (32 robots of
-// 4x4x4 cells, one an SM: 1.84 -> 1.55 us a step; 5.0 us when they shared
-// four CTAs of the other kernel).
+// 4x4x4 cells, one an SM: 1.84 -> 1.55 us a step; 282 robots of 5-8 cells, two
+// masses a thread: 4.3 us, 5.0 on 24 warps).  The last three of a row go
+// together too, and with one mass a thread the first words are read before the
+// barriers: a robot of one cell, seven springs a row, 1.18 -> 1.08 us, with
+// tracking 1.52 -> 1.16.
 template <int MODE, bool TRACK, int MPT, bool WIDE>
 __global__ void __launch_bounds__(32 * (WIDE ? kTmWideWarps : kTmMaxWarps), 1) tm_step_kernel(const __grid_constant__ TmParams q) {
     constexpr bool XPBD = MODE == kModeXpbd;
     constexpr bool FACES = MODE == kModeForceWaterFaces;  // face drag compiled in
+    // one mass a thread and registers to spare: the slice's data stay in
+    // registers, and the first words are read ahead of the barriers
+    constexpr bool AHEAD = WIDE && MPT == 1;
     // (all shared memory is dynamic, so that the plan's sum is what a launch asks
     // for; its first kTmHeadBytes: every group's TmBin, the allocation's word)
     extern __shared__ __align__(128) uint8_t tm_smem[];
-    TmBin* const bin_all = reinterpret_cast<TmBin*>(tm_smem);
     const StepParams& p = q.p;
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     // the CTA's columns, a power of two, shared by its warps' four lane quarters
     const uint32_t per_quarter = (blockDim.x / 32 + 3) / 4;
     const uint32_t cols = per_quarter <= 2 ? 256u : 512u, my_cols = (cols / per_quarter) & ~3u;
-    const uint32_t tmem0 = tm_alloc(reinterpret_cast<uint32_t*>(bin_all + kTmMaxGroups), cols);
+    const uint32_t tmem0 = tm_alloc(reinterpret_cast<uint32_t*>(tm_smem + kTmMaxGroups * sizeof(TmBin)), cols);
     const uint32_t tm = tmem0 + ((warp & 3u) << 21) + (warp >> 2) * my_cols;  // this warp's words
 
     // this warp's group (lane g of 8 looks at group g); warps without one wait
@@ -189,7 +218,7 @@ __global__ void __launch_bounds__(32 * (WIDE ? kTmWideWarps : kTmMaxWarps), 1) t
     const uint32_t gt = gw * 32 + lane;    // thread of the group
     const uint32_t GT = 32u * grp.warps;   // the group's threads
     const uint32_t bar = 1 + gi;
-    volatile TmBin& t = bin_all[gi];
+    const uint32_t bin_mine = smem_addr(tm_smem) + gi * (uint32_t)sizeof(TmBin);
     const float dt = p.dt;
     // shared memory of the group: material factors {dL0 sin(..), 1/K}, the
     // positions, the corrections
@@ -218,23 +247,23 @@ __global__ void __launch_bounds__(32 * (WIDE ? kTmWideWarps : kTmMaxWarps), 1) t
         for (uint32_t i = gt + GT; i < n_mat; i += GT)
             sts1(mat0 + 8u * i + 4u, __ldg(&p.invk[__ldg(&q.r.mat[256u * ref.bin + i])]));
         if (gt == 0) {
-            t.bin = ref.bin;
-            t.mass_begin = ref.mass_begin;
-            t.n_mass = ref.n_mass;
-            t.slice_begin = ref.slice_begin;
-            t.n_mat = n_mat;
-            t.x0 = x0;
-            t.mat0 = mat0;
-            t.xy0 = xy0;
-            t.z0 = z0;
-            t.row = *p.n_mat;
+            TM_BIN_SET(bin, ref.bin);
+            TM_BIN_SET(mass_begin, ref.mass_begin);
+            TM_BIN_SET(n_mass, ref.n_mass);
+            TM_BIN_SET(slice_begin, ref.slice_begin);
+            TM_BIN_SET(n_mat, n_mat);
+            TM_BIN_SET(x0, x0);
+            TM_BIN_SET(mat0, mat0);
+            TM_BIN_SET(xy0, xy0);
+            TM_BIN_SET(z0, z0);
+            TM_BIN_SET(row, *p.n_mat);
             if (FACES) {
                 const uint32_t slots = __ldg(&q.r.n_slots[ref.bin]);
-                t.n_face = ref.n_face;
-                t.face0 = smem0 + grp.face_off;
-                t.v_base = smem0 + grp.v_off - x0 / 2;
-                t.face_xy = xy0 + 8u * slots;
-                t.face_z = z0 + 4u * slots;
+                TM_BIN_SET(n_face, ref.n_face);
+                TM_BIN_SET(face0, smem0 + grp.face_off);
+                TM_BIN_SET(v_base, smem0 + grp.v_off - x0 / 2);
+                TM_BIN_SET(face_xy, xy0 + 8u * slots);
+                TM_BIN_SET(face_z, z0 + 4u * slots);
             }
             sts2(mat0 + 8u * n_mat, 0.0f, 0.0f);
         }
@@ -258,6 +287,7 @@ __global__ void __launch_bounds__(32 * (WIDE ? kTmWideWarps : kTmMaxWarps), 1) t
         uint32_t gidx = 0;  // WIDE: the mass's index and w components, for the write-back
         float vw = 0.0f;
         uint32_t free_col = 0;
+        uint4 info_own = make_uint4(0, 0, 0, 0), info_gather = info_own;  // AHEAD
 #pragma unroll
         for (int j = 0; j < MPT; ++j) {
             const uint32_t m = gt + j * GT, sl = gw + j * grp.warps;
@@ -274,7 +304,7 @@ __global__ void __launch_bounds__(32 * (WIDE ? kTmWideWarps : kTmMaxWarps), 1) t
                 x[j] = make_float3(P.x, P.y, P.z);
                 mass[j] = P.w;
                 v[j] = make_float3(V.x, V.y, V.z);
-                if (WIDE) {
+                if (WIDE && MPT == 1) {
                     gidx = g;
                     vw = V.w;
                 }
@@ -286,35 +316,43 @@ __global__ void __launch_bounds__(32 * (WIDE ? kTmWideWarps : kTmMaxWarps), 1) t
             // what fits the columns left: own springs first (in pairs), then
             // the gather words
             // (the step loop reads up to two pairs past the last one: room for them)
-            constexpr uint32_t kPast = WIDE && !TRACK ? 8u : 4u;
+            constexpr uint32_t kPast = WIDE ? 8u : 4u;
             const uint32_t left = my_cols - free_col, room = left - kPast;
-            const uint32_t own_kept = left < kPast ? 0u : min(own, TRACK ? 2 * (room / 6u) : 2 * (room / 4u) + 1u);
+            const uint32_t own_kept = left < kPast ? 0u : min(own, TRACK ? 2 * (room / 6u) : 2 * (room / 4u) + (WIDE ? 0u : 1u));
             const TmColumns tc(own_kept, words, TRACK);
             const uint32_t words_kept = tc.gather <= left ? min(words, left - tc.gather) : 0u;
             // gather words that the columns do not hold: in the group's spare
             // shared memory, else in global memory
             const uint32_t spare = j && words > words_kept && words - words_kept <= kTmSpareWords
                                        ? smem0 + grp.spare_off + (128u * kTmSpareWords) * gw : 0u;
-            if (lane == 0) {
-                sts_info(info_mine + j * GT, xy0 + 8u * h.y, z0 + 4u * h.y, own_kept | own << 16, tm + free_col);
-                sts_info(info_mine + j * GT + 16u, tm + free_col + tc.gather, words_kept | words << 16, spare, 0u);
-            }
             const uint32_t c0 = tm + free_col;
             __syncwarp();
 #pragma unroll 4
             for (uint32_t k = 0; k < own_kept; k += 2) {
                 const uint2 e0 = __ldg(&q.r.own[rw + 32 * k]);
-                const uint2 e1 = k + 1 < own_kept ? __ldg(&q.r.own[rw + 32 * (k + 1)]) : make_uint2(1u << 31, 0u);
+                const uint2 e1 = k + 1 < own_kept ? __ldg(&q.r.own[rw + 32 * (k + 1)]) : make_uint2(1u << 31, __float_as_uint(1.0f));
                 tm_st2(c0 + 2 * k, spring_word(e0.x, x0, mat0, n_mat), spring_word(e1.x, x0, mat0, n_mat));
                 tm_st2(c0 + 2 * k + 2, e0.y, e1.y);
             }
+            uint32_t odd = 0;  // some mean length's reciprocal needs the general one
             if (TRACK)
-                for (uint32_t k = 0; k < own_kept; ++k) {
+                for (uint32_t k = 0; k < own; ++k) {
+                    const float lb = __uint_as_float(__ldg(&q.r.own[rw + 32 * k]).y);
+                    odd |= __float_as_uint(rcp_fast(lb)) != __float_as_uint(__frcp_rn(lb));
+                    if (k >= own_kept) continue;
                     const uint32_t g = __ldg(&q.r.gidx[rw + 32 * k]);
                     const float st = g != ~0u ? p.stress[g & 0x7FFFFFFFu] : 0.0f;
                     __syncwarp();
                     tm_st(c0 + tc.stress + k, __float_as_uint(st));
                 }
+            if (TRACK) odd = __any_sync(0xffffffffu, odd);
+            info_own = make_uint4(xy0 + 8u * h.y, z0 + 4u * h.y, own_kept | own << 16 | odd << 31, c0);
+            info_gather = make_uint4(c0 + tc.gather, words_kept | words << 16, spare, 0u);
+            if (lane == 0) {
+                sts_info(info_mine + j * GT, info_own);
+                sts_info(info_mine + j * GT + 16u, info_gather);
+            }
+            __syncwarp();
 #pragma unroll 4
             for (uint32_t k = 0; k < words; ++k) {
                 const uint32_t w = !FACES || k < spring_words
@@ -331,19 +369,19 @@ __global__ void __launch_bounds__(32 * (WIDE ? kTmWideWarps : kTmMaxWarps), 1) t
         }
         tm_wait_st();
         __syncwarp();
-        group_sync(bar, GT);
+        group_sync<WIDE>(bar, GT);
 
         for (uint32_t step = 0; step < p.steps; ++step) {
             // (1) actuation factors (sim_kernel.cu:222); predicted positions
             // x~ = x + v dt (sim_kernel.cu:147-152), or the current ones
             if (my_mat) {
                 sts1(mat_mine, next_rate);
-                rate_at += t.row;
+                rate_at += TM_BIN(row);
                 if (step + 1 < p.steps) next_rate = __ldg(p.rates + rate_at);
             }
             if (more_mats)
-                for (uint32_t i = gt + GT; i < t.n_mat; i += GT)
-                    sts1(t.mat0 + 8u * i, __ldg(p.rates + (size_t)step * t.row + __ldg(&q.r.mat[256u * t.bin + i])));
+                for (uint32_t i = gt + GT; i < TM_BIN(n_mat); i += GT)
+                    sts1(TM_BIN(mat0) + 8u * i, __ldg(p.rates + (size_t)step * TM_BIN(row) + __ldg(&q.r.mat[256u * TM_BIN(bin) + i])));
             float ax[MPT], ay[MPT], az[MPT];
 #pragma unroll
             for (int j = 0; j < MPT; ++j) {
@@ -352,12 +390,29 @@ __global__ void __launch_bounds__(32 * (WIDE ? kTmWideWarps : kTmMaxWarps), 1) t
                                                      __fadd_rn(x[j].z, __fmul_rn(v[j].z, dt)))
                                        : x[j];
                 sts4(x_mine + 16u * j * GT, xt.x, xt.y, xt.z, FACES ? v[j].x : 0.0f);
-                if (FACES) sts2(x_mine / 2 + 8u * j * GT + t.v_base, v[j].y, v[j].z);
+                if (FACES) sts2(x_mine / 2 + 8u * j * GT + TM_BIN(v_base), v[j].y, v[j].z);
             }
             __syncwarp();
-            group_sync(bar, GT);
+            // a slice's next own springs {words, lengths} x 2 (and stresses), the two
+            // after them, and gather words: a block of four, then two and one
+            struct Words {
+                uint32_t c[4], st[2], c2[4], st2[2], g4[4], g2[2], g1[1];
+            } ahead;
+            auto first_springs = [&](const uint4& info, Words& w) {
+                const uint32_t kept = info.z & 0xFFFFu, ta = info.w, ts = ta + 4 * ((kept + 1) / 2);
+                if (!kept) return;
+                tm_ld(ta, w.c);
+                if (TRACK) tm_ld(ts, w.st);
+                if (WIDE) {
+                    tm_ld(ta + 4, w.c2);
+                    if (TRACK) tm_ld(ts + 2, w.st2);
+                }
+            };
+            if (TRACK) tm_wait_st();  // the last step's stresses
+            if (AHEAD && mine) first_springs(info_own, ahead);
+            group_sync<WIDE>(bar, GT);
             if (FACES) {  // the share of each corner, per face, stored like a correction
-                const uint32_t n = t.n_face, face0 = t.face0, vb = t.v_base, fxy = t.face_xy, fz = t.face_z;
+                const uint32_t n = TM_BIN(n_face), face0 = TM_BIN(face0), vb = TM_BIN(v_base), fxy = TM_BIN(face_xy), fz = TM_BIN(face_z);
                 for (uint32_t f = gt; f < n; f += GT) {
                     const float2 c = lds2(face0 + 8u * f);
                     const uint32_t a0 = __float_as_uint(c.x) & 0xFFFFu, a1 = __float_as_uint(c.x) >> 16, a2 = __float_as_uint(c.y);
@@ -374,8 +429,9 @@ __global__ void __launch_bounds__(32 * (WIDE ? kTmWideWarps : kTmMaxWarps), 1) t
 #pragma unroll
             for (int j = 0; j < MPT; ++j) {
                 if (j >= mine) break;
-                const uint4 info = lds_info(info_mine + j * GT);
-                const uint32_t kept = info.z & 0xFFFFu, own = info.z >> 16, x_first = x_mine - 16u * gt;
+                const uint4 info = AHEAD ? info_own : lds_info(info_mine + j * GT);
+                const uint32_t kept = info.z & 0xFFFFu, own = TRACK ? (info.z >> 16) & 0x7FFFu : info.z >> 16, x_first = x_mine - 16u * gt;
+                const bool plain_rcp = TRACK && info.z >> 31;
                 // this mass's position, negated: differences are sums then
                 f32x2 nxy;
                 float nz;
@@ -416,8 +472,8 @@ __global__ void __launch_bounds__(32 * (WIDE ? kTmWideWarps : kTmMaxWarps), 1) t
                         sz = __fadd_rn(sz, pz);
                     };
                     // stress: lambda/Lbar (reference, sim_kernel.cu:234); k (d - L)/Lbar (force)
-                    auto stressed = [&](float st, float lam, float lb) {
-                        return __fadd_rn(st, __fmul_rn(XPBD ? lam : -lam, __frcp_rn(lb)));
+                    auto stressed = [&](uint32_t st, float lam, float inv) {
+                        return __float_as_uint(__fadd_rn(__uint_as_float(st), __fmul_rn(XPBD ? lam : -lam, inv)));
                     };
                     // reference step: lambda = -C/K, dp = lambda n (sim_kernel.cu:230-232);
                     // force modes: Hooke force, -k (d - L) n
@@ -433,15 +489,18 @@ __global__ void __launch_bounds__(32 * (WIDE ? kTmWideWarps : kTmMaxWarps), 1) t
                     };
                     struct Pair {
                         f32x2 d0, d1, ns, L, nd, r;
-                        float z0, z1, k0, k1, l0, l1;
+                        float z0, z1, k0, k1, i0, i1;  // (i: 1 / mean length, for the stress)
                     };
                     auto load = [&](Pair& u, const uint32_t (&c)[4]) {
                         const float2 m0 = lds2(c[0] >> 16), m1 = lds2(c[1] >> 16);
                         const float n0 = delta(c[0], u.d0, u.z0), n1 = delta(c[1], u.d1, u.z1);
                         u.ns = pack2(n0, n1);
-                        u.l0 = __uint_as_float(c[2]);
-                        u.l1 = __uint_as_float(c[3]);
-                        u.L = pack2(__fmaf_rn(u.l0, m0.x, u.l0), __fmaf_rn(u.l1, m1.x, u.l1));
+                        const float l0 = __uint_as_float(c[2]), l1 = __uint_as_float(c[3]);
+                        u.L = pack2(__fmaf_rn(l0, m0.x, l0), __fmaf_rn(l1, m1.x, l1));
+                        if (TRACK) {
+                            u.i0 = rcp_fast(l0);
+                            u.i1 = rcp_fast(l1);
+                        }
                         u.k0 = m0.y;
                         u.k1 = m1.y;
                     };
@@ -453,7 +512,10 @@ __global__ void __launch_bounds__(32 * (WIDE ? kTmWideWarps : kTmMaxWarps), 1) t
                         unpack2(e, e0, e1);
                         return length_is_fast(nd0, e0) && length_is_fast(nd1, e1);
                     };
-                    auto exact = [&](Pair& u, uint32_t w0, uint32_t w1) {
+                    // (plain_rcp: kept out of the common path, where even a
+                    // branch around the general reciprocal cost 0.3 us of a
+                    // one-warp step)
+                    auto exact = [&](Pair& u, uint32_t w0, uint32_t w1, float l0, float l1) {
                         float n0, n1, d0, d1, r0, r1, L0, L1;
                         unpack2(u.ns, n0, n1);
                         unpack2(u.L, L0, L1);
@@ -463,48 +525,68 @@ __global__ void __launch_bounds__(32 * (WIDE ? kTmWideWarps : kTmMaxWarps), 1) t
                         if (stand_in(w1)) clear(u.d1, u.z1, d1, r1, L1);
                         u.nd = pack2(d0, d1);
                         u.r = pack2(r0, r1);
+                        u.i0 = __frcp_rn(l0);
+                        u.i1 = __frcp_rn(l1);
                         __syncwarp();
                     };
-                    auto finish = [&](const Pair& u, uint32_t off, const uint32_t (&st)[2], uint32_t ts) {
+                    auto finish = [&](const Pair& u, uint32_t off, const uint32_t (&st)[2], uint32_t ts, bool both = true) {
                         float t0, t1, f0, f1;
                         unpack2(add2(u.L, u.nd), t0, t1);  // -C
                         const float lam0 = __fmul_rn(t0, u.k0), lam1 = __fmul_rn(t1, u.k1);
                         unpack2(mul2(pack2(lam0, lam1), u.r), f0, f1);
                         apply(f0, u.d0, u.z0, off);
-                        apply(f1, u.d1, u.z1, off + 1);
+                        if (both) apply(f1, u.d1, u.z1, off + 1);
                         if (TRACK)
-                            tm_st2(ts, __float_as_uint(stressed(__uint_as_float(st[0]), lam0, u.l0)),
-                                   __float_as_uint(stressed(__uint_as_float(st[1]), lam1, u.l1)));
+                            tm_st2(ts, stressed(st[0], lam0, u.i0), stressed(st[1], lam1, u.i1));
                     };
                     uint32_t ta = info.w, ts = ta + 4 * ((kept + 1) / 2);
                     const uint32_t end = ta + 2 * (kept & ~1u);
-                    uint32_t c[4], st[2];
-                    if (kept) {
-                        tm_ld(ta, c);
-                        if (TRACK) tm_ld(ts, st);
-                    }
-                    if (WIDE && !TRACK) {  // four springs at a time
-                        uint32_t c2[4];
-                        if (kept) tm_ld(ta + 4, c2);
-                        while (end - ta >= 8) {
+                    Words own_words, &w0 = AHEAD ? ahead : own_words;
+                    uint32_t(&c)[4] = w0.c, (&c2)[4] = w0.c2, (&st)[2] = w0.st, (&st2)[2] = w0.st2;
+                    if (!AHEAD) first_springs(info, w0);
+                    if (WIDE) {  // four springs at a time, then the rest together
+                        auto wait = [&] {
+                            if (TRACK)
+                                asm volatile("tcgen05.wait::ld.sync.aligned;"
+                                             : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3]), "+r"(c2[0]), "+r"(c2[1]), "+r"(c2[2]), "+r"(c2[3]),
+                                               "+r"(st[0]), "+r"(st[1]), "+r"(st2[0]), "+r"(st2[1]));
+                            else
+                                asm volatile("tcgen05.wait::ld.sync.aligned;"
+                                             : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3]), "+r"(c2[0]), "+r"(c2[1]), "+r"(c2[2]), "+r"(c2[3]));
+                        };
+                        // springs ta .. (the last one of four missing unless `all`), the next four's words in flight
+                        auto four = [&](bool all) {
                             Pair u, w;
-                            asm volatile("tcgen05.wait::ld.sync.aligned;"
-                                         : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3]), "+r"(c2[0]), "+r"(c2[1]), "+r"(c2[2]), "+r"(c2[3]));
+                            wait();
                             load(u, c);
                             load(w, c2);
+                            const uint4 k0 = make_uint4(c[0], c[1], c[2], c[3]), k1 = make_uint4(c2[0], c2[1], c2[2], c2[3]);
+                            const uint32_t s0[2] = {st[0], st[1]}, s1[2] = {st2[0], st2[1]};
                             ta += 8;
                             tm_ld(ta, c);
                             tm_ld(ta + 4, c2);
+                            if (TRACK) {
+                                tm_ld(ts + 4, st);
+                                tm_ld(ts + 6, st2);
+                            }
                             const bool ok0 = lengths(u), ok1 = lengths(w);
                             fast = fast && ok0 && ok1;
-                            finish(u, 0, st, 0);
-                            finish(w, 2, st, 0);
-                            a_xy += 1024u;
-                            a_z += 512u;
-                        }
-                        asm volatile("tcgen05.wait::ld.sync.aligned;" : "+r"(c2[0]), "+r"(c2[1]), "+r"(c2[2]), "+r"(c2[3]));
+                            // (the warp together: tensor-memory accesses want it converged)
+                            if (TRACK && __any_sync(0xffffffffu, !ok0 || !ok1 || plain_rcp)) {
+                                exact(u, k0.x, k0.y, __uint_as_float(k0.z), __uint_as_float(k0.w));
+                                exact(w, k1.x, k1.y, __uint_as_float(k1.z), __uint_as_float(k1.w));
+                            }
+                            finish(u, 0, s0, ts);
+                            finish(w, 2, s1, ts + 2, all);
+                            a_xy += all ? 1024u : 768u;
+                            a_z += all ? 512u : 384u;
+                            ts += 4;
+                        };
+                        while (end - ta >= 8) four(true);
+                        if ((kept & 3u) == 3u) four(false);
+                        wait();
                     }
-                    while (ta != end) {
+                    while (WIDE ? (int32_t)(end - ta) > 0 : ta != end) {
                         Pair u;
                         if (TRACK)
                             asm volatile("tcgen05.wait::ld.sync.aligned;"
@@ -512,36 +594,39 @@ __global__ void __launch_bounds__(32 * (WIDE ? kTmWideWarps : kTmMaxWarps), 1) t
                         else
                             asm volatile("tcgen05.wait::ld.sync.aligned;" : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3]));
                         load(u, c);
-                        const uint32_t st0[2] = {st[0], st[1]}, w0 = c[0], w1 = c[1];
+                        const uint32_t st0[2] = {st[0], st[1]};
+                        const uint4 k0 = make_uint4(c[0], c[1], c[2], c[3]);
                         ta += 4;
                         tm_ld(ta, c);  // the next pair (or words past the last one), in flight during this one's arithmetic
                         if (TRACK) tm_ld(ts + 2, st);
                         const bool ok = lengths(u);
                         fast = fast && ok;
                         // (the warp together: tensor-memory accesses want it converged)
-                        if (TRACK && __any_sync(0xffffffffu, !ok)) exact(u, w0, w1);
+                        if (TRACK && __any_sync(0xffffffffu, !ok || plain_rcp))
+                            exact(u, k0.x, k0.y, __uint_as_float(k0.z), __uint_as_float(k0.w));
                         finish(u, 0, st0, ts);
                         a_xy += 512u;
                         a_z += 256u;
                         ts += 2;
                     }
-                    // one spring from words {w, length}; returns lambda
-                    auto single = [&](uint32_t w, float lb) {
+                    // one spring from words {w, length}; returns the stress after it
+                    auto single = [&](uint32_t w, float lb, uint32_t st) {
                         f32x2 d;
-                        float dz, nd, e, r;
+                        float dz, nd, e, r, inv = TRACK ? rcp_fast(lb) : 0.0f;
                         const float2 mt = lds2(w >> 16);
                         const float n = delta(w, d, dz), L = __fmaf_rn(lb, mt.x, lb);
                         length_and_reciprocal_fast(n, nd, e, r);
-                        if (__any_sync(0xffffffffu, !length_is_fast(nd, e))) {
+                        if (__any_sync(0xffffffffu, !length_is_fast(nd, e) || plain_rcp)) {
                             length_and_reciprocal_exact(n, nd, r);
                             if (stand_in(w)) clear(d, dz, nd, r, L);
+                            if (TRACK) inv = __frcp_rn(lb);
                             __syncwarp();
                         }
                         const float lam = __fmul_rn(__fadd_rn(L, nd), mt.y);
                         apply(__fmul_rn(lam, r), d, dz, 0);
                         a_xy += 256u;
                         a_z += 128u;
-                        return lam;
+                        return stressed(st, lam, inv);
                     };
                     if (kept)  // (loads past the last pair included)
                         asm volatile("tcgen05.wait::ld.sync.aligned;"
@@ -558,26 +643,25 @@ __global__ void __launch_bounds__(32 * (WIDE ? kTmWideWarps : kTmMaxWarps), 1) t
                             tm_ld(info.w + 4 * (k / 2) + (k & 1u), w);
                             tm_ld(info.w + 4 * (k / 2) + (k & 1u) + 2, lb);
                             asm volatile("tcgen05.wait::ld.sync.aligned;" : "+r"(w[0]), "+r"(lb[0]));
-                            single(w[0], __uint_as_float(lb[0]));
+                            single(w[0], __uint_as_float(lb[0]), 0u);
                         }
-                    } else if (kept & 1u) {
-                        const float lb = __uint_as_float(c[2]), s0 = __uint_as_float(st[0]);
-                        const float lam = single(c[0], lb);
-                        if (TRACK) tm_st(ts, __float_as_uint(stressed(s0, lam, lb)));
+                    } else if (WIDE ? (kept & 3u) == 1u : kept & 1u) {
+                        const uint32_t s = single(c[0], __uint_as_float(c[2]), st[0]);
+                        if (TRACK) tm_st(ts, s);
                     }
                     // springs beyond the columns (rows grown by development): from global memory
                     for (uint32_t k = kept; k < own; ++k) {
-                        const uint32_t at = __ldg(&q.r.head[t.slice_begin + gw + j * grp.warps]).z + 32 * k + lane;
+                        const uint32_t at = __ldg(&q.r.head[TM_BIN(slice_begin) + gw + j * grp.warps]).z + 32 * k + lane;
                         const uint2 e = __ldg(&q.r.own[at]);
                         const float lb = __uint_as_float(e.y);
-                        const float lam = single(spring_word(e.x, t.x0, t.mat0, t.n_mat), lb);
+                        float* sp = nullptr;
                         if (TRACK) {
                             const uint32_t g = __ldg(&q.r.gidx[at]);
-                            if (g != ~0u) {
-                                float* sp = &p.stress[g & 0x7FFFFFFFu];
-                                *sp = stressed(*sp, lam, lb);
-                            }
+                            if (g != ~0u) sp = &p.stress[g & 0x7FFFFFFFu];
+                            __syncwarp();
                         }
+                        const uint32_t s = single(spring_word(e.x, TM_BIN(x0), TM_BIN(mat0), TM_BIN(n_mat)), lb, sp ? __float_as_uint(*sp) : 0u);
+                        if (sp) *sp = __uint_as_float(s);
                         __syncwarp();
                     }
                 }
@@ -587,53 +671,54 @@ __global__ void __launch_bounds__(32 * (WIDE ? kTmWideWarps : kTmMaxWarps), 1) t
                 ay[j] = __fsub_rn(0.0f, sy);
                 az[j] = __fsub_rn(0.0f, sz);
             }
-            if (TRACK) tm_wait_st();
-            group_sync(bar, GT);
+            if (AHEAD && mine && (info_gather.y & 0xFFFCu)) tm_ld(info_gather.x, ahead.g4);
+            group_sync<WIDE>(bar, GT);
             // (3) add the corrections of the springs to higher masses, in
             // summation order, and integrate (sim_kernel.cu:246-268)
 #pragma unroll
             for (int j = 0; j < MPT; ++j) {
                 if (j >= mine) break;
                 if (j) __syncwarp();  // (the integration before may diverge)
-                const uint4 info = lds_info(info_mine + j * GT + 16u);
-                const uint32_t xy0 = t.xy0, z0 = t.z0;
+                const uint4 info = AHEAD ? info_gather : lds_info(info_mine + j * GT + 16u);
                 f32x2 fxy = pack2(ax[j], ay[j]);
                 float fz = az[j];
+                const uint32_t sxy0 = AHEAD ? xy0 : TM_BIN(xy0), sz0 = AHEAD ? z0 : TM_BIN(z0);
                 auto add = [&](uint32_t w) {
                     const uint32_t i0 = w & 0xFFFFu, i1 = w >> 16;
-                    const f32x2 c0 = lds_pair(xy0 + 8u * i0), c1 = lds_pair(xy0 + 8u * i1);
-                    const float e0 = lds1(z0 + 4u * i0), e1 = lds1(z0 + 4u * i1);
+                    const f32x2 c0 = lds_pair(sxy0 + 8u * i0), c1 = lds_pair(sxy0 + 8u * i1);
+                    const float e0 = lds1(sz0 + 4u * i0), e1 = lds1(sz0 + 4u * i1);
                     fxy = add2(add2(fxy, c0), c1);
                     fz = __fadd_rn(__fadd_rn(fz, e0), e1);
                 };
-                // blocks of four words, then two and one
                 const uint32_t n = info.y & 0xFFFFu, words = info.y >> 16;
-                uint32_t c = info.x;
-                const uint32_t end = c + (n & ~3u);
-                uint32_t c4[4], c2[2], c1[1];
-                if (n & 2u) tm_ld(end, c2);
-                if (n & 1u) tm_ld(end + (n & 2u), c1);
-                for (; c != end; c += 4) {
-                    tm_ld(c, c4);
-                    asm volatile("tcgen05.wait::ld.sync.aligned;" : "+r"(c4[0]), "+r"(c4[1]), "+r"(c4[2]), "+r"(c4[3]));
+                uint32_t at = info.x;
+                const uint32_t end = at + (n & ~3u);
+                Words own_words, &w0 = AHEAD ? ahead : own_words;
+                uint32_t(&g4)[4] = w0.g4, (&g2)[2] = w0.g2, (&g1)[1] = w0.g1;
+                if (n & 2u) tm_ld(end, g2);
+                if (n & 1u) tm_ld(end + (n & 2u), g1);
+                while (at != end) {
+                    if (!AHEAD || at != info.x) tm_ld(at, g4);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" : "+r"(g4[0]), "+r"(g4[1]), "+r"(g4[2]), "+r"(g4[3]));
+                    at += 4;
 #pragma unroll
-                    for (int u = 0; u < 4; ++u) add(c4[u]);
+                    for (int u = 0; u < 4; ++u) add(g4[u]);
                 }
-                asm volatile("tcgen05.wait::ld.sync.aligned;" : "+r"(c2[0]), "+r"(c2[1]), "+r"(c1[0]));
+                asm volatile("tcgen05.wait::ld.sync.aligned;" : "+r"(g2[0]), "+r"(g2[1]), "+r"(g1[0]));
                 if (n & 2u) {
-                    add(c2[0]);
-                    add(c2[1]);
+                    add(g2[0]);
+                    add(g2[1]);
                 }
-                if (n & 1u) add(c1[0]);
+                if (n & 1u) add(g1[0]);
                 if (words > n) {  // beyond the columns
-                    const uint4 h = __ldg(&q.r.head[t.slice_begin + gw + j * grp.warps]);
+                    const uint4 h = __ldg(&q.r.head[TM_BIN(slice_begin) + gw + j * grp.warps]);
                     auto word = [&](uint32_t k) {
                         if (info.z) return __float_as_uint(lds1(info.z + 128u * (k - n) + 4u * lane));
                         if (!FACES || k < h.x >> 16) return __ldg(&q.r.gather[h.z + lane + 32 * k]);
                         const uint32_t m = gt + j * GT;
-                        return face_word(p.face_inc + p.bins[t.bin].face_inc_begin,
-                                         m < t.n_mass ? __ldg(&p.face_row[t.mass_begin + m]) : 0u, k - (h.x >> 16),
-                                         __ldg(&q.r.n_slots[t.bin]), lane);
+                        return face_word(p.face_inc + p.bins[TM_BIN(bin)].face_inc_begin,
+                                         m < TM_BIN(n_mass) ? __ldg(&p.face_row[TM_BIN(mass_begin) + m]) : 0u, k - (h.x >> 16),
+                                         __ldg(&q.r.n_slots[TM_BIN(bin)]), lane);
                     };
                     for (uint32_t k = n; k < words; ++k) add(word(k));
                     if (FACES) __syncwarp();
@@ -656,19 +741,20 @@ __global__ void __launch_bounds__(32 * (WIDE ? kTmWideWarps : kTmMaxWarps), 1) t
         }
 
         // ---- write back in the upload layout; flag non-finite positions
+        if (TRACK) tm_wait_st();
         bool bad = false;
 #pragma unroll
         for (int j = 0; j < MPT; ++j) {
             const uint32_t m = gt + j * GT;
-            if (m < t.n_mass) {
-                const uint32_t g = WIDE ? gidx : __ldg(&p.mass_gidx[t.mass_begin + m]);
-                p.pos[g] = make_float4(x[j].x, x[j].y, x[j].z, WIDE ? mass[j] : p.pos[g].w);
-                p.vel[g] = make_float4(v[j].x, v[j].y, v[j].z, WIDE ? vw : p.vel[g].w);
+            if (m < TM_BIN(n_mass)) {
+                const uint32_t g = WIDE && MPT == 1 ? gidx : __ldg(&p.mass_gidx[TM_BIN(mass_begin) + m]);
+                p.pos[g] = make_float4(x[j].x, x[j].y, x[j].z, WIDE && MPT == 1 ? mass[j] : p.pos[g].w);
+                p.vel[g] = make_float4(v[j].x, v[j].y, v[j].z, WIDE && MPT == 1 ? vw : p.vel[g].w);
                 bad |= !(isfinite(x[j].x) && isfinite(x[j].y) && isfinite(x[j].z));
             }
             __syncwarp();
             if (TRACK && j < mine) {
-                const uint32_t rw = __ldg(&q.r.head[t.slice_begin + gw + j * grp.warps]).z + lane;
+                const uint32_t rw = __ldg(&q.r.head[TM_BIN(slice_begin) + gw + j * grp.warps]).z + lane;
                 const uint4 info = lds_info(info_mine + j * GT);
                 const uint32_t kept = info.z & 0xFFFFu, ts = info.w + 4 * ((kept + 1) / 2);
                 for (uint32_t k = 0; k < kept; ++k) {
@@ -682,9 +768,9 @@ __global__ void __launch_bounds__(32 * (WIDE ? kTmWideWarps : kTmMaxWarps), 1) t
             }
         }
         __syncwarp();
-        if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(&p.bin_flags[t.bin], 1u);
+        if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(&p.bin_flags[TM_BIN(bin)], 1u);
         __syncwarp();
-        group_sync(bar, GT);  // the group's shared memory is free for its next bin
+        group_sync<WIDE>(bar, GT);  // the group's shared memory is free for its next bin
     }
     tm_free(tmem0, cols);
 }
@@ -828,19 +914,21 @@ __global__ void __launch_bounds__(1024) tm_rows_kernel(const TmSource in, const 
 using TmFn = void (*)(const TmParams);
 #define MB_TM(M)                                                                                                   \
     {                                                                                                              \
-        {tm_step_kernel<M, false, 1, false>, tm_step_kernel<M, false, 2, false>, tm_step_kernel<M, false, 1, true>}, \
-            {tm_step_kernel<M, true, 1, false>, nullptr, tm_step_kernel<M, true, 1, true>},                         \
+        {{tm_step_kernel<M, false, 1, false>, tm_step_kernel<M, false, 2, false>},                                 \
+         {tm_step_kernel<M, false, 1, true>, tm_step_kernel<M, false, 2, true>}},                                  \
+            {{tm_step_kernel<M, true, 1, false>, nullptr},                                                         \
+             {tm_step_kernel<M, true, 1, true>, tm_step_kernel<M, true, 2, true>}},                                \
     }
-const TmFn kTm[4][2][3] = {MB_TM(kModeXpbd), MB_TM(kModeForceLand), MB_TM(kModeForceWater), MB_TM(kModeForceWaterFaces)};
+const TmFn kTm[4][2][2][2] = {MB_TM(kModeXpbd), MB_TM(kModeForceLand), MB_TM(kModeForceWater), MB_TM(kModeForceWaterFaces)};
 #undef MB_TM
 
 TmFn tm_kernel(uint32_t mode, bool track, const TmPlan& plan) {
-    if (mode > kModeForceWater || !plan.ok || plan.mpt < 1 || plan.mpt > tm_max_mpt(track)) return nullptr;
+    if (mode > kModeForceWater || !plan.ok || plan.mpt < 1 || plan.mpt > kTmMaxMpt) return nullptr;
     if (plan.faces) {
         if (mode != kModeForceWater) return nullptr;
         mode = kModeForceWaterFaces;
     }
-    return kTm[mode][track ? 1 : 0][plan.mpt == 1 && plan.threads <= 32 * kTmWideWarps ? 2 : plan.mpt - 1];
+    return kTm[mode][track ? 1 : 0][plan.threads <= 32 * kTmWideWarps ? 1 : 0][plan.mpt - 1];
 }
 
 }  // namespace
@@ -890,104 +978,198 @@ uint32_t tm_count_slots(const BinDesc& d, const uint32_t* pair, const uint16_t* 
     return slots;
 }
 
+namespace {
+
+// One CTA's arrangement: its warp groups.
+struct TmCta {
+    uint32_t n_groups = 0;
+    uint32_t warps[kTmMaxGroups], most[kTmMaxGroups];   // warps; slices of the largest bin
+    uint32_t slots[kTmMaxGroups], faces[kTmMaxGroups];  // most slots (faces' included) and faces of a bin
+};
+
+// Shared memory of a CTA; 0 when its addresses do not fit 16 bits.
+uint32_t layout(const TmCta& a, uint32_t n_mat, bool faces, TmGroup* out) {
+    uint32_t off = kTmHeadBytes, w0 = 0;
+    auto take = [&](uint32_t bytes) {
+        const uint32_t at = off;
+        off += (bytes + 127u) & ~127u;
+        return at;
+    };
+    for (uint32_t g = 0; g < a.n_groups; ++g) {
+        out[g].mat_off = take(8u * (n_mat + 1));
+        out[g].x_off = take(16u * (kTmStandIns + 32 * a.most[g]));
+    }
+    if (off + kTmSmemBase > 65536u) return 0;
+    for (uint32_t g = 0; g < a.n_groups; ++g) {
+        TmGroup& t = out[g];
+        if (faces) {
+            t.v_off = take(8u * (kTmStandIns + 32 * a.most[g]));
+            t.face_off = take(8u * a.faces[g]);
+        }
+        if (a.slots[g] > 65535u) return 0;
+        t.xy_off = take(8u * a.slots[g]);
+        t.z_off = take(4u * a.slots[g]);
+        t.info_off = take(32u * a.most[g]);
+        t.spare_off = take(128u * kTmSpareWords * (a.most[g] - a.warps[g]));
+        t.warp0 = w0;
+        t.warps = a.warps[g];
+        w0 += a.warps[g];
+    }
+    return off;
+}
+
+// The compiled kernels, and the time of a step of one CTA, us: the group that
+// takes longest for its bins (per bin: a fixed part; each slice of a warp and
+// each own column of it; each warp its barriers wait for) and the CTA's issue
+// (per slice, per own column).  Fitted to 990 arrangements of 40 populations of
+// 1-8 cells and of clouds, the reference step, within 5-7 % (one standard
+// deviation); what it picks took 0.8 % longer than the best on average, 11 %
+// at most.
+struct TmKernel {
+    uint32_t max_warps, max_mpt;
+    struct Cost {
+        double bin, slice, column, warp, cta_slice, cta_column;
+    } cost[2];  // without and with stress tracking
+};
+constexpr TmKernel kTmKernels[] = {
+    {kTmWideWarps, kTmMaxMpt, {{0.070, 0.540, 0.0539, 0.0168, 0.0265, 0.0021}, {0.088, 0.528, 0.0590, 0.0101, 0.0384, 0.0033}}},
+    {kTmMaxWarps, 1, {{0.0, 0.0, 0.0975, 0.0191, 0.0682, 0.0}, {0.0, 0.0, 0.1128, 0.0187, 0.0669, 0.0009}}},
+    // (not with tracking: stresses add to a thread's words, and two masses' do
+    // not fit a column share of 24 warps)
+    {kTmMaxWarps, kTmMaxMpt, {{0.372, 0.0, 0.0801, 0.0170, 0.0714, 0.0005}, {}}},
+};
+
+struct TmArrangement {
+    bool ok = false;
+    double us = 0.0;
+    std::vector<TmCta> ctas;
+    std::vector<uint8_t> group_of;  // per bin
+};
+
+// Arranges every CTA for one of the kernels.
+void arrange(const std::vector<TmBinSize>& bins, uint32_t ctas, uint32_t n_mat, uint32_t smem_cap, const TmKernel& kernel,
+             bool faces, bool track, TmArrangement& out) {
+    const uint32_t max_warps = kernel.max_warps, max_mpt = kernel.max_mpt;
+    const TmKernel::Cost& k = kernel.cost[track];
+    out = TmArrangement{};
+    out.ctas.resize(ctas);
+    out.group_of.assign(bins.size(), 0);
+    auto slices = [&](uint32_t b) { return (bins[b].n_mass + 31) / 32; };
+    // a face counts as two springs' instructions
+    auto columns = [&](uint32_t b) { return (bins[b].slots - kTmZeros + (faces ? 2u * bins[b].n_face : 0u)) / 32.0; };
+    auto cost = [&](uint32_t b) { return columns(b) + 2.0 * slices(b); };
+    std::vector<uint32_t> mine;
+    std::vector<uint8_t> group;
+    std::vector<double> work;
+    for (uint32_t c = 0; c < ctas; ++c) {
+        mine.clear();
+        double issue = 0.0;
+        for (uint32_t b = c; b < bins.size(); b += ctas) {
+            if (bins[b].n_mass == 0) continue;
+            mine.push_back(b);
+            issue += k.cta_slice * slices(b) + k.cta_column * columns(b);
+        }
+        std::stable_sort(mine.begin(), mine.end(), [&](uint32_t a, uint32_t b) { return cost(a) > cost(b); });
+        const uint32_t n = (uint32_t)mine.size();
+        group.resize(n);
+        double best = -1.0;
+        if (n == 0) best = 0.0;
+        for (uint32_t G = std::min(n, kTmMaxGroups); G >= 1; --G) {
+            TmCta a;
+            a.n_groups = G;
+            double load[kTmMaxGroups] = {};
+            for (uint32_t g = 0; g < G; ++g) a.warps[g] = a.most[g] = 1, a.slots[g] = kTmZeros, a.faces[g] = 0;
+            for (uint32_t i = 0; i < n; ++i) {
+                const uint32_t b = mine[i], g = (uint32_t)(std::min_element(load, load + G) - load);
+                group[i] = (uint8_t)g;
+                load[g] += cost(b);
+                a.most[g] = std::max(a.most[g], slices(b));
+                a.slots[g] = std::max(a.slots[g], bins[b].slots + (faces ? bins[b].n_face : 0u));
+                if (faces) a.faces[g] = std::max(a.faces[g], bins[b].n_face);
+            }
+            // warps: a slice each; where that is too many, one warp at a time
+            // off the group with the most for its work
+            uint32_t total = 0;
+            for (uint32_t g = 0; g < G; ++g) total += a.warps[g] = a.most[g];
+            const bool all = total <= max_warps;
+            while (total > max_warps) {
+                int from = -1;
+                for (uint32_t g = 0; g < G; ++g)
+                    if (a.warps[g] > 1 && (a.warps[g] - 1) * max_mpt >= a.most[g] &&
+                        (from < 0 || load[g] * a.warps[from] < load[from] * a.warps[g]))
+                        from = (int)g;
+                if (from < 0) break;
+                --a.warps[from];
+                --total;
+            }
+            TmGroup unused[kTmMaxGroups];
+            const uint32_t bytes = total <= max_warps ? layout(a, n_mat, faces, unused) : 0;
+            if (!bytes || bytes > smem_cap) continue;
+            double busy[kTmMaxGroups] = {};
+            for (uint32_t i = 0; i < n; ++i) {
+                const uint32_t b = mine[i], sl = slices(b), m = (sl + a.warps[group[i]] - 1) / a.warps[group[i]];
+                busy[group[i]] += k.bin + m * (k.slice + k.column * columns(b) / sl) + k.warp * sl;
+            }
+            const double us = issue + *std::max_element(busy, busy + G);
+            if (best >= 0.0 && us >= best) continue;
+            best = us;
+            out.ctas[c] = a;
+            for (uint32_t i = 0; i < n; ++i) out.group_of[mine[i]] = group[i];
+            if (all && G == n) break;  // every bin at once, a warp a slice
+        }
+        if (best < 0.0) return;
+        out.us = std::max(out.us, best);
+    }
+    out.ok = true;
+}
+
+TmArrangement arrange_best(const std::vector<TmBinSize>& bins, uint32_t ctas, uint32_t n_mat, uint32_t smem_cap,
+                           bool track, bool faces) {
+    TmArrangement best, a;
+    for (const TmKernel& kernel : kTmKernels) {
+        if (track && kernel.max_warps > kTmWideWarps && kernel.max_mpt > 1) continue;
+        arrange(bins, ctas, n_mat, smem_cap, kernel, faces, track, a);
+        if (a.ok && (!best.ok || a.us < best.us)) best = std::move(a);
+    }
+    return best;
+}
+
+}  // namespace
+
+double tm_estimate(const std::vector<TmBinSize>& bins, uint32_t ctas, uint32_t n_mat, uint32_t smem_cap, bool track,
+                   bool faces) {
+    const TmArrangement a = arrange_best(bins, ctas, n_mat, smem_cap, track, faces);
+    return a.ok ? a.us : 0.0;
+}
+
 void tm_plan(const std::vector<BinDesc>& bins, const std::vector<uint32_t>& slots, uint32_t ctas, uint32_t n_mat,
-             uint32_t smem_cap, uint32_t max_mpt, bool faces, TmPlan& out) {
+             uint32_t smem_cap, bool track, bool faces, TmPlan& out) {
     out = TmPlan{};
     out.faces = faces;
-    const uint32_t nb = (uint32_t)bins.size();
-    if (nb == 0 || ctas == 0) return;
-    ctas = std::min(ctas, nb);
-    auto slices = [&](uint32_t b) { return (bins[b].n_mass + 31) / 32; };
-    auto n_face = [&](uint32_t b) { return faces ? bins[b].n_face : 0u; };
-    // a slice's work: its own springs (slots), its masses, the bin's faces
-    // (about two springs' instructions each)
-    auto cost = [&](uint32_t b) { return (double)slots[b] + 64.0 * slices(b) + 2.0 * n_face(b); };
+    if (bins.empty() || ctas == 0) return;
+    ctas = std::min(ctas, (uint32_t)bins.size());
+    std::vector<TmBinSize> sizes;
+    for (size_t b = 0; b < bins.size(); ++b) sizes.push_back({bins[b].n_mass, slots[b], faces ? bins[b].n_face : 0u});
+    const TmArrangement a = arrange_best(sizes, ctas, n_mat, smem_cap, track, faces);
+    if (!a.ok) return;
+    out.groups.assign((size_t)ctas * kTmMaxGroups, TmGroup{});
     for (uint32_t c = 0; c < ctas; ++c) {
-        std::vector<uint32_t> mine;
-        for (uint32_t b = c; b < nb; b += ctas) mine.push_back(b);
-        bool placed = false;
-        for (uint32_t G = std::min<uint32_t>((uint32_t)mine.size(), kTmMaxGroups); G >= 1 && !placed; --G) {
-            std::vector<std::vector<uint32_t>> lists(G);
-            std::vector<double> load(G, 0.0);
-            std::vector<uint32_t> order(mine);
-            std::stable_sort(order.begin(), order.end(), [&](uint32_t a, uint32_t b) { return cost(a) > cost(b); });
-            for (uint32_t b : order) {
-                const uint32_t g = (uint32_t)(std::min_element(load.begin(), load.end()) - load.begin());
-                lists[g].push_back(b);
-                load[g] += cost(b);
+        const TmCta& t = a.ctas[c];
+        TmGroup* g = &out.groups[(size_t)c * kTmMaxGroups];
+        out.smem = std::max(out.smem, layout(t, n_mat, faces, g));
+        for (uint32_t i = 0; i < t.n_groups; ++i) {
+            g[i].first = (uint32_t)out.bins.size();
+            for (uint32_t b = c; b < bins.size(); b += ctas) {
+                const BinDesc& d = bins[b];
+                if (d.n_mass && a.group_of[b] == i)
+                    out.bins.push_back({b, d.mass_begin, d.n_mass, d.slice_begin, d.face_begin, sizes[b].n_face, d.face_inc_begin});
             }
-            // warps: a slice each, up to kTmMaxWarps in all; where that is not enough,
-            // one warp at a time off the group with the most for its work
-            std::vector<uint32_t> warps(G, 1), most(G, 1);
-            uint32_t total = 0;
-            for (uint32_t g = 0; g < G; ++g) {
-                for (uint32_t b : lists[g]) most[g] = std::max(most[g], slices(b));
-                warps[g] = most[g];
-                total += warps[g];
-            }
-            bool fits = true;
-            while (total > kTmMaxWarps && fits) {
-                int best = -1;
-                for (uint32_t g = 0; g < G; ++g)
-                    if (warps[g] > 1 && (warps[g] - 1) * max_mpt >= most[g] &&
-                        (best < 0 || load[g] * warps[best] < load[best] * warps[g]))
-                        best = (int)g;
-                fits = best >= 0;
-                if (fits) {
-                    --warps[best];
-                    --total;
-                }
-            }
-            if (!fits) continue;
-            uint32_t off = 0, w0 = 0;
-            std::vector<TmGroup> groups(kTmMaxGroups, TmGroup{});
-            auto take = [&](uint32_t bytes) {
-                const uint32_t at = off;
-                off += (bytes + 127u) & ~127u;
-                return at;
-            };
-            take(kTmHeadBytes);
-            for (uint32_t g = 0; g < G; ++g) {
-                groups[g].mat_off = take(8u * (n_mat + 1));
-                groups[g].x_off = take(16u * (kTmStandIns + 32 * most[g]));
-            }
-            if (off + kTmSmemBase > 65536u) continue;  // 16-bit addresses
-            for (uint32_t g = 0; g < G; ++g) {
-                uint32_t gs = 0, nf = 0;
-                for (uint32_t b : lists[g]) {
-                    gs = std::max(gs, slots[b] + n_face(b));
-                    nf = std::max(nf, n_face(b));
-                }
-                if (faces) {
-                    groups[g].v_off = take(8u * (kTmStandIns + 32 * most[g]));
-                    groups[g].face_off = take(8u * nf);
-                }
-                if (gs > 65535u) fits = false;  // 16-bit slots
-                groups[g].xy_off = take(8u * gs);
-                groups[g].z_off = take(4u * gs);
-                groups[g].info_off = take(32u * most[g]);
-                groups[g].spare_off = take(128u * kTmSpareWords * (most[g] - warps[g]));
-                groups[g].warp0 = w0;
-                groups[g].warps = warps[g];
-                w0 += warps[g];
-            }
-            if (!fits || off > smem_cap) continue;
-            for (uint32_t g = 0; g < G; ++g) {
-                groups[g].first = (uint32_t)out.bins.size();
-                groups[g].count = (uint32_t)lists[g].size();
-                for (uint32_t b : lists[g]) {
-                    const BinDesc& d = bins[b];
-                    out.bins.push_back({b, d.mass_begin, d.n_mass, d.slice_begin, d.face_begin, n_face(b), d.face_inc_begin});
-                }
-                out.mpt = std::max(out.mpt, (most[g] + warps[g] - 1) / warps[g]);
-            }
-            out.groups.insert(out.groups.end(), groups.begin(), groups.end());
-            out.threads = std::max(out.threads, 32 * w0);
-            out.smem = std::max(out.smem, off);
-            placed = true;
+            g[i].count = (uint32_t)out.bins.size() - g[i].first;
+            out.mpt = std::max(out.mpt, (t.most[i] + t.warps[i] - 1) / t.warps[i]);
+            out.threads = std::max(out.threads, 32 * (g[i].warp0 + g[i].warps));
         }
-        if (!placed) return;
     }
+    out.threads = std::max(out.threads, 32u);
     out.ctas = ctas;
     out.ok = true;
 }

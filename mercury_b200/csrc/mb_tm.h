@@ -28,7 +28,7 @@ struct alignas(16) TmBinRef {
 };
 
 constexpr uint32_t kTmMaxWarps = 24;      // warps per CTA: 80 registers a thread
-constexpr uint32_t kTmWideWarps = 8;      // up to which the variant with more registers runs
+constexpr uint32_t kTmWideWarps = 16;     // up to which the variant with more registers runs
 constexpr uint32_t kTmMaxGroups = 8;      // groups (named barriers) per CTA
 constexpr uint32_t kTmMaxMpt = 2;         // masses per thread
 constexpr uint32_t kTmZeros = 32;         // zero slots before a bin's corrections, one per bank
@@ -37,9 +37,6 @@ constexpr uint32_t kTmSmemBase = 4096;    // bound on the address where dynamic 
 constexpr uint32_t kTmHeadBytes = 512;    // start of the dynamic shared memory: what the groups need of their bins
 constexpr uint32_t kTmMaxSlices = 128;    // slices of 32 masses per bin
 constexpr uint32_t kTmSpareWords = 8;     // gather words of a slice kept in shared memory when the columns are full
-
-// Masses per thread: stresses add to a thread's words, one mass then.
-inline uint32_t tm_max_mpt(bool track) { return track ? 1u : kTmMaxMpt; }
 
 // Populations the kernel steps: resident bins of a 1,024-thread shape with at
 // most one mass per thread, no mass with more springs than a lattice has.
@@ -59,11 +56,17 @@ struct TmPlan {
 };
 
 // Plans the launch over `bins` (slots[b]: correction slots of bin b, from
-// launch_tm_rows): CTA c of `ctas` steps bins c, c + ctas, ...  max_mpt:
-// masses per thread.  faces: with the face drag.  Not ok when a CTA's bins fit
-// no arrangement.
+// launch_tm_rows): CTA c of `ctas` steps bins c, c + ctas, ...  Not ok when a
+// CTA's bins fit no arrangement.
 void tm_plan(const std::vector<BinDesc>& bins, const std::vector<uint32_t>& slots, uint32_t ctas, uint32_t n_mat,
-             uint32_t smem_cap, uint32_t max_mpt, bool faces, TmPlan& out);
+             uint32_t smem_cap, bool track, bool faces, TmPlan& out);
+
+// Estimated time of a step of such a launch, us (0: no arrangement).
+struct TmBinSize {
+    uint32_t n_mass, slots, n_face;
+};
+double tm_estimate(const std::vector<TmBinSize>& bins, uint32_t ctas, uint32_t n_mat, uint32_t smem_cap, bool track,
+                   bool faces);
 
 // Correction slots of a bin from its SELL rows on the host, as the row kernel
 // counts them (launch planning without a GPU).

@@ -310,12 +310,13 @@ class Simulator:
         _lib.check(_lib.LIB.mb_get_launch_config(self._ctx, ctypes.byref(c)), self._ctx)
         return {f: getattr(c, f) for f, _ in c._fields_}
 
-    def step_variant(self) -> dict:
-        """The step kernel the next launches use (mb_get_step_variant):
-        register_rows (1 when each mass's row is held per thread) and the dynamic
-        shared memory per CTA."""
+    def step_variant(self, track_stresses: bool = False) -> dict:
+        """The step kernel the next launches use, without or with stress tracking
+        (mb_get_step_variant, mb_get_tracked_step_variant): register_rows (1 when
+        each mass's row is held per thread) and the dynamic shared memory per CTA."""
         rr, smem = ctypes.c_uint32(), ctypes.c_uint32()
-        _lib.check(_lib.LIB.mb_get_step_variant(self._ctx, ctypes.byref(rr), ctypes.byref(smem)), self._ctx)
+        get = _lib.LIB.mb_get_tracked_step_variant if track_stresses else _lib.LIB.mb_get_step_variant
+        _lib.check(get(self._ctx, ctypes.byref(rr), ctypes.byref(smem)), self._ctx)
         return {"register_rows": rr.value, "smem_bytes": smem.value}
 
     def packed_springs(self) -> np.ndarray:

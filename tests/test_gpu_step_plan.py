@@ -1,17 +1,20 @@
-"""Populations whose launch plan takes all the shared memory of a CTA, against
-the CPU oracle bit for bit, on the kernel that the host planner names."""
+"""Launch plans that take all the shared memory of a CTA, and the first that
+does not fit, against the CPU oracle bit for bit, on the kernel that the host
+planner names; whole populations of large bins."""
 import numpy as np
 import pytest
 
 import mercury_b200 as mb
 from oracle import core
+from test_gpu_tm import random_robot
 from test_step_plan import SMEM, population
 
 pytestmark = pytest.mark.gpu
 
 
-def run(batch, steps, track):
+def run(batch, steps, track, **cfg):
     sim = mb.Simulator(0)
+    sim.set_launch_config(**cfg)
     sim.setTimeStep(1e-3)
     sim.set_batch(batch)
     sim.run_steps(steps, track)
@@ -24,9 +27,42 @@ def run(batch, steps, track):
 
 
 @pytest.mark.parametrize("count,lo", [(480, 4), (512, 5), (400, 5), (590, 3)])
-def test_full_ctas_bit_exact(count, lo):
+def test_large_populations_bit_exact(count, lo):
     b = population(count, lo, 8, 1)
-    sim = run(b, 20, False)
-    v = sim.step_variant()
-    assert v == mb.plan_step_variant(b)
-    assert v["register_rows"] == 1 and SMEM - 1024 <= v["smem_bytes"] <= SMEM
+    sim = run(b, 20, False, bins=444)
+    assert sim.step_variant() == mb.plan_step_variant(b, bins=444)
+    assert sim.step_variant()["register_rows"] == 1
+
+
+@pytest.mark.parametrize("track", [False, True])
+@pytest.mark.parametrize("n", [1000, 1024])
+def test_full_cta_bit_exact(n, track):
+    """One robot with as many springs as the plan has room for, and with one
+    more: in every slice of 32 masses one mass has its springs to lower masses,
+    so that a spring more is a column of 32 slots more."""
+    rng = np.random.default_rng(n)
+    whole = random_robot(n, rng, 0)
+    deg, pairs = np.zeros(n, int), []
+    for _ in range(22):
+        for m in range(63, n, 32):
+            used = [b for a, b in pairs if a == m]
+            free = np.setdiff1d(np.arange(m), used)
+            low = free[np.argmin(deg[free])]
+            pairs.append((m, low))
+            deg[[m, low]] += 1
+    pairs = np.array(pairs, np.uint16)
+    lbar = rng.uniform(0.2, 1.0, len(pairs)).astype(np.float32)
+
+    def robot(k):
+        return mb.pack([mb.Element(whole.pos, whole.mass_material, pairs[:k], lbar[:k], np.full(k, 5, np.uint8),
+                                   vel=whole.vel)])
+
+    few, many = n // 4, len(pairs)  # the former fits, the latter does not
+    assert mb.plan_step_variant(robot(few), track)["register_rows"] > mb.plan_step_variant(robot(many), track)["register_rows"]
+    while many - few > 1:
+        k = (few + many) // 2
+        few, many = (k, many) if mb.plan_step_variant(robot(k), track)["register_rows"] else (few, k)
+    v = run(robot(few), 20, track).step_variant(track)
+    assert v == mb.plan_step_variant(robot(few), track) and v["register_rows"] == 1
+    assert SMEM - 1024 < v["smem_bytes"] <= SMEM
+    assert run(robot(many), 20, track).step_variant(track)["register_rows"] == 0
