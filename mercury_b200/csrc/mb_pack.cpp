@@ -137,6 +137,7 @@ struct RobotPack {
     uint32_t n_face = 0;     // faces with three distinct corners
     uint32_t face_smem = 0;  // shared memory of the face drag, bytes (upper bound)
     uint32_t max_degree = 0;  // most non-air springs at one mass
+    uint32_t own_slots = 0;   // correction slots of the tensor-memory kernel (estimate)
     uint64_t mats[4] = {0, 0, 0, 0};  // composite ids of its non-air springs (bit set)
     std::string error;
     mb_status status = MB_OK;
@@ -177,7 +178,7 @@ void preprocess(const mb_batch_desc* b, uint32_t r, RobotPack& p) {
             p.status = MB_ERR_ARGUMENT;
             return;
         }
-    std::vector<uint32_t> deg((size_t)cm, 0);
+    std::vector<uint32_t> deg((size_t)cm, 0), own((size_t)cm, 0);  // springs of a mass; those to lower masses
     auto& sp = p.springs;
     sp.reserve((size_t)(s1 - s0));
     for (int64_t s = s0; s < s1; ++s) {
@@ -205,6 +206,7 @@ void preprocess(const mb_batch_desc* b, uint32_t r, RobotPack& p) {
         sp.push_back((uint32_t)(s - s0));
         deg[a]++;
         deg[c]++;
+        own[std::max(a, c)]++;
     }
     // order (b - a, a), ties by spring index: sp is in index order, so two
     // stable counting passes -- by a, then by b - a -- give exactly that
@@ -274,9 +276,10 @@ void preprocess(const mb_batch_desc* b, uint32_t r, RobotPack& p) {
     p.cost = (uint64_t)sp.size() * 4 + (uint64_t)cm + 2ull * p.n_face;
     uint64_t est = 0;  // incidence entries with rows padded to the slice maximum
     for (int64_t i = 0; i < cm; i += 32) {
-        uint32_t w = 0;
-        for (int64_t k = i; k < std::min<int64_t>(i + 32, cm); ++k) w = std::max(w, deg[k]);
+        uint32_t w = 0, o = 0;
+        for (int64_t k = i; k < std::min<int64_t>(i + 32, cm); ++k) w = std::max(w, deg[k]), o = std::max(o, own[k]);
         est += 32ull * w;
+        p.own_slots += 32 * o;
         p.max_degree = std::max(p.max_degree, w);
     }
     p.inc_estimate = est + 64;  // slack for slices straddling robots
@@ -318,17 +321,13 @@ bool plan_bins(const std::vector<RobotPack>& packs, uint32_t nb, const KernelSha
 }
 
 // Two-level LPT for launches of more than one wave.  A launch of `groups`
-// CTAs runs bins g, g + groups, g + 2 groups ... one after another on CTA g,
-// so what has to be even is the load of a group, not of a bin: robots are
-// first spread over the groups by LPT (a group holds nb / groups bins'
-// capacity), then each group's robots are spread over its own bins by LPT
-// under the per-bin limits.  Returns false when a group cannot be split,
-// and the caller falls back to plan_bins.
-bool plan_bins_grouped(const std::vector<RobotPack>& packs, uint32_t nb, uint32_t groups,
-                       const KernelShape& sh, uint32_t smem_cap,
-                       std::vector<std::vector<uint32_t>>& plan) {
-    if (groups == 0 || nb <= groups || nb % groups) return false;
-    const uint32_t per = nb / groups;
+// CTAs runs bins g, g + groups, g + 2 groups ... on CTA g, so what has to be
+// even is the load of a group, not of a bin: robots are first spread over the
+// groups by LPT (a group holds `per` bins' capacity), then each group's robots
+// are spread over its own bins by LPT under the per-bin limits.  Both return
+// false when that is not possible.
+bool group_robots(const std::vector<RobotPack>& packs, uint32_t groups, uint32_t per, const KernelShape& sh,
+                  std::vector<std::vector<uint32_t>>& members) {
     const uint32_t n = (uint32_t)packs.size();
     std::vector<uint32_t> order(n);
     for (uint32_t i = 0; i < n; ++i) order[i] = i;
@@ -337,7 +336,7 @@ bool plan_bins_grouped(const std::vector<RobotPack>& packs, uint32_t nb, uint32_
     const uint64_t cap_s = std::min<uint64_t>((uint64_t)sh.threads * sh.spt, kMaxBinSprings);
     const uint64_t cap_m = std::min<uint64_t>((uint64_t)sh.threads * sh.mpt, 4096);
     std::vector<uint64_t> gload(groups, 0), gm(groups, 0), gs(groups, 0);
-    std::vector<std::vector<uint32_t>> members(groups);
+    members.assign(groups, {});
     for (uint32_t r : order) {
         const auto& p = packs[r];
         int best = -1;
@@ -351,9 +350,18 @@ bool plan_bins_grouped(const std::vector<RobotPack>& packs, uint32_t nb, uint32_
         gs[best] += p.springs.size();
         members[best].push_back(r);  // descending cost within the group
     }
-    plan.assign(nb, {});
+    return true;
+}
+
+bool fill_groups(const std::vector<RobotPack>& packs, const std::vector<std::vector<uint32_t>>& members, uint32_t per,
+                 const KernelShape& sh, uint32_t smem_cap, std::vector<std::vector<uint32_t>>& plan) {
+    const uint32_t groups = (uint32_t)members.size();
+    const uint64_t cap_s = std::min<uint64_t>((uint64_t)sh.threads * sh.spt, kMaxBinSprings);
+    const uint64_t cap_m = std::min<uint64_t>((uint64_t)sh.threads * sh.mpt, 4096);
+    plan.assign((size_t)groups * per, {});
+    std::vector<uint64_t> load(per), bm(per), bs(per), bi(per), bx(per);
     for (uint32_t g = 0; g < groups; ++g) {
-        std::vector<uint64_t> load(per, 0), bm(per, 0), bs(per, 0), bi(per, 0), bx(per, 0);
+        for (auto* v : {&load, &bm, &bs, &bi, &bx}) std::fill(v->begin(), v->end(), 0);
         for (uint32_t r : members[g]) {
             const auto& p = packs[r];
             int best = -1;
@@ -375,6 +383,60 @@ bool plan_bins_grouped(const std::vector<RobotPack>& packs, uint32_t nb, uint32_
     }
     for (auto& v : plan) std::sort(v.begin(), v.end());
     return true;
+}
+
+bool plan_bins_grouped(const std::vector<RobotPack>& packs, uint32_t nb, uint32_t groups,
+                       const KernelShape& sh, uint32_t smem_cap,
+                       std::vector<std::vector<uint32_t>>& plan) {
+    if (groups == 0 || nb <= groups || nb % groups) return false;
+    std::vector<std::vector<uint32_t>> members;
+    return group_robots(packs, groups, nb / groups, sh, members) &&
+           fill_groups(packs, members, nb / groups, sh, smem_cap, plan);
+}
+
+// Bins of the tensor-memory kernel when there are at least as many robots as
+// CTAs: the number of bins a CTA whose estimated step is shortest.  No one rule
+// of sizes does: a robot a bin suits robots of many slices (1,638 of 6x6x6 cells
+// 17.3 us a step at 12 bins a CTA, 21.0 at 8, where some bins get a second
+// robot), but steps 4,096 robots of a cell one after another on a few
+// threads (4.9 us at 27 bins a CTA, 1.2 at 8), and 512 robots of 3-8 cells take
+// 5.2 us at 3 bins, 5.6 at 2.  Returns the bins a CTA, or 0 when none fits.
+uint32_t plan_tm_bins(const std::vector<RobotPack>& packs, uint32_t ctas, const KernelShape& sh, uint32_t smem_cap,
+                      uint32_t n_mat, unsigned threads, std::vector<std::vector<uint32_t>>& plan) {
+    const uint32_t most = ((uint32_t)packs.size() + ctas - 1) / ctas;
+    std::vector<uint32_t> per;
+    for (uint32_t k : {1u, 2u, 3u, 4u, 6u, 8u, 12u, 16u})
+        if (k < most) per.push_back(k);
+    if (most <= 16) per.push_back(most);  // a robot a bin
+    std::vector<std::vector<uint32_t>> members;
+    if (!group_robots(packs, ctas, per.back(), sh, members)) return 0;
+    const uint32_t n = (uint32_t)per.size();
+    std::vector<std::vector<std::vector<uint32_t>>> plans(n);
+    std::vector<double> us(n, 0.0);
+    parallel_for(n, threads, [&](uint32_t i) {
+        if (!fill_groups(packs, members, per[i], sh, smem_cap, plans[i])) return;
+        std::vector<TmBinSize> sizes;
+        for (const auto& robots : plans[i]) {
+            TmBinSize b{0, kTmZeros, 0};
+            double slots = 0.0;  // of a mass's share of its slice
+            for (uint32_t r : robots) {
+                const RobotPack& p = packs[r];
+                b.n_mass += p.n_mass;
+                slots += p.own_slots * (p.n_mass / (32.0 * ((p.n_mass + 31) / 32)));
+            }
+            if (b.n_mass) b.slots += (uint32_t)(slots * (32 * ((b.n_mass + 31) / 32)) / b.n_mass);
+            sizes.push_back(b);
+        }
+        us[i] = tm_estimate(sizes, ctas, n_mat, smem_cap, false, false);
+        // (between equals, the one that tracks stresses faster)
+        if (us[i] > 0.0) us[i] += 0.02 * tm_estimate(sizes, ctas, n_mat, smem_cap, true, false);
+    });
+    uint32_t best = n;
+    for (uint32_t i = 0; i < n; ++i)
+        if (us[i] > 0.0 && (best == n || us[i] < us[best])) best = i;
+    if (best == n) return 0;
+    plan.swap(plans[best]);
+    return per[best];
 }
 
 struct BinLocal {
@@ -1361,22 +1423,26 @@ mb_status pack_population(const mb_batch_desc* b, const PackOptions& o, Packed& 
             nb = (uint32_t)std::max<uint64_t>(need, R < sms ? R : 1);
             if (R >= sms) {
                 nb = std::max<uint32_t>(nb, wave);
-                // whole waves; for the tensor-memory kernel, which steps a
-                // CTA's bins side by side, about a robot a bin (512 uneven
-                // robots: 5.46 us a step in 444 bins, 5.73 in 296)
-                if (one_mass) nb = std::max(nb, R / wave * wave);
-                nb = (nb + wave - 1) / wave * wave;
+                nb = (nb + wave - 1) / wave * wave;  // whole waves
             }
             nb = std::min<uint32_t>(nb, R);
         }
-        uint32_t grid = 0;
+        uint32_t grid = 0, nb_rule = nb;
         for (uint32_t tries = 0; tries < 16; ++tries) {
             // Several waves: one CTA per group of bins, groups balanced
             // (plan_bins_grouped); otherwise one CTA per bin.
             grid = 0;
             bool planned = false;
             const KernelShape psh{sh.threads, sh.spt, one_mass ? 1u : sh.mpt};
-            if (R >= sms && nb >= 2 * wave && nb % wave == 0 &&
+            if (one_mass && !fixed && R >= sms && tries == 0) {
+                const uint32_t per = plan_tm_bins(packs, wave, psh, o.smem_cap, (uint32_t)out.mat_ids.size(), threads, plan);
+                if (per) {
+                    planned = true;
+                    nb = per * wave;
+                    grid = per > 1 ? wave : 0;
+                }
+            }
+            if (!planned && R >= sms && nb >= 2 * wave && nb % wave == 0 &&
                 plan_bins_grouped(packs, nb, wave, psh, o.smem_cap, plan)) {
                 planned = true;
                 grid = wave;
@@ -1389,8 +1455,8 @@ mb_status pack_population(const mb_batch_desc* b, const PackOptions& o, Packed& 
                     break;
                 }
             }
-            if (fixed || nb >= R) break;
-            nb = std::min<uint32_t>(R, nb + wave);
+            if (fixed || nb_rule >= R) break;
+            nb = nb_rule = std::min<uint32_t>(R, nb_rule + wave);
         }
         if (ok) {
             out.shape = sh;

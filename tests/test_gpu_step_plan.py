@@ -66,3 +66,11 @@ def test_full_cta_bit_exact(n, track):
     assert v == mb.plan_step_variant(robot(few), track) and v["register_rows"] == 1
     assert SMEM - 1024 < v["smem_bytes"] <= SMEM
     assert run(robot(many), 20, track).step_variant(track)["register_rows"] == 0
+
+
+@pytest.mark.parametrize("track", [False, True])
+@pytest.mark.parametrize("count,lo,hi", [(149, 1, 1), (300, 1, 4), (1000, 1, 2), (2000, 1, 1)])
+def test_small_robots_bit_exact(count, lo, hi, track):
+    """Bins of several small robots, and CTAs that get fewer bins than others."""
+    b = population(count, lo, hi, 2)
+    assert run(b, 20, track).step_variant(track)["register_rows"] == 1

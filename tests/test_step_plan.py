@@ -36,3 +36,14 @@ def test_the_resident_kernel_has_no_static_shared_memory():
     src = open(os.path.join(ROOT, "mercury_b200", "csrc", "mb_tm.cu")).read()
     kernel = src[src.index("tm_step_kernel("):src.index("tm_rows_kernel(")]
     assert not re.search(r"^(?!.*extern).*__shared__", kernel, re.M)
+
+
+@pytest.mark.parametrize("count,side,least,most", [(4096, 1, 1, 8), (16384, 1, 1, 16), (4096, 2, 1, 12), (1638, 6, 12, 12),
+                                                   (512, 6, 3, 4), (149, 8, 2, 2)])
+def test_small_robots_share_bins(count, side, least, most):
+    """Bins a CTA: robots of a slice or less share bins, so that a CTA steps its
+    bins side by side; large ones have a bin each."""
+    one = robots.voxel_robot(np.full((side,) * 3, robots.BONE, np.uint8))
+    st = mb.plan(mb.pack([one] * count))
+    assert st["ctas"] == 148 and st["bins"] % 148 == 0 and least <= st["bins"] // 148 <= most
+    assert mb.plan_step_variant(mb.pack([one] * count))["register_rows"] == 1
