@@ -123,20 +123,24 @@ struct mb_context {
     mb::KernelShape shape{512, 8, 2};
     uint32_t n_bins = 0;
     uint32_t max_bin_mass = 0;  // most (own) masses in one bin
+    uint32_t max_bin_springs = 0;  // most springs in one bin when packed (of a voxel population: in the template)
     // resident bins on the tensor-memory step kernel (mb_tm.h): the rows it
-    // reads, built on the device before the first step after the packed rows
-    // changed, and the launch plan without and with stress tracking
+    // reads, built on the device behind the packed rows, and the launch plan
+    // without and with stress tracking, made before the first step that needs it
     struct TmLaunch {
         mb::TmPlan plan;
         bool planned = false;
         size_t groups = 0, bins = 0;  // bytes into `arrays`
         mb::DevBuf<uint8_t> arrays;
+        std::vector<uint8_t> host;  // what was copied to `arrays`
     } tm[2];
     bool tm_stale = true;
     uint32_t n_slices = 0;
     mb::TmRows tm_rows{};          // into tm_arena
     mb::DevBuf<uint8_t> tm_arena;
-    std::vector<uint32_t> tm_slots;  // per bin: correction slots
+    std::vector<uint32_t> tm_slots;  // per bin: correction slots the plans leave room for
+    std::vector<uint32_t> h_status;  // read back: devo_status
+    bool springs_placed = true;      // resident springs are in the order of the general kernel's loads
     uint32_t max_degree = 0;    // most springs at one mass when uploaded
     uint32_t grid = 0;  // CTAs per step launch (0 = one per bin)
     uint32_t chunk = 1000;
@@ -215,7 +219,8 @@ struct mb_context {
     mb::DevBuf<uint16_t> d_pairs;
     mb::DevBuf<uint8_t> d_spring_mat, slot_of;
     mb::DevBuf<float> d_lbar;
-    mb::DevBuf<uint32_t> pslot, robot_mass_base, free_count, free_taken, free_slots, devo_status, new_begin;
+    mb::DevBuf<uint32_t> pslot, robot_mass_base, free_count, free_taken, free_slots, new_begin;
+    mb::DevBuf<uint32_t> devo_status;  // two words of the row kernel, then the correction slots of every bin
     mb::DevBuf<unsigned long long> rows_scratch;
     // development of split populations on the device (the partition of the
     // last packing; regions with spare capacity per bin, set up by the first
@@ -235,7 +240,6 @@ struct mb_context {
         int sx = 0, sy = 0, sz = 0;
         uint32_t h_bits = 0, mass_bits = 0, mode = 0;
         uint32_t n_points = 0, n_springs = 0;  // per robot
-        uint32_t max_bin_springs = 0;          // the template's largest bin (active springs bound)
         mb::DevBuf<float> pos;
         mb::DevBuf<uint16_t> src;
         mb::DevBuf<uint8_t> dir, cells;
@@ -293,7 +297,12 @@ namespace mb_detail {
 
 bool tm_eligible(const mb_context* c);
 bool use_tm(const mb_context* c, bool track);
+cudaError_t reset_rows(mb_context* c);
+cudaError_t build_rows(mb_context* c, bool place, uint32_t max_bin_springs);
+cudaError_t tm_queue_rows(mb_context* c);
+cudaError_t read_status(mb_context* c, uint32_t* status, bool new_bins);
 cudaError_t tm_update(mb_context* c, bool track);
+cudaError_t place_springs(mb_context* c);
 
 // Whether the step applies the face drag (water mode, rho != 0): split
 // robots are then packed with their faces (velocities exchanged with the
@@ -334,6 +343,39 @@ mb_status pack(mb_context* ctx, const mb_batch_desc* b, bool fallback_auto, mb::
     return MB_OK;
 }
 
+// Buffers and status words of the row kernel, for rows without inert springs.
+cudaError_t reset_rows(mb_context* c) {
+    const uint32_t nb = c->n_bins;
+    cudaStream_t st = c->stream;
+    cudaError_t e = c->rows_scratch.alloc(2 * std::max<size_t>(c->n_packed, 1));
+    for (auto* b : {&c->free_count, &c->free_taken}) {
+        if (e == cudaSuccess) e = b->alloc(nb);
+        if (e == cudaSuccess) e = cudaMemsetAsync(b->p, 0, nb * sizeof(uint32_t), st);
+    }
+    if (e == cudaSuccess) e = c->devo_status.alloc(2 + nb);
+    if (e == cudaSuccess) e = cudaMemsetAsync(c->devo_status.p, 0, 2 * sizeof(uint32_t), st);
+    return e;
+}
+
+// Queues the rows of resident or streamed bins from their springs (place: put
+// into the order of the general kernel's endpoint loads first).  No packed slot
+// is inert: spring_gidx < n_spring everywhere.
+cudaError_t build_rows(mb_context* c, bool place, uint32_t max_bin_springs) {
+    const uint32_t nb = c->n_bins;
+    cudaStream_t st = c->stream;
+    cudaError_t e = cudaSuccess;
+    if (place)
+        e = mb::launch_bank_place(c->bins.p, nb, max_bin_springs, c->spring_pair.p, c->spring_gidx.p, c->spring_lbar.p,
+                                  c->rows_scratch.p, st);
+    const mb::RebuildParams rp{c->bins.p,        nb,                      c->spring_pair.p,
+                               c->spring_gidx.p, (uint32_t)c->n_spring,   c->slice_off.p,
+                               c->slice_width.p, c->inc.p,                c->inc32.p,
+                               c->streamed ? 1u : 0u, c->rows_scratch.p,  c->free_count.p,
+                               c->free_taken.p,  c->devo_status.p};
+    if (e == cudaSuccess) e = mb::launch_rebuild(rp, st);
+    return e;
+}
+
 // Uploads the packed arrays of `out` and the per-launch buffers sized by
 // them; positions, velocities and stresses are not touched.  Rows the host
 // did not build are built on the device (the development re-pack kernel);
@@ -346,7 +388,11 @@ mb_status upload_packed(mb_context* ctx, const mb::Packed& out, bool* rows_faile
     ctx->grid = out.grid;
     ctx->max_bin_mass = 0;
     ctx->max_degree = out.max_degree;
-    for (const mb::BinDesc& d : out.bins) ctx->max_bin_mass = std::max(ctx->max_bin_mass, d.n_mass);
+    ctx->max_bin_springs = 0;
+    for (const mb::BinDesc& d : out.bins) {
+        ctx->max_bin_mass = std::max(ctx->max_bin_mass, d.n_mass);
+        ctx->max_bin_springs = std::max(ctx->max_bin_springs, d.n_spring);
+    }
     ctx->smem_bytes = out.max_smem;
     ctx->streamed = out.streamed;
     ctx->cluster = out.cluster;
@@ -454,43 +500,35 @@ mb_status upload_packed(mb_context* ctx, const mb::Packed& out, bool* rows_faile
     ctx->h_mat_ids = out.mat_ids;
     ctx->n_packed = (uint32_t)out.pair.size();
     ctx->devo_ready = false;
+    ctx->springs_placed = true;
+    ctx->tm_stale = true;
+    ctx->n_slices = (uint32_t)out.slice_off.size();
     MB_CUDA(ctx, ctx->bin_flags.alloc(nb));
     MB_CUDA(ctx, cudaMemsetAsync(ctx->bin_flags.p, 0, nb * sizeof(uint32_t), st));
     if (out.rows_on_device) {
         MB_CUDA(ctx, ctx->inc.alloc(std::max<uint64_t>(out.row_total, 1)));
-        MB_CUDA(ctx, ctx->rows_scratch.alloc(2 * std::max<size_t>(out.pair.size(), 1)));
-        MB_CUDA(ctx, ctx->free_count.alloc(nb));
-        MB_CUDA(ctx, ctx->free_taken.alloc(nb));
-        MB_CUDA(ctx, ctx->devo_status.alloc(2));
-        MB_CUDA(ctx, cudaMemsetAsync(ctx->free_count.p, 0, nb * sizeof(uint32_t), st));
-        MB_CUDA(ctx, cudaMemsetAsync(ctx->free_taken.p, 0, nb * sizeof(uint32_t), st));
-        MB_CUDA(ctx, cudaMemsetAsync(ctx->devo_status.p, 0, 2 * sizeof(uint32_t), st));
-        // the springs of every bin placed for the endpoint loads (the host
-        // packer left them in upload order), then the rows built
-        uint32_t max_springs = 0;
-        for (const mb::BinDesc& d : out.bins) max_springs = std::max(max_springs, d.n_spring);
-        MB_CUDA(ctx, mb::launch_bank_place(ctx->bins.p, nb, max_springs, ctx->spring_pair.p, ctx->spring_gidx.p,
-                                           ctx->spring_lbar.p, ctx->rows_scratch.p, st));
-        // no packed slot is inert here: spring_gidx < n_spring everywhere
-        const mb::RebuildParams rp{ctx->bins.p,        nb,                   ctx->spring_pair.p,
-                                   ctx->spring_gidx.p, (uint32_t)ctx->n_spring, ctx->slice_off.p,
-                                   ctx->slice_width.p, ctx->inc.p,           ctx->inc32.p,
-                                   0u,                 ctx->rows_scratch.p,  ctx->free_count.p,
-                                   ctx->free_taken.p,  ctx->devo_status.p};
-        MB_CUDA(ctx, mb::launch_rebuild(rp, st));
+        // the springs of every bin placed for the general kernel's endpoint loads
+        // (the host packer left them in upload order), unless another one
+        // steps them; then the rows
+        ctx->springs_placed = !tm_eligible(ctx);
+        MB_CUDA(ctx, reset_rows(ctx));
+        MB_CUDA(ctx, build_rows(ctx, ctx->springs_placed, ctx->max_bin_springs));
+        MB_CUDA(ctx, tm_queue_rows(ctx));
         uint32_t status[2] = {0, 0};
-        MB_CUDA(ctx, cudaMemcpyAsync(status, ctx->devo_status.p, sizeof(status), cudaMemcpyDeviceToHost, st));
         MB_CUDA(ctx, cudaMemcpyAsync(ctx->h_bins.data(), ctx->bins.p, nb * sizeof(mb::BinDesc),
                                      cudaMemcpyDeviceToHost, st));
-        MB_CUDA(ctx, cudaStreamSynchronize(st));
+        MB_CUDA(ctx, read_status(ctx, status, true));
         if (status[0] || status[1] > mb::max_step_smem(ctx->device)) {
             if (rows_failed) *rows_failed = true;
             return MB_OK;
         }
         ctx->smem_bytes = status[1];  // the largest bin's need, exactly
+    } else if (tm_eligible(ctx)) {
+        uint32_t unused[2];
+        MB_CUDA(ctx, ctx->devo_status.alloc(2 + nb));
+        MB_CUDA(ctx, tm_queue_rows(ctx));
+        MB_CUDA(ctx, read_status(ctx, unused, true));
     }
-    ctx->tm_stale = true;
-    ctx->n_slices = (uint32_t)out.slice_off.size();
     // the host vectors of `out` may die after this call: wait for the copies
     MB_CUDA(ctx, cudaStreamSynchronize(st));
     return MB_OK;
@@ -697,7 +735,7 @@ mb_status split_devo_setup(mb_context* c) {
     MB_CUDA(c, c->free_taken.alloc(nb));
     MB_CUDA(c, c->free_slots.alloc(std::max<uint64_t>(ts, 1)));
     MB_CUDA(c, c->rows_scratch.alloc(2 * std::max<uint64_t>(ts, 1)));
-    MB_CUDA(c, c->devo_status.alloc(2));
+    MB_CUDA(c, c->devo_status.alloc(2 + nb));
     MB_CUDA(c, mb::launch_split_devo_setup(split_params(c, nullptr, 0, 0), nb, (uint32_t)S, st));
     MB_CUDA(c, cudaStreamSynchronize(st));
     c->n_packed = (uint32_t)ts;
@@ -734,7 +772,7 @@ mb_status devo_setup(mb_context* c) {
     MB_CUDA(c, cudaMemsetAsync(c->free_taken.p, 0, nb * sizeof(uint32_t), st));
     MB_CUDA(c, c->free_slots.alloc(c->n_packed));
     MB_CUDA(c, c->rows_scratch.alloc(2 * (size_t)c->n_packed));
-    MB_CUDA(c, c->devo_status.alloc(2));
+    MB_CUDA(c, c->devo_status.alloc(2 + nb));
     // rows get spare capacity: half their size plus 8 slice columns
     std::vector<uint32_t> begin(nb);
     std::vector<mb::BinDesc> nbins = c->h_bins;
@@ -913,7 +951,6 @@ mb_status voxel_setup(mb_context* c, uint32_t R, int sx, int sy, int sz, float h
     for (size_t i = 0; i < word.size(); ++i) word[i] = out.pair[i] & 0xFFFFFFu;
     for (size_t b = 0; b < out.bins.size(); ++b) nsp[b] = out.bins[b].n_spring;
     auto& v = c->vox;
-    v.max_bin_springs = nsp.empty() ? 0u : *std::max_element(nsp.begin(), nsp.end());
     MB_CUDA(c, up(v.word, word.data(), word.size()));
     MB_CUDA(c, up(v.lbar, out.lbar.data(), out.lbar.size()));
     MB_CUDA(c, up(v.gidx, out.spring_gidx.data(), out.spring_gidx.size()));
@@ -934,11 +971,7 @@ mb_status voxel_setup(mb_context* c, uint32_t R, int sx, int sy, int sz, float h
     MB_CUDA(c, cudaMemsetAsync(c->stress.p, 0, (S + 1) * sizeof(float), cs));
     MB_CUDA(c, c->robot_flags.alloc(R));
     MB_CUDA(c, c->com.alloc(3 * (size_t)R));
-    const uint32_t nb = c->n_bins;
-    MB_CUDA(c, c->free_count.alloc(nb));
-    MB_CUDA(c, c->free_taken.alloc(nb));
-    MB_CUDA(c, c->rows_scratch.alloc(2 * (size_t)c->n_packed));
-    MB_CUDA(c, c->devo_status.alloc(2));
+    MB_CUDA(c, c->devo_status.alloc(2 + c->n_bins));
     MB_CUDA(c, v.cells.alloc((size_t)R * sx * sy * sz));
     MB_CUDA(c, cudaStreamSynchronize(cs));
     v.valid = true;
@@ -1103,6 +1136,8 @@ mb_status mb_get_packed_springs(const mb_context* ctx, uint32_t* words, uint64_t
     if (!words) return MB_OK;
     if (capacity < ctx->n_packed) return MB_ERR_CAPACITY;
     cudaSetDevice(ctx->device);
+    // (springs are placed on demand; the caller sees them placed)
+    if (mb_detail::place_springs(const_cast<mb_context*>(ctx)) != cudaSuccess) return MB_ERR_CUDA;
     if (ctx->n_packed &&
         cudaMemcpyAsync(words, ctx->spring_pair.p, ctx->n_packed * sizeof(uint32_t), cudaMemcpyDeviceToHost,
                         ctx->stream) != cudaSuccess)
@@ -1328,40 +1363,82 @@ bool tm_eligible(const mb_context* c) {
     return mb::tm_holds(c->shape, c->streamed, c->cluster, c->max_bin_mass, c->max_degree);
 }
 
+// Queues the rows of the tensor-memory kernel from the packed rows, with their
+// slot counts behind the status words.
+cudaError_t tm_queue_rows(mb_context* c) {
+    if (!tm_eligible(c)) return cudaSuccess;
+    // one allocation for all arrays
+    const size_t n = c->inc.n + 32ull * c->n_slices;
+    size_t bytes = 0;
+    auto carve = [&](size_t count, size_t size) {
+        const size_t at = bytes;
+        bytes += (count * size + 255) & ~size_t(255);
+        return at;
+    };
+    const size_t own = carve(n, 8), gidx = carve(n, 4), gather = carve(n, 4), head = carve(c->n_slices, 16),
+                 n_mat = carve(c->n_bins, 4), mat = carve(c->n_bins, 256), col = carve(c->n_packed, 2);
+    const cudaError_t e = c->tm_arena.alloc(bytes);
+    if (e != cudaSuccess) return e;
+    uint8_t* p = c->tm_arena.p;
+    const mb::TmRows rows{reinterpret_cast<uint2*>(p + own),       reinterpret_cast<uint32_t*>(p + gidx),
+                          reinterpret_cast<uint32_t*>(p + gather), reinterpret_cast<uint4*>(p + head),
+                          c->devo_status.p + 2,                    reinterpret_cast<uint32_t*>(p + n_mat),
+                          p + mat,                                 reinterpret_cast<uint16_t*>(p + col)};
+    if (std::memcmp(&rows, &c->tm_rows, sizeof(rows)) != 0) c->clear_graphs();  // they hold the old ones
+    c->tm_rows = rows;
+    const mb::TmSource in{c->bins.p,        c->n_bins,  c->spring_pair.p, c->spring_lbar.p,
+                          c->spring_gidx.p, c->inc.p,   c->slice_off.p,   c->slice_width.p};
+    return mb::launch_tm_rows(in, c->tm_rows, c->stream);
+}
+
+// Waits for the status words of queued rows.  The plans of the tensor-memory
+// kernel, and the graphs that hold them, stay when they leave room for every
+// bin's slots (new_bins: they are of other bins).
+cudaError_t read_status(mb_context* c, uint32_t* status, bool new_bins) {
+    const uint32_t nb = c->n_bins;
+    const bool tm = tm_eligible(c);
+    c->h_status.resize(2 + nb);
+    cudaError_t e = cudaMemcpyAsync(c->h_status.data(), c->devo_status.p, (tm ? 2 + nb : 2) * sizeof(uint32_t),
+                                    cudaMemcpyDeviceToHost, c->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+    if (e != cudaSuccess) return e;
+    status[0] = c->h_status[0];
+    status[1] = c->h_status[1];
+    if (!tm) return cudaSuccess;
+    bool room = !new_bins && c->tm_slots.size() == nb;
+    if (!room) c->tm_slots.assign(nb, 0);
+    for (uint32_t b = 0; b < nb; ++b) {
+        if (c->h_status[2 + b] > c->tm_slots[b]) room = false;
+        c->tm_slots[b] = std::max(c->tm_slots[b], c->h_status[2 + b]);
+    }
+    if (!room) {
+        c->clear_graphs();
+        c->tm[0].planned = c->tm[1].planned = false;
+    }
+    c->tm_stale = false;
+    return cudaSuccess;
+}
+
+// Puts the springs into the order of the general kernel's loads, when they were
+// left in upload order for the tensor-memory kernel (whose rows do not depend on
+// it).
+cudaError_t place_springs(mb_context* c) {
+    if (c->springs_placed) return cudaSuccess;
+    cudaError_t e = reset_rows(c);
+    if (e == cudaSuccess) e = build_rows(c, true, c->max_bin_springs);
+    c->springs_placed = e == cudaSuccess;
+    return e;
+}
+
 // The rows of the tensor-memory kernel, when the packed rows changed (waits
 // for the stream), and its launch plan.
 cudaError_t tm_update(mb_context* c, bool track) {
     cudaError_t e = cudaSuccess;
     if (c->tm_stale) {
-        // one allocation for all arrays
-        const size_t n = c->inc.n + 32ull * c->n_slices;
-        size_t bytes = 0;
-        auto carve = [&](size_t count, size_t size) {
-            const size_t at = bytes;
-            bytes += (count * size + 255) & ~size_t(255);
-            return at;
-        };
-        const size_t own = carve(n, 8), gidx = carve(n, 4), gather = carve(n, 4), head = carve(c->n_slices, 16),
-                     slots = carve(c->n_bins, 4), n_mat = carve(c->n_bins, 4), mat = carve(c->n_bins, 256),
-                     col = carve(c->n_packed, 2);
-        e = c->tm_arena.alloc(bytes);
+        uint32_t unused[2];
+        e = tm_queue_rows(c);
+        if (e == cudaSuccess) e = read_status(c, unused, false);
         if (e != cudaSuccess) return e;
-        uint8_t* p = c->tm_arena.p;
-        c->tm_rows = mb::TmRows{reinterpret_cast<uint2*>(p + own),      reinterpret_cast<uint32_t*>(p + gidx),
-                                reinterpret_cast<uint32_t*>(p + gather), reinterpret_cast<uint4*>(p + head),
-                                reinterpret_cast<uint32_t*>(p + slots),  reinterpret_cast<uint32_t*>(p + n_mat),
-                                p + mat,                                 reinterpret_cast<uint16_t*>(p + col)};
-        const mb::TmSource in{c->bins.p,        c->n_bins,  c->spring_pair.p, c->spring_lbar.p,
-                              c->spring_gidx.p, c->inc.p,   c->slice_off.p,   c->slice_width.p};
-        e = mb::launch_tm_rows(in, c->tm_rows, c->stream);
-        c->tm_slots.resize(c->n_bins);
-        if (e == cudaSuccess)
-            e = cudaMemcpyAsync(c->tm_slots.data(), c->tm_rows.n_slots, c->n_bins * sizeof(uint32_t),
-                                cudaMemcpyDeviceToHost, c->stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-        if (e != cudaSuccess) return e;
-        c->clear_graphs();  // they hold the old rows and plan
-        c->tm_stale = c->tm[0].planned = c->tm[1].planned = false;
     }
     mb_context::TmLaunch& l = c->tm[track ? 1 : 0];
     const bool faces = face_drag_on(c) && c->faces_packed;
@@ -1371,7 +1448,8 @@ cudaError_t tm_update(mb_context* c, bool track) {
     mb::tm_plan(c->h_bins, c->tm_slots, c->grid ? c->grid : c->n_bins, c->n_mat_host, mb::max_step_smem(c->device),
                 track, faces, l.plan);
     if (l.plan.ok) {
-        std::vector<uint8_t> host;
+        std::vector<uint8_t>& host = l.host;
+        host.clear();
         auto put = [&](const auto& v) {
             const size_t at = (host.size() + 15) & ~size_t(15), n = v.size() * sizeof(v[0]);
             host.resize(at + n);
@@ -1385,7 +1463,6 @@ cudaError_t tm_update(mb_context* c, bool track) {
         if (l.arrays.p != old) c->clear_graphs();
         if (e == cudaSuccess)
             e = cudaMemcpyAsync(l.arrays.p, host.data(), host.size(), cudaMemcpyHostToDevice, c->stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);  // `host` dies here
     }
     l.planned = e == cudaSuccess;
     return e;
@@ -1520,6 +1597,7 @@ mb_status run(mb_context* c, uint32_t steps, bool track) {
     }
     cudaSetDevice(c->device);
     if (tm_eligible(c)) MB_CUDA(c, tm_update(c, track));
+    if (!use_tm(c, track)) MB_CUDA(c, place_springs(c));
     const float t0 = c->total_time;
     if (c->use_graph) {
         uint32_t bits;
@@ -1661,6 +1739,8 @@ mb_status mb_devo(mb_context* ctx, uint32_t replaced_per_robot, uint64_t seed, u
     // device (split_devo_setup prepares it once; MB_ERR_CAPACITY there, for
     // split populations with faces or beyond its limits: host re-pack)
     const bool split = ctx->cluster != 0;
+    // (development keeps the springs' slots from here on)
+    if (on_device) MB_CUDA(ctx, mb_detail::place_springs(ctx));
     if (on_device && !ctx->devo_ready) {
         const mb_status s = split ? mb_detail::split_devo_setup(ctx) : mb_detail::devo_setup(ctx);
         if (s == MB_ERR_CAPACITY && split)
@@ -1686,7 +1766,6 @@ mb_status mb_devo(mb_context* ctx, uint32_t replaced_per_robot, uint64_t seed, u
                              ctx->free_taken.p,  ctx->devo_status.p,   ctx->sp_keys.p,
                              ctx->sp_key_begin.p};
         MB_CUDA(ctx, mb::launch_rebuild(rp, st));
-        MB_CUDA(ctx, cudaMemcpyAsync(status, ctx->devo_status.p, sizeof(status), cudaMemcpyDeviceToHost, st));
         MB_CUDA(ctx, cudaMemcpyAsync(ctx->h_bins.data(), ctx->bins.p, ctx->h_bins.size() * sizeof(mb::BinDesc),
                                      cudaMemcpyDeviceToHost, st));
     } else if (on_device) {
@@ -1707,12 +1786,15 @@ mb_status mb_devo(mb_context* ctx, uint32_t replaced_per_robot, uint64_t seed, u
                              ctx->free_taken.p,  ctx->devo_status.p};
         MB_CUDA(ctx, mb::launch_rebuild(rp, st));
         ctx->tm_stale = true;
-        MB_CUDA(ctx, cudaMemcpyAsync(status, ctx->devo_status.p, sizeof(status), cudaMemcpyDeviceToHost, st));
+        MB_CUDA(ctx, mb_detail::tm_queue_rows(ctx));
     }
     ctx->h_devo.resize(nrec);
     MB_CUDA(ctx, cudaMemcpyAsync(ctx->h_devo.data(), ctx->devo_out.p, nrec * sizeof(mb::DevoRecord),
                                  cudaMemcpyDeviceToHost, st));
-    MB_CUDA(ctx, cudaStreamSynchronize(st));
+    if (on_device)
+        MB_CUDA(ctx, mb_detail::read_status(ctx, status, false));
+    else
+        MB_CUDA(ctx, cudaStreamSynchronize(st));
     uint32_t count = 0;
     for (const mb::DevoRecord& rec : ctx->h_devo) {
         if (rec.spring == 0xFFFFFFFFu) continue;
@@ -1778,9 +1860,7 @@ mb_status mb_set_voxel_population(mb_context* ctx, uint32_t n_robots, int sx, in
     cudaStream_t st = ctx->stream;
     const size_t nc = (size_t)n_robots * sx * sy * sz;
     MB_CUDA(ctx, cudaMemcpyAsync(v.cells.p, cells, nc, cudaMemcpyHostToDevice, st));
-    MB_CUDA(ctx, cudaMemsetAsync(ctx->devo_status.p, 0, 2 * sizeof(uint32_t), st));
-    MB_CUDA(ctx, cudaMemsetAsync(ctx->free_count.p, 0, ctx->n_bins * sizeof(uint32_t), st));
-    MB_CUDA(ctx, cudaMemsetAsync(ctx->free_taken.p, 0, ctx->n_bins * sizeof(uint32_t), st));
+    MB_CUDA(ctx, mb_detail::reset_rows(ctx));
     const mb::VoxelBuildParams bp{n_robots, sx, sy, sz, v.cells.p, v.pos.p, v.src.p, v.dir.p, v.n_springs, mass,
                                   ctx->pos.p, ctx->vel.p, ctx->mass_mat.p, ctx->d_spring_mat.p, ctx->stress.p,
                                   ctx->devo_status.p};
@@ -1789,23 +1869,15 @@ mb_status mb_set_voxel_population(mb_context* ctx, uint32_t n_robots, int sx, in
                                ctx->d_spring_mat.p, ctx->slot_of.p, ctx->spring_pair.p, ctx->spring_lbar.p,
                                ctx->spring_gidx.p, ctx->devo_status.p};
     MB_CUDA(ctx, mb::launch_compact(cp, st));
-    if (!ctx->streamed) {
-        // the compaction keeps the template's placement minus the air
-        // springs, which breaks its groups: the active springs are placed
-        // again for the endpoint loads (the template's counts bound the bins)
-        MB_CUDA(ctx, mb::launch_bank_place(ctx->bins.p, ctx->n_bins, v.max_bin_springs, ctx->spring_pair.p,
-                                           ctx->spring_gidx.p, ctx->spring_lbar.p, ctx->rows_scratch.p, st));
-    }
-    const mb::RebuildParams rp{ctx->bins.p,        ctx->n_bins,          ctx->spring_pair.p,
-                               ctx->spring_gidx.p, (uint32_t)ctx->n_spring, ctx->slice_off.p,
-                               ctx->slice_width.p, ctx->inc.p,           ctx->inc32.p,
-                               ctx->streamed ? 1u : 0u, ctx->rows_scratch.p, ctx->free_count.p,
-                               ctx->free_taken.p,  ctx->devo_status.p};
-    MB_CUDA(ctx, mb::launch_rebuild(rp, st));
-    uint32_t status[2] = {0, 0};
-    MB_CUDA(ctx, cudaMemcpyAsync(status, ctx->devo_status.p, sizeof(status), cudaMemcpyDeviceToHost, st));
-    MB_CUDA(ctx, cudaStreamSynchronize(st));
+    // the compaction keeps the template's placement minus the air springs, which
+    // breaks its groups: the active springs are placed again, unless a kernel
+    // steps them that does not read their order
+    ctx->springs_placed = ctx->streamed || !mb_detail::tm_eligible(ctx);
+    MB_CUDA(ctx, mb_detail::build_rows(ctx, !ctx->streamed && ctx->springs_placed, ctx->max_bin_springs));
     ctx->tm_stale = true;
+    MB_CUDA(ctx, mb_detail::tm_queue_rows(ctx));
+    uint32_t status[2] = {0, 0};
+    MB_CUDA(ctx, mb_detail::read_status(ctx, status, false));
     ctx->host_topology_stale = true;
     ctx->vox_live = true;
     ctx->devo_ready = false;

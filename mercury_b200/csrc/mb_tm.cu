@@ -1046,9 +1046,10 @@ struct TmArrangement {
     std::vector<uint8_t> group_of;  // per bin
 };
 
-// Arranges every CTA for one of the kernels.
+// Arranges every CTA for one of the kernels; not ok when a CTA's bins do not fit
+// or take `bound` us.
 void arrange(const std::vector<TmBinSize>& bins, uint32_t ctas, uint32_t n_mat, uint32_t smem_cap, const TmKernel& kernel,
-             bool faces, bool track, TmArrangement& out) {
+             bool faces, bool track, double bound, TmArrangement& out) {
     const uint32_t max_warps = kernel.max_warps, max_mpt = kernel.max_mpt;
     const TmKernel::Cost& k = kernel.cost[track];
     out = TmArrangement{};
@@ -1089,8 +1090,12 @@ void arrange(const std::vector<TmBinSize>& bins, uint32_t ctas, uint32_t n_mat, 
             }
             // warps: a slice each; where that is too many, one warp at a time
             // off the group with the most for its work
-            uint32_t total = 0;
-            for (uint32_t g = 0; g < G; ++g) total += a.warps[g] = a.most[g];
+            uint32_t total = 0, least = 0;
+            for (uint32_t g = 0; g < G; ++g) {
+                total += a.warps[g] = a.most[g];
+                least += (a.most[g] + max_mpt - 1) / max_mpt;
+            }
+            if (least > max_warps) continue;
             const bool all = total <= max_warps;
             while (total > max_warps) {
                 int from = -1;
@@ -1117,7 +1122,7 @@ void arrange(const std::vector<TmBinSize>& bins, uint32_t ctas, uint32_t n_mat, 
             for (uint32_t i = 0; i < n; ++i) out.group_of[mine[i]] = group[i];
             if (all && G == n) break;  // every bin at once, a warp a slice
         }
-        if (best < 0.0) return;
+        if (best < 0.0 || best >= bound) return;
         out.us = std::max(out.us, best);
     }
     out.ok = true;
@@ -1128,8 +1133,8 @@ TmArrangement arrange_best(const std::vector<TmBinSize>& bins, uint32_t ctas, ui
     TmArrangement best, a;
     for (const TmKernel& kernel : kTmKernels) {
         if (track && kernel.max_warps > kTmWideWarps && kernel.max_mpt > 1) continue;
-        arrange(bins, ctas, n_mat, smem_cap, kernel, faces, track, a);
-        if (a.ok && (!best.ok || a.us < best.us)) best = std::move(a);
+        arrange(bins, ctas, n_mat, smem_cap, kernel, faces, track, best.ok ? best.us : 1e30, a);
+        if (a.ok) best = std::move(a);
     }
     return best;
 }
