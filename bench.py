@@ -46,16 +46,19 @@ WORKLOADS = {
 }
 
 # Algorithmic bytes per spring-update.
-#   Shared memory (the binding resource of the resident step kernel, which
-#   keeps every robot on chip for a whole launch): 24 B for the two endpoint
-#   positions (2 x 3 floats) + 12 B for the correction the spring stores
-#   (3 floats) + 24 B for the two reads of that correction when its ends
-#   gather it (2 x 3 floats) = 60 B.
+#   Shared memory (the resident step kernels keep every robot on chip for a
+#   whole launch).  The tensor-memory kernel (tm_step_kernel): 12 B for the
+#   lower end's position (3 floats; the upper end's thread holds its own) + 12 B
+#   for the correction the spring stores + 12 B for the lower end's read of it
+#   + 12 B x masses/springs for the positions stored.  The general kernel
+#   (step_kernel): 24 B for two positions, 12 B stored and 24 B for two reads,
+#   and the positions.
 #   HBM, for a step that keeps nothing on chip (the reference's design):
 #   9 B topology (2 x u16 pair, u8 material, f32 mean length) + 8 B stress
 #   read+write when tracking + per-mass state (pos and vel, 3 floats each,
 #   read and write: 48 B) x masses/springs.
-SMEM_B = 60.0
+SMEM_B = {"tm_step_kernel": 36.0, "step_kernel": 60.0}
+SMEM_MASS_B = 12.0
 SMEM_NOMINAL_B_PER_CLK = 128.0  # shared-memory bandwidth of an SM (32 banks x 4 B per clock)
 HBM_TOPO_B, HBM_STRESS_B, HBM_MASS_B = 9.0, 8.0, 48.0
 
@@ -242,7 +245,10 @@ def run_ours(args, rank, local_rank, world):
     clocks = clk.summary()
     smem_peak, smem_clk = smem_peak_gbs(local_rank)
     hbm_ach = hbm_b * upd_launch / t_launch / 1e9
-    smem_ach = SMEM_B * upd_launch / t_launch / 1e9
+    kernel = ("stream_kernel" if cfg["streamed"] else
+              "tm_step_kernel" if sim.step_variant(track)["register_rows"] else "step_kernel")
+    smem_b = SMEM_B.get(kernel, SMEM_B["step_kernel"]) + SMEM_MASS_B * batch.n_masses / active
+    smem_ach = smem_b * upd_launch / t_launch / 1e9
 
     # plain configuration: one robot per CTA, one step per launch, no graph
     plain = None
@@ -329,11 +335,11 @@ def run_ours(args, rank, local_rank, world):
             "parallelism": f"population sharded over {world} GPU(s), no collective in the step",
         },
         "roofline": {"bound": "smem", "achieved": smem_ach, "peak": smem_peak, "unit": "GB/s",
-                     "frac": smem_ach / smem_peak, **_step_traffic(args.workload, cfg, active),
-                     "bytes_per_update": SMEM_B,
+                     "frac": smem_ach / smem_peak, **_step_traffic(args.workload, kernel, cfg),
+                     "bytes_per_update": smem_b,
                      "peak_source": f"measured: shared-memory read probe (mb_measure_smem_bandwidth) on this GPU, "
                                     f"{smem_clk:.1f} B/clk/SM",
-                     "kernel": "tm_step_kernel (resident: robots on chip for the whole launch)"},
+                     "kernel": kernel},
         "roofline_hbm": {"bound": "hbm", "achieved": hbm_ach, "peak": hbm_peak, "unit": "GB/s",
                          "frac": hbm_ach / hbm_peak, "bytes_per_update": hbm_b, "peak_source": hbm_src,
                          "note": "the HBM bytes a step that keeps nothing on chip (the reference's design) "
@@ -367,17 +373,15 @@ def _device_rate(sim, active, steps, track, dev):
 
 
 # DRAM bytes (read + write) of one 1,000-step launch of the step kernel on
-# the uneven population in the configurations the tuner picks (ncu,
-# dram__bytes_read.sum + dram__bytes_write.sum): the state and topology, read
-# once per launch.
-STEP_TRAFFIC = {("uneven", 1024, 8, 2, 296, 1000): 24.664e6 + 0.0,
-                ("uneven", 1024, 10, 2, 296, 1000): 24.666e6 + 0.0}
+# the uneven population (ncu, dram__bytes_read.sum + dram__bytes_write.sum): the
+# state and topology, read once per launch; by kernel, bins and steps.
+STEP_TRAFFIC = {("uneven", "tm_step_kernel", 444, 1000): 26.921e6 + 0.007e6}
 
 
-def _step_traffic(workload, cfg, active):
+def _step_traffic(workload, kernel, cfg):
     """Measured DRAM bytes per launch, when the bench runs the profiled
     configuration."""
-    key = (workload, cfg["threads"], cfg["springs_per_thread"], cfg["masses_per_thread"], cfg["bins"], cfg["chunk"])
+    key = (workload, kernel, cfg["bins"], cfg["chunk"])
     t = STEP_TRAFFIC.get(key)
     if t is None:
         return {"traffic": None}
