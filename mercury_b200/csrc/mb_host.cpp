@@ -1376,18 +1376,18 @@ cudaError_t tm_queue_rows(mb_context* c) {
         return at;
     };
     const size_t own = carve(n, 8), gidx = carve(n, 4), gather = carve(n, 4), head = carve(c->n_slices, 16),
-                 n_mat = carve(c->n_bins, 4), mat = carve(c->n_bins, 256), col = carve(c->n_packed, 2);
+                 n_mat = carve(c->n_bins, 4), mat = carve(c->n_bins, 256);
     const cudaError_t e = c->tm_arena.alloc(bytes);
     if (e != cudaSuccess) return e;
     uint8_t* p = c->tm_arena.p;
     const mb::TmRows rows{reinterpret_cast<uint2*>(p + own),       reinterpret_cast<uint32_t*>(p + gidx),
                           reinterpret_cast<uint32_t*>(p + gather), reinterpret_cast<uint4*>(p + head),
                           c->devo_status.p + 2,                    reinterpret_cast<uint32_t*>(p + n_mat),
-                          p + mat,                                 reinterpret_cast<uint16_t*>(p + col)};
+                          p + mat};
     if (std::memcmp(&rows, &c->tm_rows, sizeof(rows)) != 0) c->clear_graphs();  // they hold the old ones
     c->tm_rows = rows;
-    const mb::TmSource in{c->bins.p,        c->n_bins,  c->spring_pair.p, c->spring_lbar.p,
-                          c->spring_gidx.p, c->inc.p,   c->slice_off.p,   c->slice_width.p};
+    const mb::TmSource in{c->bins.p,        c->n_bins, c->max_bin_springs, c->spring_pair.p, c->spring_lbar.p,
+                          c->spring_gidx.p, c->inc.p,  c->slice_off.p,     c->slice_width.p};
     return mb::launch_tm_rows(in, c->tm_rows, c->stream);
 }
 
@@ -1405,13 +1405,14 @@ cudaError_t read_status(mb_context* c, uint32_t* status, bool new_bins) {
     status[0] = c->h_status[0];
     status[1] = c->h_status[1];
     if (!tm) return cudaSuccess;
+    const uint32_t* slots = c->h_status.data() + 2;
     bool room = !new_bins && c->tm_slots.size() == nb;
-    if (!room) c->tm_slots.assign(nb, 0);
-    for (uint32_t b = 0; b < nb; ++b) {
-        if (c->h_status[2 + b] > c->tm_slots[b]) room = false;
-        c->tm_slots[b] = std::max(c->tm_slots[b], c->h_status[2 + b]);
-    }
+    for (uint32_t b = 0; b < nb && room; ++b) room = slots[b] <= c->tm_slots[b];
     if (!room) {
+        // rows that have grown (development) will grow again: an eighth more
+        c->tm_slots.assign(slots, slots + nb);
+        if (!new_bins)
+            for (uint32_t& n : c->tm_slots) n += n / 8;
         c->clear_graphs();
         c->tm[0].planned = c->tm[1].planned = false;
     }
@@ -1447,6 +1448,15 @@ cudaError_t tm_update(mb_context* c, bool track) {
     l.planned = false;
     mb::tm_plan(c->h_bins, c->tm_slots, c->grid ? c->grid : c->n_bins, c->n_mat_host, mb::max_step_smem(c->device),
                 track, faces, l.plan);
+    if (!l.plan.ok && c->h_status.size() == 2 + (size_t)c->n_bins) {  // without room to grow
+        const std::vector<uint32_t> slots(c->h_status.begin() + 2, c->h_status.end());
+        if (slots != c->tm_slots) {
+            c->tm_slots = slots;
+            c->tm[track ? 0 : 1].planned = false;
+            mb::tm_plan(c->h_bins, c->tm_slots, c->grid ? c->grid : c->n_bins, c->n_mat_host,
+                        mb::max_step_smem(c->device), track, faces, l.plan);
+        }
+    }
     if (l.plan.ok) {
         std::vector<uint8_t>& host = l.host;
         host.clear();

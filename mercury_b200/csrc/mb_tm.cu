@@ -326,6 +326,11 @@ __global__ void __launch_bounds__(32 * (WIDE ? kTmWideWarps : kTmMaxWarps), 1) t
             const uint32_t spare = j && words > words_kept && words - words_kept <= kTmSpareWords
                                        ? smem0 + grp.spare_off + (128u * kTmSpareWords) * gw : 0u;
             const uint32_t c0 = tm + free_col;
+            uint32_t odd = 0;  // tracking: some mean length's reciprocal needs the general one
+            auto check_length = [&](uint32_t lb) {
+                const float x = __uint_as_float(lb);
+                if (TRACK) odd |= __float_as_uint(rcp_fast(x)) != __float_as_uint(__frcp_rn(x));
+            };
             __syncwarp();
 #pragma unroll 4
             for (uint32_t k = 0; k < own_kept; k += 2) {
@@ -333,19 +338,26 @@ __global__ void __launch_bounds__(32 * (WIDE ? kTmWideWarps : kTmMaxWarps), 1) t
                 const uint2 e1 = k + 1 < own_kept ? __ldg(&q.r.own[rw + 32 * (k + 1)]) : make_uint2(1u << 31, __float_as_uint(1.0f));
                 tm_st2(c0 + 2 * k, spring_word(e0.x, x0, mat0, n_mat), spring_word(e1.x, x0, mat0, n_mat));
                 tm_st2(c0 + 2 * k + 2, e0.y, e1.y);
+                check_length(e0.y);
+                check_length(e1.y);
+                __syncwarp();
             }
-            uint32_t odd = 0;  // some mean length's reciprocal needs the general one
-            if (TRACK)
-                for (uint32_t k = 0; k < own; ++k) {
-                    const float lb = __uint_as_float(__ldg(&q.r.own[rw + 32 * k]).y);
-                    odd |= __float_as_uint(rcp_fast(lb)) != __float_as_uint(__frcp_rn(lb));
-                    if (k >= own_kept) continue;
-                    const uint32_t g = __ldg(&q.r.gidx[rw + 32 * k]);
-                    const float st = g != ~0u ? p.stress[g & 0x7FFFFFFFu] : 0.0f;
+            if (TRACK) {
+                for (uint32_t k = own_kept; k < own; ++k) check_length(__ldg(&q.r.own[rw + 32 * k]).y);
+                odd = __any_sync(0xffffffffu, odd);
+                // stresses, eight at a time (loads of two latencies in a chain)
+                for (uint32_t k = 0; k < own_kept; k += 8) {
+                    uint32_t g[8], st[8];
+#pragma unroll
+                    for (uint32_t u = 0; u < 8; ++u) g[u] = k + u < own_kept ? __ldg(&q.r.gidx[rw + 32 * (k + u)]) : ~0u;
+#pragma unroll
+                    for (uint32_t u = 0; u < 8; ++u) st[u] = g[u] != ~0u ? __float_as_uint(p.stress[g[u] & 0x7FFFFFFFu]) : 0u;
                     __syncwarp();
-                    tm_st(c0 + tc.stress + k, __float_as_uint(st));
+#pragma unroll
+                    for (uint32_t u = 0; u < 8; u += 2)
+                        if (k + u < own_kept) tm_st2(c0 + tc.stress + k + u, st[u], st[u + 1]);
                 }
-            if (TRACK) odd = __any_sync(0xffffffffu, odd);
+            }
             info_own = make_uint4(xy0 + 8u * h.y, z0 + 4u * h.y, own_kept | own << 16 | odd << 31, c0);
             info_gather = make_uint4(c0 + tc.gather, words_kept | words << 16, spare, 0u);
             if (lane == 0) {
@@ -757,13 +769,17 @@ __global__ void __launch_bounds__(32 * (WIDE ? kTmWideWarps : kTmMaxWarps), 1) t
                 const uint32_t rw = __ldg(&q.r.head[TM_BIN(slice_begin) + gw + j * grp.warps]).z + lane;
                 const uint4 info = lds_info(info_mine + j * GT);
                 const uint32_t kept = info.z & 0xFFFFu, ts = info.w + 4 * ((kept + 1) / 2);
-                for (uint32_t k = 0; k < kept; ++k) {
-                    uint32_t st[1];
+#pragma unroll 2
+                for (uint32_t k = 0; k < kept; k += 4) {
+                    uint32_t st[4], g[4];
                     __syncwarp();
-                    tm_ld(ts + k, st);
-                    asm volatile("tcgen05.wait::ld.sync.aligned;" : "+r"(st[0]));
-                    const uint32_t g = __ldg(&q.r.gidx[rw + 32 * k]);
-                    if (!(g >> 31)) p.stress[g] = __uint_as_float(st[0]);  // bit 31: a copy in a split part, or padding
+                    tm_ld(ts + k, st);  // (past the last one: words of this warp, not used)
+#pragma unroll
+                    for (uint32_t u = 0; u < 4; ++u) g[u] = k + u < kept ? __ldg(&q.r.gidx[rw + 32 * (k + u)]) : ~0u;
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" : "+r"(st[0]), "+r"(st[1]), "+r"(st[2]), "+r"(st[3]));
+#pragma unroll
+                    for (uint32_t u = 0; u < 4; ++u)  // bit 31: a copy in a split part, or padding
+                        if (!(g[u] >> 31)) p.stress[g[u]] = __uint_as_float(st[u]);
                 }
             }
         }
@@ -775,20 +791,35 @@ __global__ void __launch_bounds__(32 * (WIDE ? kTmWideWarps : kTmMaxWarps), 1) t
     tm_free(tmem0, cols);
 }
 
-// One CTA per bin, one warp per slice of 32 masses.
-__global__ void __launch_bounds__(1024) tm_rows_kernel(const TmSource in, const TmRows r) {
+// One CTA per bin, a warp per slice of 32 masses.  Bound by latency: three passes
+// over the rows that look every entry's spring up, so the springs' words and
+// columns lie in shared memory and lengths are loaded four entries at a time.
+// 444 bins of 512 robots of 3-8 cells: 102 us with 32 warps a CTA (most bins have
+// 11 slices), 89 with 16, 87 with 12, 126 with 8.
+constexpr uint32_t kRowBytes = sizeof(uint32_t) + sizeof(uint16_t);  // shared memory of a spring
+constexpr uint32_t kRowThreads = 384;
+__global__ void __launch_bounds__(kRowThreads) tm_rows_kernel(const TmSource in, const TmRows r) {
+    extern __shared__ uint32_t tm_rows_smem[];
     __shared__ uint32_t n_own[kTmMaxSlices], first_slot[kTmMaxSlices];
     __shared__ uint32_t used[8];
+    __shared__ uint8_t rank_of[256];
     const uint32_t b = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
     const BinDesc bd = in.bins[b];
     const uint32_t n_slices = (bd.n_mass + 31) / 32;
-    const uint32_t* pairs = in.spring_pair + bd.spring_begin;
-    uint16_t* col = r.col + bd.spring_begin;
+    uint32_t* pairs = tm_rows_smem;
+    uint16_t* col = reinterpret_cast<uint16_t*>(pairs + bd.n_spring);
+    uint32_t room;
+    asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(room));
+    if (bd.n_spring > room / kRowBytes) {  // the launch was sized for fewer: no plan takes the bin
+        if (tid == 0) r.n_slots[b] = ~0u;
+        return;
+    }
     // 1. the materials in use, numbered in slot order
     if (tid < 8) used[tid] = 0;
     __syncthreads();
     for (uint32_t s = tid; s < bd.n_spring; s += blockDim.x) {
-        const uint32_t slot = pairs[s] >> 24;
+        const uint32_t w = in.spring_pair[bd.spring_begin + s], slot = w >> 24;
+        pairs[s] = w;
         if (!((((volatile uint32_t*)used)[slot >> 5] >> (slot & 31u)) & 1u)) atomicOr(&used[slot >> 5], 1u << (slot & 31u));
     }
     __syncthreads();
@@ -797,17 +828,21 @@ __global__ void __launch_bounds__(1024) tm_rows_kernel(const TmSource in, const 
         for (uint32_t k = 0; k < (slot >> 5); ++k) i += __popc(used[k]);
         return i;
     };
-    if (tid < 256 && ((used[tid >> 5] >> (tid & 31u)) & 1u)) r.mat[256u * b + rank(tid)] = (uint8_t)tid;
+    if (tid < 256) {
+        rank_of[tid] = (uint8_t)rank(tid);
+        if ((used[tid >> 5] >> (tid & 31u)) & 1u) r.mat[256u * b + rank_of[tid]] = (uint8_t)tid;
+    }
     if (tid == 0) {
         uint32_t n = 0;
         for (uint32_t k = 0; k < 8; ++k) n += __popc(used[k]);
         r.n_mat[b] = n;
     }
+    __syncthreads();
     // an entry of mass m: 0 padding, 1 its own (other end lower), 2 to gather
     auto kind = [&](uint32_t e, uint32_t m, uint32_t& pw, uint32_t& other) {
         pw = other = 0;
         if (e == kPadEntry) return 0u;
-        pw = __ldg(&pairs[e >> 1]);
+        pw = pairs[e >> 1];
         other = (e & 1u) ? pw & 0xFFFu : (pw >> 12) & 0xFFFu;
         // a spring from a mass to itself (no force): owned once
         return other < m || (other == m && (e & 1u)) ? 1u : other == m ? 0u : 2u;
@@ -819,7 +854,7 @@ __global__ void __launch_bounds__(1024) tm_rows_kernel(const TmSource in, const 
         const uint16_t* inc = in.inc + off + lane;
         uint32_t nneg = 0, npos = 0, cneg = 0, cpos = 0, pw, o;
         bool pure = true;  // every column is all own or all to gather
-#pragma unroll 4
+#pragma unroll 8
         for (uint32_t k = 0; k < w; ++k) {
             const uint32_t t = kind(inc[32 * k], m, pw, o);
             const bool an = __any_sync(0xffffffffu, t == 1u), ap = __any_sync(0xffffffffu, t == 2u);
@@ -838,25 +873,40 @@ __global__ void __launch_bounds__(1024) tm_rows_kernel(const TmSource in, const 
                 r.gidx[at0 + 32 * k] = ~0u;
             }
         uint32_t at = 0;  // next own column: of the slice when pure, else of the lane
-#pragma unroll 2
-        for (uint32_t k = 0; k < w; ++k) {
-            const uint32_t e = inc[32 * k], t = kind(e, m, pw, o);
-            const bool an = __any_sync(0xffffffffu, t == 1u);
-            if (t == 1u) {
-                r.own[at0 + 32 * at] = make_uint2(o | rank(pw >> 24) << 16, __float_as_uint(in.spring_lbar[bd.spring_begin + (e >> 1)]));
-                r.gidx[at0 + 32 * at] = in.spring_gidx[bd.spring_begin + (e >> 1)];
-                col[e >> 1] = (uint16_t)at;
+        for (uint32_t k0 = 0; k0 < w; k0 += 4) {
+            uint32_t es[4], ts[4], os[4], ms[4], gi[4];
+            float lb[4];
+#pragma unroll
+            for (uint32_t u = 0; u < 4; ++u) es[u] = k0 + u < w ? inc[32 * (k0 + u)] : kPadEntry;
+#pragma unroll
+            for (uint32_t u = 0; u < 4; ++u) {
+                ts[u] = kind(es[u], m, pw, os[u]);
+                ms[u] = rank_of[pw >> 24];
+                gi[u] = ts[u] == 1u ? in.spring_gidx[bd.spring_begin + (es[u] >> 1)] : ~0u;
+                lb[u] = ts[u] == 1u ? in.spring_lbar[bd.spring_begin + (es[u] >> 1)] : 1.0f;
             }
-            if (pure && an) {  // stand-ins of a bank group the quarter-warp's others leave free
-                uint32_t mask = t == 1u ? 1u << (o & 7u) : 0u;
-                for (uint32_t x = 1; x < 8; x *= 2) mask |= __shfl_xor_sync(0xffffffffu, mask, x);
-                if (t != 1u) {
-                    r.own[at0 + 32 * at] = make_uint2(1u << 31 | (mask == 0xFFu ? 0u : (uint32_t)__ffs(~mask & 0xFFu) - 1u),
-                                                      __float_as_uint(1.0f));
-                    r.gidx[at0 + 32 * at] = ~0u;
+#pragma unroll
+            for (uint32_t u = 0; u < 4; ++u) {
+                if (k0 + u >= w) break;
+                const uint32_t t = ts[u];
+                o = os[u];
+                const bool an = __any_sync(0xffffffffu, t == 1u);
+                if (t == 1u) {
+                    r.own[at0 + 32 * at] = make_uint2(o | ms[u] << 16, __float_as_uint(lb[u]));
+                    r.gidx[at0 + 32 * at] = gi[u];
+                    col[es[u] >> 1] = (uint16_t)at;
                 }
+                if (pure && an) {  // stand-ins of a bank group the quarter-warp's others leave free
+                    uint32_t mask = t == 1u ? 1u << (o & 7u) : 0u;
+                    for (uint32_t x = 1; x < 8; x *= 2) mask |= __shfl_xor_sync(0xffffffffu, mask, x);
+                    if (t != 1u) {
+                        r.own[at0 + 32 * at] = make_uint2(1u << 31 | (mask == 0xFFu ? 0u : (uint32_t)__ffs(~mask & 0xFFu) - 1u),
+                                                          __float_as_uint(1.0f));
+                        r.gidx[at0 + 32 * at] = ~0u;
+                    }
+                }
+                at += pure ? an : t == 1u;
             }
-            at += pure ? an : t == 1u;
         }
     }
     __syncthreads();
@@ -887,7 +937,7 @@ __global__ void __launch_bounds__(1024) tm_rows_kernel(const TmSource in, const 
             const uint32_t e = inc[32 * k], t = kind(e, m, pw, o);
             const bool ap = __any_sync(0xffffffffu, t == 2u);
             if (t == 2u) {
-                const uint32_t slot = first_slot[o / 32] + 32u * __ldcg(&col[e >> 1]) + (o & 31u);
+                const uint32_t slot = first_slot[o / 32] + 32u * col[e >> 1] + (o & 31u);
                 half[2 * (32 * (at / 2) + lane) + (at & 1u)] = (uint16_t)slot;
             }
             at += pure ? ap : t == 2u;
@@ -935,7 +985,11 @@ TmFn tm_kernel(uint32_t mode, bool track, const TmPlan& plan) {
 
 cudaError_t launch_tm_rows(const TmSource& in, const TmRows& r, cudaStream_t s) {
     if (in.n_bins == 0) return cudaSuccess;
-    tm_rows_kernel<<<in.n_bins, 1024, 0, s>>>(in, r);
+    // (one value for every launch: the attribute is the process's)
+    const cudaError_t e = cudaFuncSetAttribute(tm_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)(kMaxBinSprings * kRowBytes));
+    if (e != cudaSuccess) return e;
+    tm_rows_kernel<<<in.n_bins, kRowThreads, std::min(in.max_bin_springs, kMaxBinSprings) * kRowBytes, s>>>(in, r);
     return cudaGetLastError();
 }
 

@@ -95,11 +95,11 @@ struct TmRows {
     uint32_t* n_slots;  // per bin: correction slots
     uint32_t* n_mat;    // per bin: materials in use
     uint8_t* mat;       // per bin: 256 material slots, in order
-    uint16_t* col;      // scratch, one entry per packed spring
 };
 struct TmSource {
     const BinDesc* bins;
     uint32_t n_bins;
+    uint32_t max_bin_springs;  // packed springs of a bin, at most
     const uint32_t* spring_pair;
     const float* spring_lbar;
     const uint32_t* spring_gidx;
