@@ -870,7 +870,9 @@ cudaError_t launch_bank_place(const BinDesc* bins, uint32_t n_bins, uint32_t max
     // the opt-in covers the static windows too: static + dynamic above 48 KB
     // needs it, so it is set on every launch
     const size_t smem = (size_t)max_springs * (sizeof(uint32_t) + sizeof(uint16_t)) + 4u;
-    cudaError_t e = cudaFuncSetAttribute(bank_place_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // (the most any launch asks for: the attribute is the process's)
+    const cudaError_t e = cudaFuncSetAttribute(bank_place_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)(kMaxBinSprings * (sizeof(uint32_t) + sizeof(uint16_t)) + 4u));
     if (e != cudaSuccess) return e;
     bank_place_kernel<<<n_bins, kPlaceThreads, smem, s>>>(bins, pair, gidx, lbar, scratch);
     return cudaGetLastError();

@@ -188,6 +188,11 @@ __host__ __device__ inline uint32_t split_face_smem_bytes(uint32_t x_stride, uin
 // Largest dynamic shared memory the step kernel may use on this device.
 uint32_t max_step_smem(int device);
 
+// Lets launches of a kernel without static shared memory ask for `smem_bytes`:
+// for all that the current device gives, since the attribute is the process's and
+// another thread may be about to launch the kernel with more.
+cudaError_t allow_smem(const void* kernel, uint32_t smem_bytes);
+
 // Whether a kernel shape is compiled in.
 bool shape_supported(const KernelShape& shape);
 // Centre of mass of the non-air masses of each robot: one warp per robot.

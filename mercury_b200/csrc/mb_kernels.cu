@@ -727,6 +727,15 @@ uint32_t max_step_smem(int device) {
     return (uint32_t)v;
 }
 
+cudaError_t allow_smem(const void* kernel, uint32_t smem_bytes) {
+    int device = 0;
+    const cudaError_t e = cudaGetDevice(&device);
+    if (e != cudaSuccess) return e;
+    const uint32_t most = max_step_smem(device);
+    if (smem_bytes > most) return cudaErrorInvalidValue;
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+}
+
 bool shape_supported(const KernelShape& shape) { return find_shape(shape) != nullptr; }
 
 bool split_supported(const KernelShape& shape) { return find_split(shape) != nullptr; }
@@ -734,11 +743,9 @@ bool split_supported(const KernelShape& shape) { return find_split(shape) != nul
 cudaError_t prepare_split(const KernelShape& shape, uint32_t mode, bool track, uint32_t smem_bytes) {
     const ShapeEntry* e = find_split(shape);
     if (!e || mode > kModeForceWater) return cudaErrorInvalidValue;
-    cudaError_t r = cudaFuncSetAttribute(e->fn[mode][track ? 1 : 0], cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem_bytes);
+    cudaError_t r = allow_smem(reinterpret_cast<const void*>(e->fn[mode][track ? 1 : 0]), smem_bytes);
     if (r == cudaSuccess && mode == kModeForceWater)  // and the face-drag variant
-        r = cudaFuncSetAttribute(e->fn[kModeForceWaterFaces][track ? 1 : 0],
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes);
+        r = allow_smem(reinterpret_cast<const void*>(e->fn[kModeForceWaterFaces][track ? 1 : 0]), smem_bytes);
     return r;
 }
 
@@ -768,11 +775,9 @@ cudaError_t launch_split(const StepParams& p, const KernelShape& shape, uint32_t
 cudaError_t prepare_step(const KernelShape& shape, uint32_t mode, bool track, uint32_t smem_bytes) {
     const ShapeEntry* e = find_shape(shape);
     if (!e || mode > kModeForceWater) return cudaErrorInvalidValue;
-    cudaError_t r = cudaFuncSetAttribute(e->fn[mode][track ? 1 : 0], cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem_bytes);
+    cudaError_t r = allow_smem(reinterpret_cast<const void*>(e->fn[mode][track ? 1 : 0]), smem_bytes);
     if (r == cudaSuccess && mode == kModeForceWater)  // and the face-drag variant
-        r = cudaFuncSetAttribute(e->fn[kModeForceWaterFaces][track ? 1 : 0],
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes);
+        r = allow_smem(reinterpret_cast<const void*>(e->fn[kModeForceWaterFaces][track ? 1 : 0]), smem_bytes);
     return r;
 }
 
@@ -780,8 +785,7 @@ int ctas_per_sm(const KernelShape& shape, uint32_t mode, bool track, uint32_t sm
     const ShapeEntry* e = find_shape(shape);
     if (!e || mode > kModeForceWater) return 0;
     StepFn fn = e->fn[mode][track ? 1 : 0];
-    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes) != cudaSuccess)
-        return 0;
+    if (allow_smem(reinterpret_cast<const void*>(fn), smem_bytes) != cudaSuccess) return 0;
     int n = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, (int)shape.threads, smem_bytes) != cudaSuccess)
         return 0;
@@ -792,8 +796,7 @@ int max_active_clusters(const KernelShape& shape, uint32_t mode, uint32_t cluste
     const ShapeEntry* e = find_split(shape);
     if (!e || mode > kModeForceWater || cluster < 1 || cluster > kMaxClusterParts) return 0;
     StepFn fn = e->fn[mode][0];
-    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes) != cudaSuccess)
-        return 0;
+    if (allow_smem(reinterpret_cast<const void*>(fn), smem_bytes) != cudaSuccess) return 0;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(cluster, 1, 1);
     cfg.blockDim = dim3(shape.threads, 1, 1);
@@ -837,11 +840,9 @@ cudaError_t prepare_stream(uint32_t threads, uint32_t mpt, uint32_t mode, bool t
                            uint32_t smem_bytes) {
     const StreamEntry* e = find_stream(threads, mpt);
     if (!e || mode > kModeForceWater) return cudaErrorInvalidValue;
-    cudaError_t r = cudaFuncSetAttribute(e->fn[mode][track ? 1 : 0],
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes);
+    cudaError_t r = allow_smem(reinterpret_cast<const void*>(e->fn[mode][track ? 1 : 0]), smem_bytes);
     if (r == cudaSuccess && mode == kModeForceWater)  // and the face-drag variant
-        r = cudaFuncSetAttribute(e->fn[kModeForceWaterFaces][track ? 1 : 0],
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes);
+        r = allow_smem(reinterpret_cast<const void*>(e->fn[kModeForceWaterFaces][track ? 1 : 0]), smem_bytes);
     return r;
 }
 

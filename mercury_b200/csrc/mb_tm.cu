@@ -995,7 +995,7 @@ cudaError_t launch_tm_rows(const TmSource& in, const TmRows& r, cudaStream_t s) 
 
 cudaError_t prepare_tm(uint32_t mode, bool track, const TmPlan& plan) {
     const TmFn f = tm_kernel(mode, track, plan);
-    return f ? cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.smem) : cudaErrorInvalidValue;
+    return f ? allow_smem(reinterpret_cast<const void*>(f), plan.smem) : cudaErrorInvalidValue;
 }
 
 cudaError_t launch_tm(const TmParams& q, const TmPlan& plan, cudaStream_t s) {
