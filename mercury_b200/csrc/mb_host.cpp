@@ -301,6 +301,7 @@ cudaError_t reset_rows(mb_context* c);
 cudaError_t build_rows(mb_context* c, bool place, uint32_t max_bin_springs);
 cudaError_t tm_queue_rows(mb_context* c);
 cudaError_t read_status(mb_context* c, uint32_t* status, bool new_bins);
+void drop_plans(mb_context* c);
 cudaError_t tm_update(mb_context* c, bool track);
 cudaError_t place_springs(mb_context* c);
 
@@ -1391,6 +1392,13 @@ cudaError_t tm_queue_rows(mb_context* c) {
     return mb::launch_tm_rows(in, c->tm_rows, c->stream);
 }
 
+// The plans no longer hold, nor do the graphs with their launches: a new plan
+// takes the old one's place in device memory.
+void drop_plans(mb_context* c) {
+    c->clear_graphs();
+    c->tm[0].planned = c->tm[1].planned = false;
+}
+
 // Waits for the status words of queued rows.  The plans of the tensor-memory
 // kernel, and the graphs that hold them, stay when they leave room for every
 // bin's slots (new_bins: they are of other bins).
@@ -1413,8 +1421,7 @@ cudaError_t read_status(mb_context* c, uint32_t* status, bool new_bins) {
         c->tm_slots.assign(slots, slots + nb);
         if (!new_bins)
             for (uint32_t& n : c->tm_slots) n += n / 8;
-        c->clear_graphs();
-        c->tm[0].planned = c->tm[1].planned = false;
+        drop_plans(c);
     }
     c->tm_stale = false;
     return cudaSuccess;
@@ -1452,7 +1459,7 @@ cudaError_t tm_update(mb_context* c, bool track) {
         const std::vector<uint32_t> slots(c->h_status.begin() + 2, c->h_status.end());
         if (slots != c->tm_slots) {
             c->tm_slots = slots;
-            c->tm[track ? 0 : 1].planned = false;
+            drop_plans(c);
             mb::tm_plan(c->h_bins, c->tm_slots, c->grid ? c->grid : c->n_bins, c->n_mat_host,
                         mb::max_step_smem(c->device), track, faces, l.plan);
         }
