@@ -413,7 +413,7 @@ uint32_t plan_tm_bins(const std::vector<RobotPack>& packs, uint32_t ctas, const 
     const uint32_t n = (uint32_t)per.size();
     std::vector<std::vector<std::vector<uint32_t>>> plans(n);
     std::vector<double> us(n, 0.0);
-    parallel_for(n, threads, [&](uint32_t i) {
+    auto estimate = [&](uint32_t i, double bound) {
         if (!fill_groups(packs, members, per[i], sh, smem_cap, plans[i])) return;
         std::vector<TmBinSize> sizes;
         for (const auto& robots : plans[i]) {
@@ -427,10 +427,19 @@ uint32_t plan_tm_bins(const std::vector<RobotPack>& packs, uint32_t ctas, const 
             if (b.n_mass) b.slots += (uint32_t)(slots * (32 * ((b.n_mass + 31) / 32)) / b.n_mass);
             sizes.push_back(b);
         }
-        us[i] = tm_estimate(sizes, ctas, n_mat, smem_cap, false, false);
+        us[i] = tm_estimate(sizes, ctas, n_mat, smem_cap, false, false, bound);
         // (between equals, the one that tracks stresses faster)
-        if (us[i] > 0.0) us[i] += 0.02 * tm_estimate(sizes, ctas, n_mat, smem_cap, true, false);
-    });
+        if (us[i] > 0.0) us[i] += 0.02 * tm_estimate(sizes, ctas, n_mat, smem_cap, true, false, 1e30);
+    };
+    // few bins first: more take longer to estimate (12 and 16 bins of small
+    // robots 2 ms of an upload), and mostly end at the first CTA that is slower
+    uint32_t few = 0;
+    while (few < n && per[few] <= 4) ++few;
+    parallel_for(few, threads, [&](uint32_t i) { estimate(i, 1e30); });
+    double least = 1e30;
+    for (uint32_t i = 0; i < few; ++i)
+        if (us[i] > 0.0) least = std::min(least, us[i]);
+    parallel_for(n - few, threads, [&](uint32_t i) { estimate(few + i, least); });
     uint32_t best = n;
     for (uint32_t i = 0; i < n; ++i)
         if (us[i] > 0.0 && (best == n || us[i] < us[best])) best = i;

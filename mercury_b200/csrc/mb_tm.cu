@@ -25,8 +25,9 @@
 // A step of those 512 robots then takes 21 wavefronts per 32 springs and 98
 // instructions per spring, 5.3 us instead of 7.3.  What bounds it now is issue
 // (69 %) and the warps waiting at barriers (a quarter of the stalls).  Two
-// kernels: at most 24 warps of 80 registers (they spill 12-52 bytes a thread;
-// 28 warps of 72 registers and 32 of 64 measured 7.4 and 8.3 us there), and at
+// kernels: at most 24 warps of 80 registers (without tracking they spill 4-28
+// bytes a thread and load 4-52; 28 warps of 72 registers and 32 of 64 measured
+// 7.4 and 8.3 us there), and at
 // most 16 of up to 128 (WIDE, below); the plan takes the one whose estimated
 // step is shorter.
 // With stress tracking the same 512 robots take 7.8 us (8.5 with the springs
@@ -1183,11 +1184,11 @@ void arrange(const std::vector<TmBinSize>& bins, uint32_t ctas, uint32_t n_mat, 
 }
 
 TmArrangement arrange_best(const std::vector<TmBinSize>& bins, uint32_t ctas, uint32_t n_mat, uint32_t smem_cap,
-                           bool track, bool faces) {
+                           bool track, bool faces, double bound = 1e30) {
     TmArrangement best, a;
     for (const TmKernel& kernel : kTmKernels) {
         if (track && kernel.max_warps > kTmWideWarps && kernel.max_mpt > 1) continue;
-        arrange(bins, ctas, n_mat, smem_cap, kernel, faces, track, best.ok ? best.us : 1e30, a);
+        arrange(bins, ctas, n_mat, smem_cap, kernel, faces, track, best.ok ? best.us : bound, a);
         if (a.ok) best = std::move(a);
     }
     return best;
@@ -1196,8 +1197,8 @@ TmArrangement arrange_best(const std::vector<TmBinSize>& bins, uint32_t ctas, ui
 }  // namespace
 
 double tm_estimate(const std::vector<TmBinSize>& bins, uint32_t ctas, uint32_t n_mat, uint32_t smem_cap, bool track,
-                   bool faces) {
-    const TmArrangement a = arrange_best(bins, ctas, n_mat, smem_cap, track, faces);
+                   bool faces, double bound) {
+    const TmArrangement a = arrange_best(bins, ctas, n_mat, smem_cap, track, faces, bound);
     return a.ok ? a.us : 0.0;
 }
 

@@ -61,12 +61,13 @@ struct TmPlan {
 void tm_plan(const std::vector<BinDesc>& bins, const std::vector<uint32_t>& slots, uint32_t ctas, uint32_t n_mat,
              uint32_t smem_cap, bool track, bool faces, TmPlan& out);
 
-// Estimated time of a step of such a launch, us (0: no arrangement).
+// Estimated time of a step of such a launch, us (0: no arrangement, or none
+// shorter than `bound`).
 struct TmBinSize {
     uint32_t n_mass, slots, n_face;
 };
 double tm_estimate(const std::vector<TmBinSize>& bins, uint32_t ctas, uint32_t n_mat, uint32_t smem_cap, bool track,
-                   bool faces);
+                   bool faces, double bound);
 
 // Correction slots of a bin from its SELL rows on the host, as the row kernel
 // counts them (launch planning without a GPU).
