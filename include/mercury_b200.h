@@ -298,7 +298,7 @@ MB_API mb_status mb_set_launch_config(mb_context* ctx, const mb_launch_config* c
  * stream.  Either pointer may be NULL.  No reference counterpart. */
 MB_API mb_status mb_get_step_variant(const mb_context* ctx, uint32_t* register_rows, uint32_t* smem_bytes);
 
-/* The same for the next launches with stress tracking. */
+/* The same for the next launches with stress tracking, of more than two steps. */
 MB_API mb_status mb_get_tracked_step_variant(const mb_context* ctx, uint32_t* register_rows, uint32_t* smem_bytes);
 
 /* The packed spring slots of the uploaded batch, in device order: *count =

@@ -298,6 +298,7 @@ namespace mb_detail {
 
 bool tm_eligible(const mb_context* c);
 bool use_tm(const mb_context* c, bool track);
+bool short_launch(const mb_context* c, bool track, uint32_t steps);
 cudaError_t reset_rows(mb_context* c);
 cudaError_t build_rows(mb_context* c, bool place, uint32_t max_bin_springs);
 cudaError_t tm_queue_rows(mb_context* c);
@@ -1490,6 +1491,18 @@ cudaError_t tm_update(mb_context* c, bool track) {
     return e;
 }
 
+// Launches of one or two tracked steps, which the general kernel ends before the
+// tensor-memory kernel has stresses and springs in tensor memory and back: one
+// step of 1,000 robots of 3-8 cells 46 us instead of 62, of 512 28 instead of 34, of
+// one of 5 cells 13 instead of 17.5; three steps of 512 46 on either.  Not where a
+// CTA's bins are several and small, which the general kernel steps one after
+// another (1,500 robots of 3-6 cells, 318 masses a bin: 50 instead of 46; those
+// above have 530-580 or a bin a CTA).  Without tracking they are equal within
+// 1 us, or the tensor-memory kernel is faster.
+bool short_launch(const mb_context* c, bool track, uint32_t steps) {
+    return track && std::min(steps, c->chunk) <= 2 && (!c->grid || c->n_mass >= 384ull * c->n_bins);
+}
+
 // Whether the next steps run on it (after tm_update).
 bool use_tm(const mb_context* c, bool track) {
     const mb_context::TmLaunch& l = c->tm[track ? 1 : 0];
@@ -1551,11 +1564,11 @@ cudaError_t launch_tm_steps(mb_context* c, const mb::StepParams& p) {
 }
 
 // Kernel attributes of the next launches (they cannot change inside a capture).
-cudaError_t prepare_launch(mb_context* c, bool track) {
+cudaError_t prepare_launch(mb_context* c, bool track, bool tm) {
     const uint32_t mode = (uint32_t)c->mode;
     if (c->streamed) return mb::prepare_stream(1024, c->stream_mpt, mode, track, c->smem_bytes);
     if (c->cluster) return mb::prepare_split(c->shape, mode, track, c->smem_bytes);
-    if (use_tm(c, track)) return mb::prepare_tm(mode, track, c->tm[track ? 1 : 0].plan);
+    if (tm) return mb::prepare_tm(mode, track, c->tm[track ? 1 : 0].plan);
     return mb::prepare_step(c->shape, mode, track, c->smem_bytes);
 }
 
@@ -1588,7 +1601,7 @@ cudaError_t launch_split_groups(mb_context* c, const mb::StepParams& p) {
 }
 
 // Issues the chunk launches for `steps` steps from clock t0 on the stream.
-cudaError_t issue_chunks(mb_context* c, float t0, uint32_t steps, bool track) {
+cudaError_t issue_chunks(mb_context* c, float t0, uint32_t steps, bool track, bool tm) {
     float t = t0;
     uint32_t done = 0;
     while (done < steps) {
@@ -1599,7 +1612,7 @@ cudaError_t issue_chunks(mb_context* c, float t0, uint32_t steps, bool track) {
         mb::StepParams p = make_params(c, t, n, track);
         cudaError_t e = c->streamed  ? mb::launch_stream(p, 1024, c->stream_mpt, c->stream)
                         : c->cluster ? launch_split_groups(c, p)
-                        : use_tm(c, track) ? launch_tm_steps(c, p)
+                        : tm         ? launch_tm_steps(c, p)
                                      : mb::launch_step(p, c->shape, c->stream);
         if (e != cudaSuccess) return e;
         t = advance(t, c->dt, n);
@@ -1618,8 +1631,12 @@ mb_status run(mb_context* c, uint32_t steps, bool track) {
         if (!c->faces_packed) return fail(c, MB_ERR_CAPACITY, "face drag: the faces do not fit the step kernels");
     }
     cudaSetDevice(c->device);
-    if (tm_eligible(c)) MB_CUDA(c, tm_update(c, track));
-    if (!use_tm(c, track)) MB_CUDA(c, place_springs(c));
+    bool tm = false;
+    if (tm_eligible(c) && !short_launch(c, track, steps)) {
+        MB_CUDA(c, tm_update(c, track));
+        tm = use_tm(c, track);
+        if (!tm) MB_CUDA(c, place_springs(c));  // (for a short launch it would take longer than it saves)
+    }
     const float t0 = c->total_time;
     if (c->use_graph) {
         uint32_t bits;
@@ -1628,10 +1645,10 @@ mb_status run(mb_context* c, uint32_t steps, bool track) {
         auto it = c->graphs.find(key);
         if (it == c->graphs.end()) {
             if (c->graphs.size() >= 16) c->clear_graphs();
-            MB_CUDA(c, prepare_launch(c, track));
+            MB_CUDA(c, prepare_launch(c, track, tm));
             cudaGraph_t g;
             MB_CUDA(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-            cudaError_t e = issue_chunks(c, t0, steps, track);
+            cudaError_t e = issue_chunks(c, t0, steps, track, tm);
             cudaError_t e2 = cudaStreamEndCapture(c->stream, &g);
             if (e != cudaSuccess) {
                 if (e2 == cudaSuccess) cudaGraphDestroy(g);
@@ -1646,8 +1663,8 @@ mb_status run(mb_context* c, uint32_t steps, bool track) {
         }
         MB_CUDA(c, cudaGraphLaunch(it->second, c->stream));
     } else {
-        MB_CUDA(c, prepare_launch(c, track));
-        cudaError_t e = issue_chunks(c, t0, steps, track);
+        MB_CUDA(c, prepare_launch(c, track, tm));
+        cudaError_t e = issue_chunks(c, t0, steps, track, tm);
         if (e != cudaSuccess) return cuda_fail(c, e, "step launch");
     }
     c->total_time = advance(t0, c->dt, steps);
