@@ -311,7 +311,8 @@ class Simulator:
         return {f: getattr(c, f) for f, _ in c._fields_}
 
     def step_variant(self, track_stresses: bool = False) -> dict:
-        """The step kernel the next launches use, without or with stress tracking
+        """The step kernel the next launches use, without or with stress tracking (then
+        those of more than two steps)
         (mb_get_step_variant, mb_get_tracked_step_variant): register_rows (1 when
         each mass's row is held per thread) and the dynamic shared memory per CTA."""
         rr, smem = ctypes.c_uint32(), ctypes.c_uint32()

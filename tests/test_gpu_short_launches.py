@@ -6,6 +6,8 @@ import numpy as np
 import pytest
 
 import mercury_b200 as mb
+from mercury_b200 import robots
+from mercury_b200 import simulator as S
 from test_gpu_devo import OracleRun, check_same
 from test_step_plan import population
 
@@ -44,3 +46,27 @@ def test_chunks_of_a_step():
         sim.run_steps(5, track)
         orc.steps(5, track)
     check_same(sim, orc)
+
+
+@pytest.mark.parametrize("faces", [False, True], ids=["water", "faces"])
+@pytest.mark.parametrize("count", [3, 160])
+def test_short_launches_in_water(count, faces):
+    """Six tracked steps in one launch and in launches of one and two."""
+    els = []
+    for r in range(count):
+        cells = robots.random_cells(2 + r % 5, np.random.default_rng([count, r]))
+        els.append(robots.voxel_robot(cells, mass=0.1))
+        if faces:
+            els[-1].faces = robots.voxel_faces(cells)
+    b, got = mb.pack(els), []
+    for launches in ((6,), (1, 2, 1, 2)):
+        sim = mb.Simulator(0)
+        sim.set_materials(mb.materials.force_table())
+        sim.set_mode(S.MODE_FORCE_WATER)
+        sim.set_environment(**{**S.WATER, "face_drag": 1000.0 if faces else 0.0})
+        sim.setTimeStep(1e-4)
+        sim.set_batch(b)
+        for n in launches:
+            sim.run_steps(n, True)
+        got.append(sim.collect_arrays())
+    assert all(np.array_equal(x.view(np.uint32), y.view(np.uint32)) for x, y in zip(*got))
